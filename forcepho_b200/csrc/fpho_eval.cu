@@ -300,7 +300,7 @@ int launch_design_kernel(int variant, const TileArgs &A_in, int n_tiles, float *
     TileArgs A = A_in;
     A.live_cap = std::min(A.live_cap, DESIGN_LIVE_CAP);
     const size_t smem =
-        tile_smem_layout_bytes(V.design_nt / 32, A.live_cap, A.idx_cap, A.pgrad_stride);
+        design_smem_layout_bytes(A.live_cap, A.idx_cap);
     int dev = 0;
     CUDA_TRY(cudaGetDevice(&dev));
     if (dev >= 64) return set_error(FPHO_ERR_LIMIT, "device ordinal %d >= 64", dev);
@@ -321,7 +321,7 @@ size_t tile_smem_bytes(int variant, int live_cap, int idx_cap, int stride) {
     const Variant &V = kVariants[variant];
     if (V.split)
         return split_smem_layout_bytes(V.split, V.tile / 32, live_cap, idx_cap, stride);
-    return tile_smem_layout_bytes(V.nt / 32, live_cap, idx_cap, stride);
+    return tile_smem_layout_bytes(V.nt / 32, V.tile, live_cap, idx_cap, stride);
 }
 
 }  // namespace fpho

@@ -132,12 +132,12 @@ __global__ void __launch_bounds__(NT) normal_tiles(TileArgs A, double *pnorm, in
         Yp[j] = pk(yv[0], yv[1]);
         M[j] = 0ull;
     }
-    const int n_live = scan_tile<NT>(A, bb, g0, g1, npsf, kept);
+    const int n_live = scan_tile<NT, true>(A, bb, g0, g1, npsf, kept);
     const v2 KEXP2 = pk1(KEXP), KEXPLO2 = pk1(KEXP_LO), CM24 = pk1(-1.0f / 24.0f);
     for (int c0 = 0; c0 < n_live; c0 += cap) {
         const int n = min(cap, n_live - c0);
         if (c0 > 0) __syncthreads();
-        stage_records<NT>(recs, A.gtab + (size_t)g0 * GREC, kept, c0, n, 0, &mbar, phase, A.err);
+        stage_records<NT, GSTAGE>(recs, A.gtab + (size_t)g0 * GREC, kept, c0, n, 0, &mbar, phase, A.err);
         for (int i = 0; i < n; ++i) {
             const float *r = recs + (size_t)i * GSTAGE;
             int flag = kept[c0 + i];

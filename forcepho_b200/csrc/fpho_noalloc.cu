@@ -273,7 +273,7 @@ extern "C" int fpho_evaluate_proposal_noalloc(const fpho_patch_struct *patch, in
                          L.total, n_tiles_max, n_gauss_max, (unsigned)FPHO_NOALLOC_SCRATCH_BYTES);
     const int stride = 7 * nsrc;
     const int idx_cap = nsrc * max_psf_per_source;
-    const size_t smem = tile_smem_layout_bytes(NA_THREADS / 32, NA_LIVE_CAP, idx_cap, stride);
+    const size_t smem = tile_smem_layout_bytes(NA_THREADS / 32, NA_TILE, NA_LIVE_CAP, idx_cap, stride);
     if (smem > 227 * 1024)
         return set_error(FPHO_ERR_LIMIT, "shared memory %zu for %d image Gaussians per exposure "
                          "exceeds 227 KB", smem, idx_cap);

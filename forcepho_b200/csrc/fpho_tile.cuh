@@ -12,11 +12,13 @@
 //   3. residual pass: r = data - sum_g amp G H over kept Gaussians, in the
 //      reference's Gaussian order (ComputeResidualImage, common_kernel.cc:57-83);
 //   4. chi2 per pixel in double, exactly as compute_gaussians_kernel.cc:286-293;
-//   5. gradient pass: for each kept Gaussian, each thread accumulates the
-//      derivatives of its pixels' model w.r.t. the Gaussian's image-space
-//      parameters (A, x, y, fxx, fyy, fxy), then applies the Gaussian's
-//      Jacobian once (ComputeGaussianDerivative, common_kernel.cc:95-143, with
-//      the per-pixel Jacobian product moved out of the pixel loop);
+//   5. gradient pass, one kept Gaussian per lane (gradient_lanes): each lane
+//      walks the tile's pixels, broadcast from shared memory, and sums the
+//      moments of its Gaussian's weight; the derivatives of the model w.r.t.
+//      the Gaussian's image-space parameters (A, x, y, fxx, fyy, fxy) and the
+//      Gaussian's Jacobian are formed from them once
+//      (ComputeGaussianDerivative, common_kernel.cc:95-143, with the per-pixel
+//      Jacobian product moved out of the pixel loop);
 //   6. per-source sums are reduced across the warp and the CTA in a fixed
 //      order and written as this tile's partial; chi2 partials stay double.
 // Pixel pairs are processed as packed .f32x2 operands (two pixels per
@@ -98,75 +100,60 @@ __device__ __forceinline__ double warp_sum_d(double v) {
     return v;
 }
 
-// Reduce 7 per-lane values across the warp; afterwards lane k (k < 7) holds
-// the warp total of value k.  Uses 4+2+1+1+1 shuffles instead of 7*5.
-__device__ __forceinline__ float warp_reduce7(float v[8], int lane) {
-    // exchange 1: lanes < 16 keep 0..3, lanes >= 16 keep 4..7
-    {
-        const bool up = lane & 16;
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const float send = up ? v[i] : v[i + 4];
-            const float keep = up ? v[i + 4] : v[i];
-            v[i] = keep + __shfl_xor_sync(0xffffffffu, send, 16);
-        }
-    }
-    {
-        const bool up = lane & 8;
-#pragma unroll
-        for (int i = 0; i < 2; ++i) {
-            const float send = up ? v[i] : v[i + 2];
-            const float keep = up ? v[i + 2] : v[i];
-            v[i] = keep + __shfl_xor_sync(0xffffffffu, send, 8);
-        }
-    }
-    {
-        const bool up = lane & 4;
-        const float send = up ? v[0] : v[1];
-        const float keep = up ? v[1] : v[0];
-        v[0] = keep + __shfl_xor_sync(0xffffffffu, send, 4);
-    }
-    v[0] += __shfl_xor_sync(0xffffffffu, v[0], 2);
-    v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
-    // value index held by this lane group: bits (16 -> 4, 8 -> 2, 4 -> 1)
-    return v[0];
-}
-__device__ __forceinline__ int reduce7_index(int lane) {
-    return ((lane >> 4) & 1) * 4 + ((lane >> 3) & 1) * 2 + ((lane >> 2) & 1);
-}
-
 // ------------------------------------------------------------ shared layout
-// Dynamic shared memory of the tile kernel:
-//   [records live_cap x 128 B][kept indices idx_cap x 4 B][kept flags idx_cap x 4 B]
-//   [per-warp source sums NW x stride x 4 B]
-// Shared memory of one tile CTA: `live_cap` staged image-Gaussian records of
-// GSTAGE floats, the kept list (one int per Gaussian of the exposure: local
-// index << 2 | flags) and per-warp gradient sums.  (Reading the Jacobian half
-// of the records from global memory instead halves the stage, but the
-// exposure's records then miss L1 in the gradient epilogue; measured slower.)
-constexpr int GSTAGE = GREC;
-__host__ __device__ inline size_t tile_smem_layout_bytes(int nw, int live_cap, int idx_cap,
-                                                         int stride) {
-    return (size_t)live_cap * GSTAGE * 4 + (size_t)idx_cap * 4 + (size_t)nw * stride * 4;
+// Dynamic shared memory of a tile CTA, in order:
+//   stage   `live_cap` staged records of the residual pass (the first
+//           MODEL_STAGE floats of each: all it reads); afterwards the same
+//           bytes hold the pixels of the gradient pass, PX_BYTES each
+//           (px_block pixels at a time);
+//   kept    the kept list, one int per Gaussian of the exposure (local index
+//           << 2 | flags);
+//   wacc    per-warp gradient sums, `stride` floats each;
+//   part    split tiles only: the warps' partial models, one float per pixel.
+// The design passes stage whole records (they need the unit-flux amplitude
+// and the source index) and have neither gradient pixels nor partial models.
+constexpr int MODEL_STAGE = 16;  // floats of a record staged for the residual pass
+constexpr int GSTAGE = GREC;     // floats of a record staged for the design passes
+constexpr int PX_BYTES = 12;     // (u, -2 r ie^2) pairs and v of a gradient-pass pixel
+
+// Pixels of the tile that the gradient pass holds at a time: all of them,
+// unless `live_cap` is so small that they would need more than the 128 bytes
+// per staged record that a patch's limits are counted with.
+__host__ __device__ inline int px_block(int tile_pixels, int live_cap) {
+    int n = tile_pixels;
+    while (n * PX_BYTES > live_cap * 128) n >>= 1;
+    return n;
+}
+__host__ __device__ inline size_t stage_bytes(int tile_pixels, int live_cap) {
+    const size_t rec = (size_t)live_cap * MODEL_STAGE * 4;
+    const size_t px = ((size_t)px_block(tile_pixels, live_cap) * PX_BYTES + 127) / 128 * 128;
+    return rec > px ? rec : px;
+}
+__host__ __device__ inline size_t tile_smem_layout_bytes(int nw, int tile_pixels, int live_cap,
+                                                         int idx_cap, int stride) {
+    return stage_bytes(tile_pixels, live_cap) + (size_t)idx_cap * 4 + (size_t)nw * stride * 4;
+}
+__host__ __device__ inline size_t design_smem_layout_bytes(int live_cap, int idx_cap) {
+    return (size_t)live_cap * GSTAGE * 4 + (size_t)idx_cap * 4;
 }
 
-// Stage the records of kept entries [c0, c0 + n) of an exposure (first record
-// `gexp`) into `recs`, in list order, and wait for them.  Every thread of the
-// CTA issues the bulk copies of its records (one 128-byte copy each); issued
-// by one warp, the copies of a stage queued behind each other and the CTA
-// spent about a fifth of each tile waiting for them.  Callers have finished
-// reading `recs` (a barrier) before the call.
-template <int NT>
+// Stage the first FLOATS floats of the records of kept entries [c0, c0 + n) of
+// an exposure (first record `gexp`) into `recs`, in list order, and wait for
+// them.  Every thread of the CTA issues the bulk copies of its records (one
+// copy each); issued by one warp, the copies of a stage queued behind each
+// other and the CTA spent about a fifth of each tile waiting for them.
+// Callers have finished reading `recs` (a barrier) before the call.
+template <int NT, int FLOATS>
 __device__ __forceinline__ void stage_records(float *recs, const float *gexp, const int *kept,
                                               int c0, int n, int extra_tx, uint64_t *mbar,
                                               uint32_t &phase, int *err) {
     fence_proxy_async_smem();
     if (threadIdx.x == 0)
-        mbar_arrive_expect_tx(mbar, (uint32_t)(n * GSTAGE * 4 + extra_tx));
+        mbar_arrive_expect_tx(mbar, (uint32_t)(n * FLOATS * 4 + extra_tx));
     __syncthreads();  // the expected bytes are set before any copy can complete
     for (int i = threadIdx.x; i < n; i += NT)
-        bulk_g2s(recs + (size_t)i * GSTAGE, gexp + (size_t)(kept[c0 + i] >> 2) * GREC,
-                 GSTAGE * 4, mbar);
+        bulk_g2s(recs + (size_t)i * FLOATS, gexp + (size_t)(kept[c0 + i] >> 2) * GREC,
+                 FLOATS * 4, mbar);
     mbar_wait_bounded(mbar, phase, err);
     phase ^= 1u;
 }
@@ -325,135 +312,244 @@ __device__ __forceinline__ void residual_exact(const v2 (&X)[KP], const v2 (&Y)[
     }
 }
 
-// Pass 2 for one Gaussian over the thread's KP pixel pairs: the twelve sums
-// from which the model's derivatives w.r.t. (A, x, y, fxx, fyy, fxy) follow
-// (W = -2 r ie^2 G, H the pixel-integral correction, d = pixel - centre,
-// v = F d): sum W H, sum W H v, sum W v, sum W H d d^T, sum W, and sum W d d^T.
-// The epilogue forms sum W d.v terms from sum W d d^T and F once per
-// Gaussian (d_x v_x = fxx dx^2 + fxy dx dy, and so on), which is one packed
-// instruction per pixel pair cheaper than summing them per pixel; the
-// products dx^2, dx dy, dy^2 are formed once and weighted by both W H and W.
-struct GradSums {
-    v2 A, HVx, HVy, Vx, Vy, HXX, HXY, HYY, W, WXX, WXY, WYY;
-};
-template <int KP, bool CUT>
-__device__ __forceinline__ void gradient_pairs(const v2 (&X)[KP], const v2 (&Y)[KP],
-                                               const v2 (&R2)[KP], v2 NXC, v2 NYC, v2 FXX,
-                                               v2 FXY, v2 FYY, v2 C0, v2 C24, v2 KEXP2,
-                                               GradSums &s) {
-    s = GradSums{0ull, 0ull, 0ull, 0ull, 0ull, 0ull, 0ull, 0ull, 0ull, 0ull, 0ull, 0ull};
-#pragma unroll
-    for (int j = 0; j < KP; ++j) {
-        const v2 DX = add2(X[j], NXC), DY = add2(Y[j], NYC);
-        const v2 VX = fma2(FXY, DY, mul2(FXX, DX));
-        const v2 VY = fma2(FXY, DX, mul2(FYY, DY));
-        const v2 T1 = mul2(DX, VX);
-        const v2 Q = fma2(DY, VY, T1);
-        float e0, e1;
-        unpk(mul2(Q, KEXP2), e0, e1);
-        float g0 = ex2f(e0), g1 = ex2f(e1);
-        if (CUT) {
-            float q0, q1;
-            unpk(Q, q0, q1);
-            g0 = q0 > FPHO_MAX_EXP_ARG ? 0.0f : g0;
-            g1 = q1 > FPHO_MAX_EXP_ARG ? 0.0f : g1;
-        }
-        const v2 S = fma2(VY, VY, mul2(VX, VX));
-        const v2 H = fma2(S, C24, C0);
-        const v2 W = mul2(R2[j], pk(g0, g1));
-        const v2 WH = mul2(W, H);
-        s.A = add2(s.A, WH);
-        s.HVx = fma2(WH, VX, s.HVx);
-        s.HVy = fma2(WH, VY, s.HVy);
-        s.Vx = fma2(W, VX, s.Vx);
-        s.Vy = fma2(W, VY, s.Vy);
-        const v2 DXX = mul2(DX, DX), DXY = mul2(DX, DY), DYY = mul2(DY, DY);
-        s.HXX = fma2(WH, DXX, s.HXX);
-        s.HXY = fma2(WH, DXY, s.HXY);
-        s.HYY = fma2(WH, DYY, s.HYY);
-        s.W = add2(s.W, W);
-        s.WXX = fma2(W, DXX, s.WXX);
-        s.WXY = fma2(W, DXY, s.WXY);
-        s.WYY = fma2(W, DYY, s.WYY);
-    }
-}
-
-// Pass 2 for two consecutive kept Gaussians a, b at once (independent
-// exponentials interleave); each set of sums is formed in the same order as
-// by gradient_pairs, and the cut is applied to both (see residual_pairs2).
-template <int KP>
-__device__ __forceinline__ void gradient_pairs2(const v2 (&X)[KP], const v2 (&Y)[KP],
-                                                const v2 (&R2)[KP], const float *ra,
-                                                const float *rb, v2 C24, v2 KEXP2, GradSums &sa,
-                                                GradSums &sb) {
-    v2 NXa, NYa, FXXa, FXYa, FYYa, AMPa, HBa, C0a;
-    v2 NXb, NYb, FXXb, FXYb, FYYb, AMPb, HBb, C0b;
-    ld2(ra + R_NXC, NXa, NYa);
-    ld2(ra + R_FXX, FXXa, FXYa);
-    ld2(ra + R_FYY, FYYa, AMPa);
-    ld2(ra + R_HB, HBa, C0a);
-    ld2(rb + R_NXC, NXb, NYb);
-    ld2(rb + R_FXX, FXXb, FXYb);
-    ld2(rb + R_FYY, FYYb, AMPb);
-    ld2(rb + R_HB, HBb, C0b);
-    sa = GradSums{0ull, 0ull, 0ull, 0ull, 0ull, 0ull, 0ull, 0ull, 0ull, 0ull, 0ull, 0ull};
-    sb = sa;
-#pragma unroll
-    for (int j = 0; j < KP; ++j) {
-        const v2 DXa = add2(X[j], NXa), DYa = add2(Y[j], NYa);
-        const v2 DXb = add2(X[j], NXb), DYb = add2(Y[j], NYb);
-        const v2 VXa = fma2(FXYa, DYa, mul2(FXXa, DXa));
-        const v2 VXb = fma2(FXYb, DYb, mul2(FXXb, DXb));
-        const v2 VYa = fma2(FXYa, DXa, mul2(FYYa, DYa));
-        const v2 VYb = fma2(FXYb, DXb, mul2(FYYb, DYb));
-        const v2 T1a = mul2(DXa, VXa), T1b = mul2(DXb, VXb);
-        const v2 Qa = fma2(DYa, VYa, T1a), Qb = fma2(DYb, VYb, T1b);
-        float ea0, ea1, eb0, eb1, qa0, qa1, qb0, qb1;
-        unpk(mul2(Qa, KEXP2), ea0, ea1);
-        unpk(mul2(Qb, KEXP2), eb0, eb1);
-        unpk(Qa, qa0, qa1);
-        unpk(Qb, qb0, qb1);
-        const float ga0 = qa0 > FPHO_MAX_EXP_ARG ? 0.0f : ex2f(ea0);
-        const float ga1 = qa1 > FPHO_MAX_EXP_ARG ? 0.0f : ex2f(ea1);
-        const float gb0 = qb0 > FPHO_MAX_EXP_ARG ? 0.0f : ex2f(eb0);
-        const float gb1 = qb1 > FPHO_MAX_EXP_ARG ? 0.0f : ex2f(eb1);
-        const v2 Sa = fma2(VYa, VYa, mul2(VXa, VXa)), Sb = fma2(VYb, VYb, mul2(VXb, VXb));
-        const v2 Ha = fma2(Sa, C24, C0a), Hb = fma2(Sb, C24, C0b);
-        const v2 Wa = mul2(R2[j], pk(ga0, ga1)), Wb = mul2(R2[j], pk(gb0, gb1));
-        const v2 WHa = mul2(Wa, Ha), WHb = mul2(Wb, Hb);
-        sa.A = add2(sa.A, WHa);
-        sb.A = add2(sb.A, WHb);
-        sa.HVx = fma2(WHa, VXa, sa.HVx);
-        sb.HVx = fma2(WHb, VXb, sb.HVx);
-        sa.HVy = fma2(WHa, VYa, sa.HVy);
-        sb.HVy = fma2(WHb, VYb, sb.HVy);
-        sa.Vx = fma2(Wa, VXa, sa.Vx);
-        sb.Vx = fma2(Wb, VXb, sb.Vx);
-        sa.Vy = fma2(Wa, VYa, sa.Vy);
-        sb.Vy = fma2(Wb, VYb, sb.Vy);
-        const v2 DXXa = mul2(DXa, DXa), DXYa = mul2(DXa, DYa), DYYa = mul2(DYa, DYa);
-        const v2 DXXb = mul2(DXb, DXb), DXYb = mul2(DXb, DYb), DYYb = mul2(DYb, DYb);
-        sa.HXX = fma2(WHa, DXXa, sa.HXX);
-        sb.HXX = fma2(WHb, DXXb, sb.HXX);
-        sa.HXY = fma2(WHa, DXYa, sa.HXY);
-        sb.HXY = fma2(WHb, DXYb, sb.HXY);
-        sa.HYY = fma2(WHa, DYYa, sa.HYY);
-        sb.HYY = fma2(WHb, DYYb, sb.HYY);
-        sa.W = add2(sa.W, Wa);
-        sb.W = add2(sb.W, Wb);
-        sa.WXX = fma2(Wa, DXXa, sa.WXX);
-        sb.WXX = fma2(Wb, DXXb, sb.WXX);
-        sa.WXY = fma2(Wa, DXYa, sa.WXY);
-        sb.WXY = fma2(Wb, DXYb, sb.WXY);
-        sa.WYY = fma2(Wa, DYYa, sa.WYY);
-        sb.WYY = fma2(Wb, DYYb, sb.WYY);
-    }
-}
-
 __device__ __forceinline__ float lanesum(v2 v) {
     float a, b;
     unpk(v, a, b);
     return a + b;
+}
+
+// ------------------------------------------------------------ gradient pass
+// The pixels of the gradient pass in shared memory: x and the weight
+// r2 = -2 r ie^2 as pairs {x_2i, x_2i+1, r2_2i, r2_2i+1} (one 16-byte load is
+// two packed operands), and y.
+struct PixelStage {
+    float *xr;  // [2 pixels]
+    float *y;   // [pixels]
+};
+// Eight consecutive pixels are a run.  In the packed order of whole
+// super-pixels every run shares one coordinate: y where x varies fastest
+// inside a super-pixel, x where y does (the order of a pixel store).  These
+// bits say which coordinate is NOT shared by the runs of a tile; pixels of
+// weight zero do not count (they add nothing to the gradient), and padding
+// pixels are such.
+constexpr int MISFIT_Y = 1, MISFIT_X = 2;
+
+// One pixel's misfit bits against the first weighted pixel of its run, and
+// that pixel's coordinates in place of its own where its weight is zero.
+// Called by whole warps whose lanes hold 32 consecutive pixels.
+__device__ __forceinline__ int run_misfit(float &x, float &y, bool weighted) {
+    const int base = threadIdx.x & 24;
+    const unsigned in_run = (__ballot_sync(0xffffffffu, weighted) >> base) & 0xffu;
+    const int first = base + (in_run ? __ffs(in_run) - 1 : 0);
+    const float x0 = __shfl_sync(0xffffffffu, x, first);
+    const float y0 = __shfl_sync(0xffffffffu, y, first);
+    const int bits = weighted ? (y != y0 ? MISFIT_Y : 0) | (x != x0 ? MISFIT_X : 0) : 0;
+    x = weighted ? x : x0;
+    y = weighted ? y : y0;
+    return bits;
+}
+__device__ __forceinline__ void put_pixel(const PixelStage &px, int p, float x, float y,
+                                          float r2) {
+    float *q = px.xr + 4 * (p >> 1) + (p & 1);
+    q[0] = x;
+    q[2] = r2;
+    px.y[p] = y;
+}
+
+// Moments of one Gaussian's weight W = r2 G over pixels: m[a][b] = sum W du^a
+// dv^b, a + b <= 4, (u, v) the coordinate along the runs and the shared one.
+struct Moments {
+    float m00 = 0.f, m10 = 0.f, m20 = 0.f, m30 = 0.f, m40 = 0.f, m01 = 0.f, m11 = 0.f, m21 = 0.f,
+          m31 = 0.f, m02 = 0.f, m12 = 0.f, m22 = 0.f, m03 = 0.f, m13 = 0.f, m04 = 0.f;
+    // adds one run's moments along u (s_a = sum W du^a) at its dv
+    __device__ __forceinline__ void add(float dv, float dv2, float s0, float s1, float s2,
+                                        float s3, float s4) {
+        const float dv3 = dv2 * dv, dv4 = dv2 * dv2;
+        m00 += s0;
+        m10 += s1;
+        m20 += s2;
+        m30 += s3;
+        m40 += s4;
+        m01 = fmaf(dv, s0, m01);
+        m11 = fmaf(dv, s1, m11);
+        m21 = fmaf(dv, s2, m21);
+        m31 = fmaf(dv, s3, m31);
+        m02 = fmaf(dv2, s0, m02);
+        m12 = fmaf(dv2, s1, m12);
+        m22 = fmaf(dv2, s2, m22);
+        m03 = fmaf(dv3, s0, m03);
+        m13 = fmaf(dv3, s1, m13);
+        m04 = fmaf(dv4, s0, m04);
+    }
+};
+
+// One Gaussian in a lane: the exponent's quadratic form in (du, dv), scaled so
+// that G = 2^E.
+struct LaneForm {
+    float nu, nv;      // -centre
+    float e20, e11, e02;
+};
+constexpr float E_CUT = FPHO_MAX_EXP_ARG * KEXP;  // exp-arguments above 36: E below this
+
+// Moments over the runs [r0, r1).  Along a run the exponent is a quadratic in
+// du whose coefficients are formed once per run, and the weight's moments in
+// du are summed before they meet dv: 11 packed instructions per pixel pair and
+// 26 scalar ones per run, against 29 packed ones per pair if every pixel
+// formed its own products.  SHARED_X: the runs share x (u = y).
+template <bool SHARED_X>
+__device__ __forceinline__ void run_moments(const PixelStage &px, int r0, int r1,
+                                            const LaneForm &f, Moments &m) {
+    const v2 NU = pk1(f.nu), E20 = pk1(f.e20);
+#pragma unroll 1
+    for (int r = r0; r < r1; ++r) {
+        const float dv = (SHARED_X ? px.xr[16 * r] : px.y[8 * r]) + f.nv;
+        const float dv2 = dv * dv;
+        const v2 E11 = pk1(f.e11 * dv), E02 = pk1(f.e02 * dv2);
+        v2 S0, S1, S2, S3, S4;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            v2 U, R2;
+            ld2(px.xr + 16 * r + 4 * j, U, R2);
+            if (SHARED_X)
+                U = *reinterpret_cast<const unsigned long long *>(px.y + 8 * r + 2 * j);
+            const v2 DU = add2(U, NU);
+            float e0, e1;
+            unpk(fma2(fma2(E20, DU, E11), DU, E02), e0, e1);
+            const float g0 = e0 < E_CUT ? 0.0f : ex2f(e0);
+            const float g1 = e1 < E_CUT ? 0.0f : ex2f(e1);
+            const v2 W = mul2(R2, pk(g0, g1));
+            const v2 T1 = mul2(W, DU), T2 = mul2(T1, DU), T3 = mul2(T2, DU);
+            S0 = j ? add2(S0, W) : W;
+            S1 = j ? add2(S1, T1) : T1;
+            S2 = j ? add2(S2, T2) : T2;
+            S3 = j ? add2(S3, T3) : T3;
+            S4 = j ? fma2(T3, DU, S4) : mul2(T3, DU);
+        }
+        m.add(dv, dv2, lanesum(S0), lanesum(S1), lanesum(S2), lanesum(S3), lanesum(S4));
+    }
+}
+// The same over the pixel pairs [i0, i1) of a tile whose runs share nothing.
+__device__ __forceinline__ void pixel_moments(const PixelStage &px, int i0, int i1,
+                                              const LaneForm &f, Moments &m) {
+#pragma unroll 1
+    for (int i = i0; i < i1; ++i) {
+        const float4 ur = *reinterpret_cast<const float4 *>(px.xr + 4 * i);
+        const float2 yy = *reinterpret_cast<const float2 *>(px.y + 2 * i);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const float du = (h ? ur.y : ur.x) + f.nu, dv = (h ? yy.y : yy.x) + f.nv;
+            const float dv2 = dv * dv;
+            const float e = fmaf(fmaf(f.e20, du, f.e11 * dv), du, f.e02 * dv2);
+            const float w = (h ? ur.w : ur.z) * (e < E_CUT ? 0.0f : ex2f(e));
+            const float w1 = w * du, w2 = w1 * du, w3 = w2 * du;
+            m.add(dv, dv2, w, w1, w2, w3, w3 * du);
+        }
+    }
+}
+
+// The gradient pass over `n_px` staged pixels: every kept Gaussian of the tile
+// in a lane of its own.
+//
+// A lane forms the moments of its Gaussian's weight W = r2 G about the
+// Gaussian's centre; H = 1 + (|v|^2 - fxx - fyy)/24 is a quadratic in the
+// offsets, so every sum the derivatives need (sum W H, sum W H d, sum W H d
+// d^T, sum W, sum W d, sum W d d^T) is a combination of them, taken once per
+// Gaussian; then its Jacobian, and a sum over the lanes of each source.
+//
+// Against pixels in the lanes and Gaussians in the loop (each thread forming
+// the sums of its own 8 pixels), the per-Gaussian work is done once for a
+// whole tile instead of once per 8 pixels, and per-row work once per row.
+// Work is dealt to the warps in units of (32 Gaussians, 64 pixels), in order
+// and evenly, so that a kept list that is no multiple of 32 NW still keeps
+// every warp busy.
+template <int NW>
+__device__ __forceinline__ void gradient_lanes(const TileArgs &A, const int *kept, int n_live,
+                                               int g0, const PixelStage &px, int n_px, int misfit,
+                                               float *wacc) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int nq = (n_px + 63) >> 6;                 // 64-pixel units
+    const int units = ((n_live + 31) >> 5) * nq;
+    int left = units * (warp + 1) / NW - units * warp / NW;
+    int g = units * warp / NW / nq, q = units * warp / NW - g * nq;
+    float *row = wacc + warp * A.pgrad_stride;
+    const bool shared_x = (misfit & MISFIT_Y) && !(misfit & MISFIT_X);
+    for (; left > 0; ++g, q = 0) {
+        const int nm = min(left, nq - q);
+        left -= nm;
+        const bool alive = g * 32 + lane < n_live;
+        const int k = kept[min(g * 32 + lane, n_live - 1)] >> 2;
+        const float4 *r4 = reinterpret_cast<const float4 *>(A.gtab + (size_t)(g0 + k) * GREC);
+        const float4 ra = r4[0], rb = r4[1];
+        const float fyy = reinterpret_cast<const float *>(r4)[R_FYY];
+        const float fxx = rb.x, fxy = rb.z;
+        Moments m;
+        const LaneForm f = {shared_x ? ra.z : ra.x, shared_x ? ra.x : ra.z,
+                            (shared_x ? fyy : fxx) * KEXP, 2.0f * KEXP * fxy,
+                            (shared_x ? fxx : fyy) * KEXP};
+        if (shared_x)
+            run_moments<true>(px, 8 * q, 8 * (q + nm), f, m);
+        else if (!(misfit & MISFIT_Y))
+            run_moments<false>(px, 8 * q, 8 * (q + nm), f, m);
+        else
+            pixel_moments(px, 32 * q, 32 * (q + nm), f, m);
+        // sums over W H and over W, in (x, y)
+        const float c0 = reinterpret_cast<const float *>(r4)[R_C0];
+        const float fuu = shared_x ? fyy : fxx, fvv = shared_x ? fxx : fyy;
+        const float h20 = (fuu * fuu + fxy * fxy) * (1.0f / 24.0f);
+        const float h11 = 2.0f * fxy * (fuu + fvv) * (1.0f / 24.0f);
+        const float h02 = (fvv * fvv + fxy * fxy) * (1.0f / 24.0f);
+        const float gA = c0 * m.m00 + h20 * m.m20 + h11 * m.m11 + h02 * m.m02;
+        const float hu = c0 * m.m10 + h20 * m.m30 + h11 * m.m21 + h02 * m.m12;
+        const float hv = c0 * m.m01 + h20 * m.m21 + h11 * m.m12 + h02 * m.m03;
+        const float huu = c0 * m.m20 + h20 * m.m40 + h11 * m.m31 + h02 * m.m22;
+        const float hxy = c0 * m.m11 + h20 * m.m31 + h11 * m.m22 + h02 * m.m13;
+        const float hvv = c0 * m.m02 + h20 * m.m22 + h11 * m.m13 + h02 * m.m04;
+        const float hx = shared_x ? hv : hu, hy = shared_x ? hu : hv;
+        const float hxx = shared_x ? hvv : huu, hyy = shared_x ? huu : hvv;
+        const float wx = shared_x ? m.m01 : m.m10, wy = shared_x ? m.m10 : m.m01;
+        const float wxx = shared_x ? m.m02 : m.m20, wyy = shared_x ? m.m20 : m.m02;
+        const float wxy = m.m11, w0 = m.m00;
+        // derivatives w.r.t. (A, x, y, fxx, fyy, fxy): v = F d
+        const float sVx = fxx * wx + fxy * wy, sVy = fxy * wx + fyy * wy;
+        const float gx = fxx * hx + fxy * hy - (fxx * sVx + fxy * sVy) * (1.0f / 12.0f);
+        const float gy = fxy * hx + fyy * hy - (fxy * sVx + fyy * sVy) * (1.0f / 12.0f);
+        const float t1 = fxx * wxx + fxy * wxy;   // sum W dx vx
+        const float t2 = fyy * wyy + fxy * wxy;   // sum W dy vy
+        const float t3 = fxy * (wxx + wyy) + (fxx + fyy) * wxy;
+        const float gfxx = t1 * (1.0f / 12.0f) - 0.5f * hxx - w0 * (1.0f / 24.0f);
+        const float gfyy = t2 * (1.0f / 12.0f) - 0.5f * hyy - w0 * (1.0f / 24.0f);
+        const float gfxy = t3 * (1.0f / 12.0f) - hxy;
+        // the Jacobian (amp factors are folded into its rows)
+        const float4 j0 = r4[4], j1 = r4[5], j2 = r4[6], j3 = r4[7];
+        float P[7];
+        P[0] = j0.x * gA;
+        P[1] = fmaf(j1.z, gy, j1.y * gx);
+        P[2] = fmaf(j2.x, gy, j1.w * gx);
+        P[3] = fmaf(j2.w, gfyy, fmaf(j2.z, gfxy, fmaf(j2.y, gfxx, j0.y * gA)));
+        P[4] = fmaf(j3.z, gfyy, fmaf(j3.y, gfxy, fmaf(j3.x, gfxx, j0.z * gA)));
+        P[5] = j0.w * gA;
+        P[6] = j1.x * gA;
+        // per-source sums: sources are contiguous in the kept list, so each
+        // source's first lane collects the lanes after it
+        const int src = alive ? (int)min((unsigned)__float_as_int(j3.w),
+                                         (unsigned)(A.pv.n_sources - 1))
+                              : -1;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int so = __shfl_down_sync(0xffffffffu, src, o);
+            const bool same = lane + o < 32 && so == src;
+#pragma unroll
+            for (int c = 0; c < 7; ++c) {
+                const float v = __shfl_down_sync(0xffffffffu, P[c], o);
+                P[c] += same ? v : 0.0f;
+            }
+        }
+        const int before = __shfl_up_sync(0xffffffffu, src, 1);
+        if (src >= 0 && (lane == 0 || before != src))
+#pragma unroll
+            for (int c = 0; c < 7; ++c) row[src * 7 + c] += P[c];
+        __syncwarp();
+    }
 }
 
 // kept-list flag bits (the low two bits of each entry)
@@ -465,10 +561,10 @@ constexpr int FLAG_LAST_SRC = 2;   // last kept Gaussian of its source in the ch
 // those that can reach the tile (box overlap, then the exact minimum of the
 // exp-argument over the tile box `bb`), each entry (local index << 2 | flags)
 // with FLAG_CUT when the exp-argument can exceed 36 inside the tile (its
-// maximum over the box is at a corner) and FLAG_LAST_SRC on the last kept
-// Gaussian of each source.  Returns the number kept; ends with the list
-// visible to the whole CTA.
-template <int NT>
+// maximum over the box is at a corner) and, with LAST_SRC, FLAG_LAST_SRC on the
+// last kept Gaussian of each source.  Returns the number kept; ends with the
+// list visible to the whole CTA.
+template <int NT, bool LAST_SRC = false>
 __device__ __forceinline__ int scan_tile(const TileArgs &A, float4 bb, int g0, int g1, int npsf,
                                          int *kept) {
     constexpr int NW = NT / 32;
@@ -515,6 +611,7 @@ __device__ __forceinline__ int scan_tile(const TileArgs &A, float4 bb, int g0, i
         n_live += tot;
         __syncthreads();
     }
+    if (!LAST_SRC) return n_live;
     // last kept Gaussian of each source (sources are contiguous in the list)
     for (int i = tid; i < n_live; i += NT) {
         const int src = (kept[i] >> 2) / npsf;
@@ -539,13 +636,14 @@ __device__ __forceinline__ void tile_body(const TileArgs &A, int tile, unsigned 
     const int cap = A.live_cap;
     const int stride = A.pgrad_stride;
 
+    constexpr int TP = NT * K;  // pixels per tile
     float *recs = reinterpret_cast<float *>(smem);
     // kept list: exposure-local Gaussian index << 2 | FLAG_* bits
-    int *kept = reinterpret_cast<int *>(smem + (size_t)cap * GSTAGE * 4);
+    int *kept = reinterpret_cast<int *>(smem + stage_bytes(TP, cap));
     float *wacc = reinterpret_cast<float *>(kept + A.idx_cap);
 
     __shared__ double s_chi2[NW];
-    __shared__ int s_any_weight;
+    __shared__ int s_any_weight, s_misfit;
 
     const TileDesc td = A.tiles[tile];
     const float4 bb = A.want_residual ? A.tbox_all[tile] : A.tbox_w[tile];
@@ -559,7 +657,7 @@ __device__ __forceinline__ void tile_body(const TileArgs &A, int tile, unsigned 
     const float xmid = 0.5f * (bb.x + bb.y), ymid = 0.5f * (bb.z + bb.w);
     v2 X[KP], Y[KP], R[KP], R2[KP];
     float D[K], IE[K];
-    int any_w = 0;
+    int any_w = 0, misfit = 0;
 #pragma unroll
     for (int j = 0; j < KP; ++j) {
         float xs[2], ys[2];
@@ -573,23 +671,28 @@ __device__ __forceinline__ void tile_body(const TileArgs &A, int tile, unsigned 
             D[2 * j + h] = ok ? A.pv.data[pix] : 0.0f;
             IE[2 * j + h] = ok ? A.pv.ierr[pix] : 0.0f;
             any_w |= (IE[2 * j + h] != 0.0f);
+            if (GRAD) {
+                float x = xs[h], y = ys[h];
+                misfit |= run_misfit(x, y, IE[2 * j + h] != 0.0f);
+            }
         }
         X[j] = pk(xs[0], xs[1]);
         Y[j] = pk(ys[0], ys[1]);
         R[j] = pk(D[2 * j], D[2 * j + 1]);
     }
-    if (tid == 0) s_any_weight = 0;
+    if (tid == 0) s_any_weight = s_misfit = 0;
 
     // ---- the ordered list of kept image Gaussians
     const int n_live = scan_tile<NT>(A, bb, g0, g1, npsf, kept);
     if (any_w) s_any_weight = 1;
+    if (misfit) atomicOr(&s_misfit, misfit);
     __syncthreads();
     const bool tile_has_weight = s_any_weight != 0;
 
     // ---- stage kept records [c0, c0 + n) into shared memory with bulk copies
     auto stage = [&](int c0, int n) {
-        stage_records<NT>(recs, A.gtab + (size_t)g0 * GREC, kept, c0, n, A.test_extra_tx, mbar,
-                          phase, A.err);
+        stage_records<NT, MODEL_STAGE>(recs, A.gtab + (size_t)g0 * GREC, kept, c0, n,
+                                       A.test_extra_tx, mbar, phase, A.err);
     };
 
     const v2 KEXP2 = pk1(KEXP), KEXPLO2 = pk1(KEXP_LO);
@@ -602,15 +705,15 @@ __device__ __forceinline__ void tile_body(const TileArgs &A, int tile, unsigned 
         if (c > 0) __syncthreads();  // previous chunk fully consumed
         stage(c0, n);
         if (EXACT) {
-            for (int i = 0; i < n; ++i) residual_exact<KP>(X, Y, R, recs + (size_t)i * GSTAGE);
+            for (int i = 0; i < n; ++i) residual_exact<KP>(X, Y, R, recs + (size_t)i * MODEL_STAGE);
             continue;
         }
         int i = 0;
         for (; i + 1 < n; i += 2)
-            residual_pairs2<KP>(X, Y, R, recs + (size_t)i * GSTAGE, recs + (size_t)(i + 1) * GSTAGE,
+            residual_pairs2<KP>(X, Y, R, recs + (size_t)i * MODEL_STAGE, recs + (size_t)(i + 1) * MODEL_STAGE,
                                 CM24, KEXP2, KEXPLO2);
         for (; i < n; ++i) {
-            const float *r = recs + (size_t)i * GSTAGE;
+            const float *r = recs + (size_t)i * MODEL_STAGE;
             v2 NXC, NYC, FXX, FXY, FYY, AMP, HB, C0;
             ld2(r + R_NXC, NXC, NYC);
             ld2(r + R_FXX, FXX, FXY);
@@ -650,81 +753,25 @@ __device__ __forceinline__ void tile_body(const TileArgs &A, int tile, unsigned 
     if (lane == 0) s_chi2[warp] = chi2;
 
     // ------------------------------------------------------------ pass 2
-    // Chunks in reverse order: the last chunk of pass 1 is still staged.
-    if (GRAD && tile_has_weight) {
-        float P[7] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-        for (int c = n_chunks - 1; c >= 0; --c) {
-            const int c0 = c * cap, n = min(cap, n_live - c0);
-            if (c != n_chunks - 1) {
-                __syncthreads();
-                stage(c0, n);
-            }
-            // the Jacobian epilogue of one Gaussian, in list order
-            auto epilogue = [&](const float *r, int flag, const GradSums &s, bool last) {
-                const float4 *rj = reinterpret_cast<const float4 *>(r + R_JA_FLUX);
-                // image-space gradient of this Gaussian over the thread's pixels
-                // (amp factors are folded into the Jacobian rows), in scalars
-                const float fxx = r[R_FXX], fxy = r[R_FXY], fyy = r[R_FYY];
-                const float sVx = lanesum(s.Vx), sVy = lanesum(s.Vy), sW = lanesum(s.W);
-                const float gA = lanesum(s.A);
-                const float gx = lanesum(s.HVx) - (fxx * sVx + fxy * sVy) * (1.0f / 12.0f);
-                const float gy = lanesum(s.HVy) - (fxy * sVx + fyy * sVy) * (1.0f / 12.0f);
-                // sum W d.v terms from sum W d d^T: dx vx, dy vy, dx vy + dy vx
-                const float wxx = lanesum(s.WXX), wxy = lanesum(s.WXY), wyy = lanesum(s.WYY);
-                const float t1 = fxx * wxx + fxy * wxy;
-                const float t2 = fyy * wyy + fxy * wxy;
-                const float t3 = fxy * (wxx + wyy) + (fxx + fyy) * wxy;
-                const float gfxx = t1 * (1.0f / 12.0f) - 0.5f * lanesum(s.HXX) -
-                                   sW * (1.0f / 24.0f);
-                const float gfyy = t2 * (1.0f / 12.0f) - 0.5f * lanesum(s.HYY) -
-                                   sW * (1.0f / 24.0f);
-                const float gfxy = t3 * (1.0f / 12.0f) - lanesum(s.HXY);
-                const float4 j0 = rj[0], j1 = rj[1], j2 = rj[2], j3 = rj[3];
-                P[0] = fmaf(j0.x, gA, P[0]);
-                P[1] = fmaf(j1.z, gy, fmaf(j1.y, gx, P[1]));
-                P[2] = fmaf(j2.x, gy, fmaf(j1.w, gx, P[2]));
-                P[3] = fmaf(j2.w, gfyy, fmaf(j2.z, gfxy, fmaf(j2.y, gfxx, fmaf(j0.y, gA, P[3]))));
-                P[4] = fmaf(j3.z, gfyy, fmaf(j3.y, gfxy, fmaf(j3.x, gfxx, fmaf(j0.z, gA, P[4]))));
-                P[5] = fmaf(j0.w, gA, P[5]);
-                P[6] = fmaf(j1.x, gA, P[6]);
-                // flush at a source boundary or at the end of the chunk
-                if ((flag & FLAG_LAST_SRC) || last) {
-                    // the index comes from the staged record: bounded, so that
-                    // a stage a timed-out wait left stale cannot write outside
-                    // the sums (the error word already marks the evaluation)
-                    const int src = min((unsigned)__float_as_int(j3.w),
-                                        (unsigned)(A.pv.n_sources - 1));
-                    float v[8] = {P[0], P[1], P[2], P[3], P[4], P[5], P[6], 0.0f};
+    // the pixels in shared memory (over the staged records), px_block of them
+    // at a time; every kept Gaussian in a lane
+    if (GRAD && tile_has_weight && n_live > 0) {
+        const int pxb = px_block(TP, cap);
+        const PixelStage px = {recs, recs + 2 * pxb};
+        const int fits = s_misfit;
+        for (int b0 = 0; b0 < td.count; b0 += pxb) {
+            __syncthreads();  // records (or the previous pixels) fully consumed
 #pragma unroll
-                    for (int k = 0; k < 7; ++k) P[k] = 0.0f;
-                    const float tot = warp_reduce7(v, lane);
-                    const int k = reduce7_index(lane);
-                    if ((lane & 3) == 0 && k < 7) wacc[warp * stride + src * 7 + k] += tot;
-                }
-            };
-            int i = 0;
-            for (; i + 1 < n; i += 2) {
-                const float *ra = recs + (size_t)i * GSTAGE, *rb = ra + GSTAGE;
-                GradSums sa, sb;
-                gradient_pairs2<KP>(X, Y, R2, ra, rb, C24, KEXP2, sa, sb);
-                epilogue(ra, kept[c0 + i], sa, false);
-                epilogue(rb, kept[c0 + i + 1], sb, i + 1 == n - 1);
+            for (int k = 0; k < K; ++k) {
+                const int p = tid + k * NT - b0;  // whole warps are in or out of the block
+                float x = (k & 1) ? hi(X[k / 2]) : lo(X[k / 2]);
+                float y = (k & 1) ? hi(Y[k / 2]) : lo(Y[k / 2]);
+                if (p < 0 || p >= pxb) continue;
+                run_misfit(x, y, IE[k] != 0.0f);
+                put_pixel(px, p, x, y, (k & 1) ? hi(R2[k / 2]) : lo(R2[k / 2]));
             }
-            for (; i < n; ++i) {
-                const float *r = recs + (size_t)i * GSTAGE;
-                v2 NXC, NYC, FXX, FXY, FYY, AMP, HB, C0;
-                ld2(r + R_NXC, NXC, NYC);
-                ld2(r + R_FXX, FXX, FXY);
-                ld2(r + R_FYY, FYY, AMP);
-                ld2(r + R_HB, HB, C0);
-                const int flag = kept[c0 + i];
-                GradSums s;
-                if (flag & FLAG_CUT)
-                    gradient_pairs<KP, true>(X, Y, R2, NXC, NYC, FXX, FXY, FYY, C0, C24, KEXP2, s);
-                else
-                    gradient_pairs<KP, false>(X, Y, R2, NXC, NYC, FXX, FXY, FYY, C0, C24, KEXP2, s);
-                epilogue(r, flag, s, i == n - 1);
-            }
+            __syncthreads();
+            gradient_lanes<NW>(A, kept, n_live, g0, px, min(pxb, td.count - b0), fits, wacc);
         }
     }
     __syncthreads();
@@ -753,13 +800,10 @@ __device__ __forceinline__ void tile_body(const TileArgs &A, int tile, unsigned 
 // l, l+32, ..., K per thread, as K/2 packed pairs) and takes a contiguous
 // 1/NW of each staged chunk of kept Gaussians.
 //   pass 1: each warp sums -model over its Gaussians; the NW partial models
-//           are added to the data in warp order through shared memory, so
-//           every warp holds the same residual bit for bit;
-//   chi2:   warp 0, in double, as tile_body;
-//   pass 2: each warp forms the gradient of its Gaussians (12 packed sums per
-//           Gaussian, Jacobian applied once per Gaussian per thread) and
-//           flushes per-source sums into its own shared-memory row; the rows
-//           are added in warp order at the end.
+//           are added to the data in warp order through shared memory;
+//   chi2:   each thread its share of the pixels, in double;
+//   pass 2: gradient_lanes, as tile_body; each warp sums into its own
+//           shared-memory row; the rows are added in warp order at the end.
 // Against tile_body with NT = 32 NW threads and K' = K / NW pixels per thread
 // on the same tile, each thread does the per-Gaussian work (record loads,
 // exp-argument set-up, Jacobian epilogue) for NW times as many pixels, and a
@@ -769,8 +813,7 @@ __device__ __forceinline__ void tile_body(const TileArgs &A, int tile, unsigned 
 // tile_body's, so the two agree to rounding, not bit for bit.
 __host__ __device__ inline size_t split_smem_layout_bytes(int nw, int k, int live_cap, int idx_cap,
                                                          int stride) {
-    return (size_t)live_cap * GSTAGE * 4 + (size_t)idx_cap * 4 + (size_t)nw * stride * 4 +
-           (size_t)nw * 32 * k * 4;
+    return tile_smem_layout_bytes(nw, 32 * k, live_cap, idx_cap, stride) + (size_t)nw * 32 * k * 4;
 }
 
 template <int NW, int K, bool GRAD = true>
@@ -785,12 +828,11 @@ __device__ __forceinline__ void tile_body_split(const TileArgs &A, int tile, uns
     const int stride = A.pgrad_stride;
 
     float *recs = reinterpret_cast<float *>(smem);
-    int *kept = reinterpret_cast<int *>(smem + (size_t)cap * GSTAGE * 4);
+    int *kept = reinterpret_cast<int *>(smem + stage_bytes(TP, cap));
     float *wacc = reinterpret_cast<float *>(kept + A.idx_cap);
     float *part = wacc + (size_t)NW * stride;  // [NW][TP] partial models
 
-    __shared__ double s_chi2;
-    __shared__ int s_any_weight;
+    __shared__ double s_chi2[NW];
 
     const TileDesc td = A.tiles[tile];
     const float4 bb = A.want_residual ? A.tbox_all[tile] : A.tbox_w[tile];
@@ -803,7 +845,7 @@ __device__ __forceinline__ void tile_body_split(const TileArgs &A, int tile, uns
     // ---- the tile's pixels, in every warp: pair j holds pixels lane + 64j, lane + 64j + 32
     const float xmid = 0.5f * (bb.x + bb.y), ymid = 0.5f * (bb.z + bb.w);
     v2 X[KP], Y[KP], R[KP];
-    int any_w = 0;
+    int any_w = 0, misfit = 0;
 #pragma unroll
     for (int j = 0; j < KP; ++j) {
         float xs[2], ys[2];
@@ -814,22 +856,26 @@ __device__ __forceinline__ void tile_body_split(const TileArgs &A, int tile, uns
             const int pix = td.pix_begin + (ok ? li : 0);
             xs[h] = ok ? A.pv.xpix[pix] : xmid;
             ys[h] = ok ? A.pv.ypix[pix] : ymid;
-            any_w |= ok && (A.pv.ierr[pix] != 0.0f);
+            const bool weighted = ok && A.pv.ierr[pix] != 0.0f;
+            any_w |= weighted;
+            if (GRAD) {
+                float x = xs[h], y = ys[h];
+                misfit |= run_misfit(x, y, weighted);
+            }
         }
         X[j] = pk(xs[0], xs[1]);
         Y[j] = pk(ys[0], ys[1]);
         R[j] = 0ull;  // -model of this warp's Gaussians
     }
-    if (tid == 0) s_any_weight = 0;
+    // every warp holds every pixel: no exchange
+    const bool tile_has_weight = __any_sync(0xffffffffu, any_w);
+    misfit = __reduce_or_sync(0xffffffffu, misfit);
 
     const int n_live = scan_tile<NT>(A, bb, g0, g1, npsf, kept);
-    if (any_w) s_any_weight = 1;
-    __syncthreads();
-    const bool tile_has_weight = s_any_weight != 0;
 
     auto stage = [&](int c0, int n) {
-        stage_records<NT>(recs, A.gtab + (size_t)g0 * GREC, kept, c0, n, A.test_extra_tx, mbar,
-                          phase, A.err);
+        stage_records<NT, MODEL_STAGE>(recs, A.gtab + (size_t)g0 * GREC, kept, c0, n,
+                                       A.test_extra_tx, mbar, phase, A.err);
     };
     // this warp's share [i0, i1) of a chunk of n records: contiguous, even
     // lengths (two Gaussians per step)
@@ -852,10 +898,10 @@ __device__ __forceinline__ void tile_body_split(const TileArgs &A, int tile, uns
         share(n, i0, i1);
         int i = i0;
         for (; i + 1 < i1; i += 2)
-            residual_pairs2<KP>(X, Y, R, recs + (size_t)i * GSTAGE, recs + (size_t)(i + 1) * GSTAGE,
+            residual_pairs2<KP>(X, Y, R, recs + (size_t)i * MODEL_STAGE, recs + (size_t)(i + 1) * MODEL_STAGE,
                                 CM24, KEXP2, KEXPLO2);
         for (; i < i1; ++i) {
-            const float *r = recs + (size_t)i * GSTAGE;
+            const float *r = recs + (size_t)i * MODEL_STAGE;
             v2 NXC, NYC, FXX, FXY, FYY, AMP, HB, C0;
             ld2(r + R_NXC, NXC, NYC);
             ld2(r + R_FXX, FXX, FXY);
@@ -878,116 +924,49 @@ __device__ __forceinline__ void tile_body_split(const TileArgs &A, int tile, uns
         part[warp * TP + lane + 64 * j + 32] = m1;
     }
     __syncthreads();
-    v2 R2[KP];
+    // each thread finishes its share of the pixels: residual, chi2 (double) and
+    // the gradient pass's pixels, over the staged records (no longer read)
+    const PixelStage px = {recs, recs + 2 * TP};
     double chi2 = 0.0;
 #pragma unroll
-    for (int j = 0; j < KP; ++j) {
-        float r2v[2];
+    for (int i = 0; i < (TP + NT - 1) / NT; ++i) {
+        const int li = tid + i * NT;
+        if (li >= TP) break;  // whole warps
+        const bool ok = li < td.count;
+        const int pix = td.pix_begin + (ok ? li : 0);
+        const float d = ok ? A.pv.data[pix] : 0.0f;
+        const float ie = ok ? A.pv.ierr[pix] : 0.0f;
+        float r = d;
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const int li = lane + (2 * j + h) * 32;
-            const bool ok = li < td.count;
-            const int pix = td.pix_begin + (ok ? li : 0);
-            const float d = ok ? A.pv.data[pix] : 0.0f;
-            const float ie = ok ? A.pv.ierr[pix] : 0.0f;
-            float r = d;
-#pragma unroll
-            for (int w = 0; w < NW; ++w) r += part[w * TP + li];
-            if (warp == 0) {
-                if (A.want_residual && ok) A.pv.residual[pix] = r;
-                const float rie = r * ie, die = d * ie;
-                double c = ((double)rie - (double)die);
-                c *= ((double)rie + (double)die);
-                chi2 += (ie != 0.0f) ? c : 0.0;
-            }
-            r2v[h] = (ie != 0.0f) ? -2.0f * ((r * ie) * ie) : 0.0f;
+        for (int w = 0; w < NW; ++w) r += part[w * TP + li];
+        if (A.want_residual && ok) A.pv.residual[pix] = r;
+        const float rie = r * ie, die = d * ie;
+        double c = ((double)rie - (double)die);
+        c *= ((double)rie + (double)die);
+        chi2 += (ie != 0.0f) ? c : 0.0;
+        if (GRAD) {
+            float x = ok ? A.pv.xpix[pix] : xmid, y = ok ? A.pv.ypix[pix] : ymid;
+            run_misfit(x, y, ie != 0.0f);
+            put_pixel(px, li, x, y, (ie != 0.0f) ? -2.0f * ((r * ie) * ie) : 0.0f);
         }
-        R2[j] = pk(r2v[0], r2v[1]);
     }
-    if (warp == 0) {
-        chi2 = warp_sum_d(chi2);
-        if (lane == 0) s_chi2 = chi2;
-    }
+    chi2 = warp_sum_d(chi2);
+    if (lane == 0) s_chi2[warp] = chi2;
 
     // ------------------------------------------------------------ pass 2
-    if (GRAD && tile_has_weight) {
-        float P[7] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-        for (int c = n_chunks - 1; c >= 0; --c) {
-            const int c0 = c * cap, n = min(cap, n_live - c0);
-            if (c != n_chunks - 1) {
-                __syncthreads();
-                stage(c0, n);
-            }
-            int i0, i1;
-            share(n, i0, i1);
-            auto epilogue = [&](const float *r, int flag, const GradSums &s, bool last) {
-                const float4 *rj = reinterpret_cast<const float4 *>(r + R_JA_FLUX);
-                const float fxx = r[R_FXX], fxy = r[R_FXY], fyy = r[R_FYY];
-                const float sVx = lanesum(s.Vx), sVy = lanesum(s.Vy), sW = lanesum(s.W);
-                const float gA = lanesum(s.A);
-                const float gx = lanesum(s.HVx) - (fxx * sVx + fxy * sVy) * (1.0f / 12.0f);
-                const float gy = lanesum(s.HVy) - (fxy * sVx + fyy * sVy) * (1.0f / 12.0f);
-                // sum W d.v terms from sum W d d^T: dx vx, dy vy, dx vy + dy vx
-                const float wxx = lanesum(s.WXX), wxy = lanesum(s.WXY), wyy = lanesum(s.WYY);
-                const float t1 = fxx * wxx + fxy * wxy;
-                const float t2 = fyy * wyy + fxy * wxy;
-                const float t3 = fxy * (wxx + wyy) + (fxx + fyy) * wxy;
-                const float gfxx = t1 * (1.0f / 12.0f) - 0.5f * lanesum(s.HXX) -
-                                   sW * (1.0f / 24.0f);
-                const float gfyy = t2 * (1.0f / 12.0f) - 0.5f * lanesum(s.HYY) -
-                                   sW * (1.0f / 24.0f);
-                const float gfxy = t3 * (1.0f / 12.0f) - lanesum(s.HXY);
-                const float4 j0 = rj[0], j1 = rj[1], j2 = rj[2], j3 = rj[3];
-                P[0] = fmaf(j0.x, gA, P[0]);
-                P[1] = fmaf(j1.z, gy, fmaf(j1.y, gx, P[1]));
-                P[2] = fmaf(j2.x, gy, fmaf(j1.w, gx, P[2]));
-                P[3] = fmaf(j2.w, gfyy, fmaf(j2.z, gfxy, fmaf(j2.y, gfxx, fmaf(j0.y, gA, P[3]))));
-                P[4] = fmaf(j3.z, gfyy, fmaf(j3.y, gfxy, fmaf(j3.x, gfxx, fmaf(j0.z, gA, P[4]))));
-                P[5] = fmaf(j0.w, gA, P[5]);
-                P[6] = fmaf(j1.x, gA, P[6]);
-                if ((flag & FLAG_LAST_SRC) || last) {
-                    // the index comes from the staged record: bounded, so that
-                    // a stage a timed-out wait left stale cannot write outside
-                    // the sums (the error word already marks the evaluation)
-                    const int src = min((unsigned)__float_as_int(j3.w),
-                                        (unsigned)(A.pv.n_sources - 1));
-                    float v[8] = {P[0], P[1], P[2], P[3], P[4], P[5], P[6], 0.0f};
-#pragma unroll
-                    for (int k = 0; k < 7; ++k) P[k] = 0.0f;
-                    const float tot = warp_reduce7(v, lane);
-                    const int k = reduce7_index(lane);
-                    if ((lane & 3) == 0 && k < 7) wacc[warp * stride + src * 7 + k] += tot;
-                }
-            };
-            int i = i0;
-            for (; i + 1 < i1; i += 2) {
-                const float *ra = recs + (size_t)i * GSTAGE, *rb = ra + GSTAGE;
-                GradSums sa, sb;
-                gradient_pairs2<KP>(X, Y, R2, ra, rb, C24, KEXP2, sa, sb);
-                epilogue(ra, kept[c0 + i], sa, false);
-                epilogue(rb, kept[c0 + i + 1], sb, i + 1 == i1 - 1);
-            }
-            for (; i < i1; ++i) {
-                const float *r = recs + (size_t)i * GSTAGE;
-                v2 NXC, NYC, FXX, FXY, FYY, AMP, HB, C0;
-                ld2(r + R_NXC, NXC, NYC);
-                ld2(r + R_FXX, FXX, FXY);
-                ld2(r + R_FYY, FYY, AMP);
-                ld2(r + R_HB, HB, C0);
-                const int flag = kept[c0 + i];
-                GradSums s;
-                if (flag & FLAG_CUT)
-                    gradient_pairs<KP, true>(X, Y, R2, NXC, NYC, FXX, FXY, FYY, C0, C24, KEXP2, s);
-                else
-                    gradient_pairs<KP, false>(X, Y, R2, NXC, NYC, FXX, FXY, FYY, C0, C24, KEXP2, s);
-                epilogue(r, flag, s, i == i1 - 1);
-            }
-        }
+    if (GRAD && tile_has_weight && n_live > 0) {
+        __syncthreads();  // every pixel staged
+        gradient_lanes<NW>(A, kept, n_live, g0, px, td.count, misfit, wacc);
     }
     __syncthreads();
 
     // ---- tile partials (fixed-order sums)
-    if (tid == 0) A.pchi2[tile] = s_chi2;
+    if (tid == 0) {
+        double c = 0.0;
+#pragma unroll
+        for (int w = 0; w < NW; ++w) c += s_chi2[w];
+        A.pchi2[tile] = c;
+    }
     for (int j = tid; GRAD && j < stride; j += NT) {
         float v = 0.0f;
 #pragma unroll
@@ -1113,12 +1092,12 @@ __device__ __forceinline__ void design_body(const TileArgs &A, int tile, unsigne
         Yp[j] = pk(ys[0], ys[1]);
         M[j] = 0ull;
     }
-    const int n_live = scan_tile<NT>(A, bb, g0, g1, npsf, kept);
+    const int n_live = scan_tile<NT, true>(A, bb, g0, g1, npsf, kept);
     const v2 KEXP2 = pk1(KEXP), KEXPLO2 = pk1(KEXP_LO), CM24 = pk1(-1.0f / 24.0f);
     for (int c0 = 0; c0 < n_live; c0 += cap) {
         const int n = min(cap, n_live - c0);
         if (c0 > 0) __syncthreads();
-        stage_records<NT>(recs, A.gtab + (size_t)g0 * GREC, kept, c0, n, 0, mbar, phase, A.err);
+        stage_records<NT, GSTAGE>(recs, A.gtab + (size_t)g0 * GREC, kept, c0, n, 0, mbar, phase, A.err);
         for (int i = 0; i < n; ++i) {
             const float *r = recs + (size_t)i * GSTAGE;
             int flag = kept[c0 + i];
