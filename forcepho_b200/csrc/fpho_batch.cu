@@ -83,7 +83,7 @@ __global__ void __launch_bounds__(NT, MINB) batch_tiles(const TileArgs *args, co
         if (it >= n_work) break;
         const int2 w = work[it];
         if constexpr (SPLIT > 0)
-            tile_body_split<SPLIT, K>(args[w.x], w.y, smem, &mbar, phase);
+            tile_body_split<SPLIT, K>(args[w.x], w.y, 0, smem, &mbar, phase);
         else
             tile_body<NT, K>(args[w.x], w.y, smem, &mbar, phase);
         __syncthreads();  // shared memory of this tile fully consumed
@@ -292,6 +292,8 @@ extern "C" int fpho_batch_create_config(fpho_patch *const *patches, int n, int v
         A.idx_cap = std::max(p->max_g, 1);
         A.err = b->d_err;
         A.pairs = nullptr;
+        A.tile_misfit = p->d_tile_misfit;
+        A.runs = p->d_runs;
         b->h_args.push_back(A);
         b->max_stride = std::max(b->max_stride, 7 * p->n_sources);
         for (int t = 0; t < p->n_tiles; ++t) {

@@ -124,7 +124,7 @@ __global__ void __launch_bounds__(NT) design_kernel(TileArgs A, float *X, long l
 // least MINB resident CTAs per SM, a register cap of 64K / (32 NW MINB); the
 // default, 16 / NW, caps at 128 registers a thread (left free, the compiler
 // takes up to 180 and halves the resident warps).
-template <int NW, int K, bool GRAD, int MINB = 16 / NW>
+template <int NW, int K, bool GRAD, int MINB = 16 / NW, int PS = 1>
 __global__ void __launch_bounds__(32 * NW, MINB) split_kernel(TileArgs A) {
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ uint64_t mbar;
@@ -134,7 +134,7 @@ __global__ void __launch_bounds__(32 * NW, MINB) split_kernel(TileArgs A) {
     }
     __syncthreads();
     uint32_t phase = 0;
-    tile_body_split<NW, K, GRAD>(A, blockIdx.x, smem, &mbar, phase);
+    tile_body_split<NW, K, GRAD, PS>(A, blockIdx.x / PS, blockIdx.x % PS, smem, &mbar, phase);
 }
 
 template <int NW, int K, bool GRAD, int MINB = 16 / NW>
@@ -154,7 +154,7 @@ __global__ void __launch_bounds__(32 * NW, MINB) split_kernel_dyn(TileArgs A, co
         __syncthreads();
         const int item = s_item;
         if (item >= n_tiles) break;
-        tile_body_split<NW, K, GRAD>(A, order[item], smem, &mbar, phase);
+        tile_body_split<NW, K, GRAD>(A, order[item], 0, smem, &mbar, phase);
         __syncthreads();
     }
 }
@@ -164,12 +164,16 @@ __global__ void __launch_bounds__(32 * NW, MINB) split_kernel_dyn(TileArgs A, co
 // with the residual pass in the reference's float arithmetic (the
 // exact-residual mode; compiled for the default 64x4 tile only).
 enum { KIND_CHI2 = 0, KIND_GRAD = 1, KIND_EXACT = 2, N_KINDS = 3 };
+// Parts per tile of the parted forms (tile_body_split's PS).
+enum { N_PARTED = 2 };
+constexpr int PARTS[N_PARTED] = {2, 4};
 struct Variant {
     int nt;                    // threads per CTA
     int tile;                  // pixels per tile
     int split;                 // 0: tile_body (every thread its own pixels); NW: tile_body_split
     const void *fn[N_KINDS];   // one CTA per tile, by kind (nullptr: not compiled)
     const void *dyn[N_KINDS];  // persistent forms of the same
+    const void *parts[N_PARTED][2];  // PARTS[i] CTAs per tile: chi2, + gradient
     const void *design;        // design-matrix rows over tiles of the same size
     int design_nt;             // its threads per CTA
 };
@@ -178,6 +182,7 @@ struct Variant {
      {(const void *)tile_kernel<NT, K, false>, (const void *)tile_kernel<NT, K, true>, nullptr}, \
      {(const void *)tile_kernel_dyn<NT, K, false>, (const void *)tile_kernel_dyn<NT, K, true>,  \
       nullptr},                                                                                  \
+     {{nullptr, nullptr}, {nullptr, nullptr}},                                                   \
      (const void *)design_kernel<NT, K>, NT}
 #define FPHO_VARIANT_EXACT(NT, K)                                                                \
     {NT, NT * K, 0,                                                                              \
@@ -185,6 +190,7 @@ struct Variant {
       (const void *)tile_kernel<NT, K, true, true>},                                             \
      {(const void *)tile_kernel_dyn<NT, K, false>, (const void *)tile_kernel_dyn<NT, K, true>,  \
       (const void *)tile_kernel_dyn<NT, K, true, true>},                                         \
+     {{nullptr, nullptr}, {nullptr, nullptr}},                                                   \
      (const void *)design_kernel<NT, K>, NT}
 // DNT x DK: the design kernel's shape over the same 32 K pixel tiles
 #define FPHO_SPLIT(NW, K, DNT, DK)                                                               \
@@ -193,6 +199,7 @@ struct Variant {
       nullptr},                                                                                  \
      {(const void *)split_kernel_dyn<NW, K, false>, (const void *)split_kernel_dyn<NW, K, true>, \
       nullptr},                                                                                  \
+     {{nullptr, nullptr}, {nullptr, nullptr}},                                                   \
      (const void *)design_kernel<DNT, DK>, DNT}
 #define FPHO_SPLIT_MINB(NW, K, MINB, DNT, DK)                                                    \
     {32 * NW, 32 * K, NW,                                                                        \
@@ -200,13 +207,25 @@ struct Variant {
       nullptr},                                                                                  \
      {(const void *)split_kernel_dyn<NW, K, false, MINB>,                                        \
       (const void *)split_kernel_dyn<NW, K, true, MINB>, nullptr},                               \
+     {{nullptr, nullptr}, {nullptr, nullptr}},                                                   \
+     (const void *)design_kernel<DNT, DK>, DNT}
+#define FPHO_SPLIT_PARTED(NW, K, MINB, DNT, DK)                                                    \
+    {32 * NW, 32 * K, NW,                                                                        \
+     {(const void *)split_kernel<NW, K, false, MINB>, (const void *)split_kernel<NW, K, true, MINB>, \
+      nullptr},                                                                                  \
+     {(const void *)split_kernel_dyn<NW, K, false, MINB>,                                        \
+      (const void *)split_kernel_dyn<NW, K, true, MINB>, nullptr},                               \
+     {{(const void *)split_kernel<NW, K, false, MINB, 2>,                                        \
+       (const void *)split_kernel<NW, K, true, MINB, 2>},                                        \
+      {(const void *)split_kernel<NW, K, false, MINB, 4>,                                        \
+       (const void *)split_kernel<NW, K, true, MINB, 4>}},                                       \
      (const void *)design_kernel<DNT, DK>, DNT}
 // Indices are part of the tuning interface (fpho_patch_set_config): new
 // shapes are appended.
 static const Variant kVariants[] = {
     FPHO_VARIANT(128, 4), FPHO_VARIANT(128, 2), FPHO_VARIANT(256, 2), FPHO_VARIANT_EXACT(64, 4),
     FPHO_VARIANT(256, 4), FPHO_VARIANT(128, 8), FPHO_VARIANT(64, 8), FPHO_VARIANT(32, 8),
-    FPHO_SPLIT(4, 8, 64, 4), FPHO_SPLIT(2, 8, 64, 4), FPHO_SPLIT(8, 8, 64, 4),
+    FPHO_SPLIT_PARTED(4, 8, 4, 64, 4), FPHO_SPLIT(2, 8, 64, 4), FPHO_SPLIT(8, 8, 64, 4),
     FPHO_SPLIT(4, 4, 32, 4), FPHO_SPLIT_MINB(4, 8, 5, 64, 4),
     FPHO_SPLIT_MINB(4, 6, 5, 32, 6),  // 192-pixel tiles, 95 registers: 5 CTAs per SM
 };
@@ -214,6 +233,7 @@ static const Variant kVariants[] = {
 #undef FPHO_VARIANT_EXACT
 #undef FPHO_SPLIT
 #undef FPHO_SPLIT_MINB
+#undef FPHO_SPLIT_PARTED
 constexpr int kNumVariants = sizeof(kVariants) / sizeof(kVariants[0]);
 
 int variant_count() { return kNumVariants; }
@@ -226,7 +246,7 @@ static std::mutex g_attr_mu;
 // per device, variant, kernel kind, form: the dynamic shared memory the
 // attribute allows, and for the persistent form the resident CTAs per SM and
 // the SM count at that size
-static size_t g_attr_set[64][kNumVariants][N_KINDS][2];
+static size_t g_attr_set[64][kNumVariants][N_KINDS][2 + N_PARTED];
 static int g_occ[64][kNumVariants][N_KINDS], g_sms[64];
 static size_t g_occ_smem[64][kNumVariants][N_KINDS];
 
@@ -249,8 +269,28 @@ int device_sms() {
     return g_sms[dev];
 }
 
+// CTAs per tile for a patch of `n_tiles`: the number p of parts that needs the
+// least time on the fullest SM, ceil(p n_tiles / SMs) parts of 1/p of a tile
+// each plus a tenth of a tile for what every part repeats (scan, staging,
+// epilogue).
+int tile_parts(int variant, int n_tiles) {
+    const Variant &V = kVariants[variant];
+    const int sms = device_sms();
+    if (!V.parts[0][0] || n_tiles > 4 * sms) return 1;
+    int best = 1;
+    double least = 1e30;
+    for (int p : {1, PARTS[0], PARTS[1]}) {
+        const double t = ((p * n_tiles + sms - 1) / sms) * (1.0 / p + 0.1);
+        if (t < least) {
+            least = t;
+            best = p;
+        }
+    }
+    return best;
+}
+
 int launch_tile_kernel(int variant, const TileArgs &A, int n_tiles, cudaStream_t stream,
-                       bool grad, const int *order, int *counter, bool exact) {
+                       bool grad, const int *order, int *counter, bool exact, int parts) {
     if (n_tiles <= 0) return FPHO_OK;
     const Variant &V = kVariants[variant];
     const bool dyn = order && counter;
@@ -263,6 +303,15 @@ int launch_tile_kernel(int variant, const TileArgs &A, int n_tiles, cudaStream_t
     int dev = 0;
     CUDA_TRY(cudaGetDevice(&dev));
     if (dev >= 64) return set_error(FPHO_ERR_LIMIT, "device ordinal %d >= 64", dev);
+    if (parts > 1) {
+        const int form = parts == PARTS[0] ? 0 : 1;
+        const void *pfn = V.parts[form][kind];
+        int rc = prepare_fn(pfn, dev, variant, kind, 2 + form, smem);
+        if (rc) return rc;
+        void *args[] = {(void *)&A};
+        CUDA_TRY(cudaLaunchKernel(pfn, dim3(n_tiles * parts), dim3(V.nt), args, smem, stream));
+        return FPHO_OK;
+    }
     int rc = prepare_fn(fn, dev, variant, kind, dyn ? 1 : 0, smem);
     if (rc) return rc;
     if (!dyn) {
@@ -367,6 +416,7 @@ void free_meta(fpho_patch *p) {
 }
 void free_plan(fpho_patch *p) {
     dfree(p->d_tiles); dfree(p->d_tbox_all); dfree(p->d_tbox_w); dfree(p->d_tile_band_start);
+    dfree(p->d_tile_misfit); dfree(p->d_runs);
     dfree(p->d_pchi2); dfree(p->d_pgrad);
     dfree(p->d_tile_cost); dfree(p->d_tile_order); dfree(p->d_tile_counter);
 }
@@ -588,15 +638,20 @@ int build_plan(fpho_patch *p, cudaStream_t s) {
         return rc;
     if ((rc = dalloc(&p->d_tbox_all, tiles.size()))) return rc;
     if ((rc = dalloc(&p->d_tbox_w, tiles.size()))) return rc;
-    if ((rc = dalloc(&p->d_pchi2, tiles.size()))) return rc;
-    if ((rc = dalloc(&p->d_pgrad, tiles.size() * (size_t)7 * p->n_sources))) return rc;
+    if ((rc = dalloc(&p->d_tile_misfit, tiles.size()))) return rc;
+    if ((rc = dalloc(&p->d_runs, tiles.size() * (size_t)(tp / 8)))) return rc;
+    p->max_parts = p->n_tiles > 4 * device_sms() ? 1 : MAX_TILE_PARTS;
+    const size_t partials = tiles.size() * p->max_parts;
+    if ((rc = dalloc(&p->d_pchi2, partials))) return rc;
+    if ((rc = dalloc(&p->d_pgrad, partials * 7 * p->n_sources))) return rc;
     if ((rc = dalloc(&p->d_tile_cost, tiles.size()))) return rc;
     if ((rc = dalloc(&p->d_tile_order, tiles.size()))) return rc;
     if ((rc = dalloc(&p->d_tile_counter, 1))) return rc;
     CUDA_TRY(cudaMemsetAsync(p->d_tile_cost, 0, sizeof(int) * std::max<size_t>(tiles.size(), 1), s));
     if (p->n_tiles > 0) {
         tile_bboxes<<<p->n_tiles, 128, 0, s>>>(make_view(p), p->d_tiles, p->d_tbox_all,
-                                              p->d_tbox_w, nullptr);
+                                              p->d_tbox_w, nullptr, p->d_tile_misfit,
+                                              p->d_runs, tp / 8);
         CUDA_TRY(cudaGetLastError());
     }
     CUDA_TRY(cudaStreamSynchronize(s));
@@ -670,7 +725,7 @@ extern "C" int fpho_patch_replace_meta(fpho_patch *p, const fpho_patch_struct *h
     if (rc) return rc;
     if (p->n_sources != old_nsrc) {
         dfree(p->d_pgrad);
-        if ((rc = dalloc(&p->d_pgrad, (size_t)std::max(p->n_tiles, 1) * 7 * p->n_sources)))
+        if ((rc = dalloc(&p->d_pgrad, (size_t)p->n_tiles * p->max_parts * 7 * p->n_sources)))
             return rc;
     }
     return refresh_struct(p, s);
@@ -866,23 +921,28 @@ int enqueue_evaluate(fpho_patch *p, const fpho_source *d_prop, double *d_chi2, f
     A.idx_cap = std::max(p->max_g, 1);
     A.err = p->d_err;
     A.pairs = p->count_pairs ? p->d_pairs : nullptr;
+    A.tile_misfit = p->d_tile_misfit;
+    A.runs = p->d_runs;
     A.test_extra_tx = p->test_extra_tx;
+    // one CTA per tile otherwise, or per part of one (the exact mode has no parts)
+    const int parts =
+        p->exact_residual ? 1 : std::min(tile_parts(p->variant, p->n_tiles), p->max_parts);
     if (p->ev_tile0) CUDA_TRY(cudaEventRecord(p->ev_tile0, s));
     int rc;
     if (ordered) {
         A.tile_cost = p->d_tile_cost;
         rc = launch_tile_kernel(p->variant, A, p->n_tiles, s, grad, p->d_tile_order,
-                                p->d_tile_counter, p->exact_residual != 0);
+                                p->d_tile_counter, p->exact_residual != 0, 1);
     } else {
         rc = launch_tile_kernel(p->variant, A, p->n_tiles, s, grad, nullptr, nullptr,
-                                p->exact_residual != 0);
+                                p->exact_residual != 0, parts);
     }
     if (rc) return rc;
     if (p->ev_tile1) CUDA_TRY(cudaEventRecord(p->ev_tile1, s));
     dim3 rg(p->n_bands, grad ? (out_stride + REDUCE_WARPS - 1) / REDUCE_WARPS : 1);
     reduce_bands<<<rg, 32 * REDUCE_WARPS, 0, s>>>(p->d_tile_band_start, p->d_pchi2, p->d_pgrad,
                                     7 * p->n_sources, d_chi2, grad ? d_dchi2 : nullptr,
-                                    out_stride, p->d_err, d_err_out);
+                                    out_stride, parts, p->d_err, d_err_out);
     CUDA_TRY(cudaGetLastError());
     return FPHO_OK;
 }

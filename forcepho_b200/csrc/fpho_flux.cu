@@ -132,7 +132,8 @@ __global__ void __launch_bounds__(NT) normal_tiles(TileArgs A, double *pnorm, in
         Yp[j] = pk(yv[0], yv[1]);
         M[j] = 0ull;
     }
-    const int n_live = scan_tile<NT, true>(A, bb, g0, g1, npsf, kept);
+    const int n_live = scan_tile<NT, true>(A, bb, g0, g1, npsf, kept,
+                                            reinterpret_cast<unsigned *>(recs), cap * GSTAGE);
     const v2 KEXP2 = pk1(KEXP), KEXPLO2 = pk1(KEXP_LO), CM24 = pk1(-1.0f / 24.0f);
     for (int c0 = 0; c0 < n_live; c0 += cap) {
         const int n = min(cap, n_live - c0);
@@ -148,7 +149,7 @@ __global__ void __launch_bounds__(NT) normal_tiles(TileArgs A, double *pnorm, in
                 r += GSTAGE;
                 flag = kept[c0 + i];
             } else {
-                design_one<KP>(Xp, Yp, M, r, flag, CM24, KEXP2, KEXPLO2);
+                design_one<KP>(Xp, Yp, M, r, CM24, KEXP2, KEXPLO2);
             }
             if ((flag & FLAG_LAST_SRC) || i == n - 1) {
                 // a source's Gaussians are contiguous in the kept list; one

@@ -42,6 +42,9 @@ struct fpho_patch {
     std::vector<int> tile_band_start;
     fpho::TileDesc *d_tiles = nullptr;
     float4 *d_tbox_all = nullptr, *d_tbox_w = nullptr;
+    int max_parts = 1;              // partial results per tile there is room for
+    int *d_tile_misfit = nullptr;   // per tile: misfit bits of its pixel runs
+    float2 *d_runs = nullptr;       // per run of 8 pixels: where it starts
     int *d_tile_band_start = nullptr;
     // tile scheduling: 0 = one CTA per tile (hardware order), 1 = persistent
     // CTAs taking tiles by decreasing cost of the previous evaluation

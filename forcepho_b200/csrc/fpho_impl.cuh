@@ -4,7 +4,7 @@
 //   gtab  float[n_gauss][32]  one 128-byte record per image Gaussian
 //                             (exposure-major, then source, then PSF component),
 //                             written by build_image_gaussians and staged into
-//                             shared memory per tile by bulk copies;
+//                             shared memory per tile;
 //   gbox  float4[n_gauss]     axis-aligned box enclosing the Gaussian's
 //                             exp-argument <= 36 ellipse (plus a safety margin),
 //                             used to cull Gaussians per pixel tile.
@@ -69,6 +69,46 @@ struct TileDesc {
     int pix_begin;  // index into the patch pixel arrays
     int count;      // valid pixels (<= tile size)
 };
+
+// ---------------------------------------------------------------- pixel runs
+// Eight consecutive pixels are a run.  In the packed order of whole
+// super-pixels every run shares one coordinate and steps by one pixel in the
+// other: y is shared where x varies fastest inside a super-pixel, x where y
+// does (the order of a pixel store).  These bits say which of the two does NOT
+// hold somewhere in a tile; pixels that do not count (no weight, so nothing
+// for the gradient; padding pixels are such) may lie anywhere.
+constexpr int MISFIT_Y = 1, MISFIT_X = 2;
+
+// One pixel's misfit bits against the first counting pixel of its run, whose
+// lane is also returned.  Called by whole warps whose lanes hold 32
+// consecutive pixels.
+__device__ __forceinline__ int run_misfit(float x, float y, bool counts, int &first) {
+    const int lane = threadIdx.x & 31, base = lane & 24;
+    const unsigned in_run = (__ballot_sync(0xffffffffu, counts) >> base) & 0xffu;
+    first = base + (in_run ? __ffs(in_run) - 1 : 0);
+    const float x0 = __shfl_sync(0xffffffffu, x, first);
+    const float y0 = __shfl_sync(0xffffffffu, y, first);
+    const float step = (float)(lane - first);
+    if (!counts) return 0;
+    return (y != y0 || x - x0 != step ? MISFIT_Y : 0) | (x != x0 || y - y0 != step ? MISFIT_X : 0);
+}
+// Where the calling lane's run starts (called as run_misfit is): the
+// coordinate along the run at its first pixel, and the shared one, both from
+// the run's first counting pixel.
+__device__ __forceinline__ float2 run_start(float x, float y, bool counts, bool shared_x) {
+    int first;
+    run_misfit(x, y, counts, first);
+    const float u = (shared_x ? y : x) - (float)(threadIdx.x & 7);
+    return make_float2(__shfl_sync(0xffffffffu, u, first),
+                       __shfl_sync(0xffffffffu, shared_x ? x : y, first));
+}
+// Bits of a tile: of its weighted pixels, and (shifted by MISFIT_ALL) of all
+// of them, which is what a residual output needs.
+constexpr int MISFIT_ALL = 2;
+// Does every run of the tile share x (and step in y)?
+__device__ __forceinline__ bool runs_share_x(int misfit) {
+    return (misfit & MISFIT_Y) && !(misfit & MISFIT_X);
+}
 
 // ---------------------------------------------------------------- 2x2 algebra
 // Row-major 2x2 matrix (a b / c d) and the operations of

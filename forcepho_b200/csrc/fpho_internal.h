@@ -25,12 +25,16 @@ bool variant_has_exact(int v);  // exact-residual kernels compiled for variant v
 int variant_split(int v);       // 0: tile_body; NW: tile_body_split with NW warps per tile
 size_t tile_smem_bytes(int variant, int live_cap, int idx_cap, int stride);
 int device_sms();  // SMs of the current device (cached)
-// One CTA per tile; or, with `order` and `counter` (both device pointers), the
+// Parts a tile's pixels are dealt to (a CTA each, a partial result each) when
+// the tiles are too few to fill the GPU evenly; at most MAX_TILE_PARTS.
+constexpr int MAX_TILE_PARTS = 4;
+int tile_parts(int variant, int n_tiles);
+// One CTA per part of a tile; or, with `order` and `counter` (both device pointers), the
 // persistent form taking tiles in that order (see order_tiles).
 // `exact` selects the exact-residual kernel (variant_has_exact must hold).
 int launch_tile_kernel(int variant, const TileArgs &A, int n_tiles, cudaStream_t stream,
                        bool grad, const int *order = nullptr, int *counter = nullptr,
-                       bool exact = false);
+                       bool exact = false, int parts = 1);
 
 PatchView make_view(const fpho_patch *p);
 

@@ -21,8 +21,12 @@ static __global__ void build_image_gaussians(PatchView pv, const fpho_source *sr
 
 // Bounding boxes of every tile: over all pixels and over pixels with
 // ierr != 0.  If n_tiles_dev is given, blocks at or beyond *n_tiles_dev exit.
+// With `misfit`, also the tile's misfit bits and its runs (`runs_per_tile` of
+// them).
 static __global__ void tile_bboxes(PatchView pv, const TileDesc *tiles, float4 *tbox_all,
-                                   float4 *tbox_w, const int *n_tiles_dev) {
+                                   float4 *tbox_w, const int *n_tiles_dev,
+                                   int *misfit = nullptr, float2 *runs = nullptr,
+                                   int runs_per_tile = 0) {
     if (n_tiles_dev && (int)blockIdx.x >= *n_tiles_dev) return;
     const TileDesc td = tiles[blockIdx.x];
     float ax0 = INFINITY, ax1 = -INFINITY, ay0 = INFINITY, ay1 = -INFINITY;
@@ -53,6 +57,29 @@ static __global__ void tile_bboxes(PatchView pv, const TileDesc *tiles, float4 *
         tbox_all[blockIdx.x] = make_float4(red[0][0], -red[1][0], red[2][0], -red[3][0]);
         tbox_w[blockIdx.x] = make_float4(red[4][0], -red[5][0], red[6][0], -red[7][0]);
     }
+    if (!misfit) return;
+    __shared__ int s_misfit;
+    if (threadIdx.x == 0) s_misfit = 0;
+    __syncthreads();
+    int bits = 0, first;
+    for (int i = threadIdx.x; i < 8 * runs_per_tile; i += blockDim.x) {  // whole warps
+        const bool ok = i < td.count;
+        const int pix = td.pix_begin + (ok ? i : 0);
+        const float x = pv.xpix[pix], y = pv.ypix[pix];
+        bits |= run_misfit(x, y, ok && pv.ierr[pix] != 0.0f, first);
+        bits |= run_misfit(x, y, ok, first) << MISFIT_ALL;
+    }
+    if (bits) atomicOr(&s_misfit, bits);
+    __syncthreads();
+    const bool shared_x = runs_share_x(s_misfit);
+    for (int i = threadIdx.x; i < 8 * runs_per_tile; i += blockDim.x) {
+        const bool ok = i < td.count;
+        const int pix = td.pix_begin + (ok ? i : 0);
+        const float2 uv = run_start(pv.xpix[pix], pv.ypix[pix], ok && pv.ierr[pix] != 0.0f,
+                                    shared_x);
+        if ((i & 7) == 0) runs[(size_t)blockIdx.x * runs_per_tile + (i >> 3)] = uv;
+    }
+    if (threadIdx.x == 0) misfit[blockIdx.x] = s_misfit;
 }
 
 // Work order for the persistent tile kernel: tiles by decreasing cost in the
@@ -142,16 +169,16 @@ constexpr int REDUCE_WARPS = 4;
 // Sum tile partials per band in double.  grid (n_bands, ceil(out_stride /
 // REDUCE_WARPS)), block 32 REDUCE_WARPS: warp w of block y sums component
 // y REDUCE_WARPS + w; block y = 0, warp 0 also sums chi2.
-// With err_out, block (0, 0) also copies the evaluation's error word there
+// A tile has `parts` partials.  With err_out, block (0, 0) also copies the evaluation's error word there
 // (beside the results, so that one transfer brings both to the host).
 static __global__ void reduce_bands(const int *tile_band_start, const double *pchi2,
                                     const float *pgrad, int stride, double *chi2_out,
-                                    float *dchi2_out, int out_stride, const int *err = nullptr,
-                                    int *err_out = nullptr) {
+                                    float *dchi2_out, int out_stride, int parts = 1,
+                                    const int *err = nullptr, int *err_out = nullptr) {
     const int b = blockIdx.x;
     if (err_out && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) *err_out = *err;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int t0 = tile_band_start[b], t1 = tile_band_start[b + 1];
+    const int t0 = parts * tile_band_start[b], t1 = parts * tile_band_start[b + 1];
     const int j = blockIdx.y * REDUCE_WARPS + w;
     if (dchi2_out && j < out_stride) {
         const double acc = j < stride ? warp_column_sum(pgrad + j, stride, t0, t1, lane) : 0.0;

@@ -49,7 +49,7 @@ constexpr int NA_K = 4;
 constexpr int NA_TILE = NA_THREADS * NA_K;
 constexpr int NA_LIVE_CAP = 256;
 
-// device status / error word bits (bit 0, a bounded bulk-copy wait that gave
+// device status / error word bits (bit 0, a bounded staging wait that gave
 // up, is set by the tile kernel itself)
 constexpr int NA_ERR_INDEX = 2;   // inconsistent band / exposure index arrays
 constexpr int NA_ERR_BOUND = 4;    // the caller's size bounds were exceeded

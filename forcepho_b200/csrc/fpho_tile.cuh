@@ -6,9 +6,8 @@
 //      overlaps the tile's pixel bounding box (provably equivalent to the
 //      reference's per-pixel `exparg > 36` skip, which is still applied to
 //      every Gaussian that can cross the threshold inside the tile);
-//   2. stage the kept 128-byte records into shared memory with cp.async.bulk
-//      (one bulk copy per record, issued by every thread of the CTA,
-//      completion on an mbarrier);
+//   2. stage the kept records into shared memory with asynchronous copies
+//      issued by every thread of the CTA (completion on an mbarrier);
 //   3. residual pass: r = data - sum_g amp G H over kept Gaussians, in the
 //      reference's Gaussian order (ComputeResidualImage, common_kernel.cc:57-83);
 //   4. chi2 per pixel in double, exactly as compute_gaussians_kernel.cc:286-293;
@@ -42,14 +41,16 @@ struct TileArgs {
     int want_residual;
     int live_cap;             // records that fit in the shared-memory stage (>= 1)
     int idx_cap;              // most image Gaussians of any exposure (kept-list capacity)
-    int *err;                 // error word (bit 0: bulk-copy wait gave up)
+    int *err;                 // error word (bit 0: a staging wait gave up)
     long long *pairs;         // optional: evaluated (pixel, Gaussian) pairs, or nullptr
+    const int *tile_misfit = nullptr; // the plan's misfit bits and runs of every tile, or nullptr
+    const float2 *runs = nullptr;     // (formed per tile then)
     int *tile_cost = nullptr; // optional: [n_tiles] kept Gaussians x pixels, written per tile
     int test_extra_tx = 0;    // test of the error path only: bytes the staging wait
                               // expects beyond those copied, so that it runs out
 };
 
-// ------------------------------------------------------------ mbarrier + bulk copy
+// ------------------------------------------------------------ mbarrier + asynchronous copies
 __device__ __forceinline__ uint32_t smem_u32(const void *p) {
     return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
@@ -71,16 +72,15 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t *bar, uint32_t parity) {
         : "memory");
     return ok != 0;
 }
-__device__ __forceinline__ void bulk_g2s(void *dst_smem, const void *src_gmem, uint32_t bytes,
-                                         uint64_t *bar) {
-    asm volatile(
-        "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-            smem_u32(dst_smem)),
-        "l"(src_gmem), "r"(bytes), "r"(smem_u32(bar))
-        : "memory");
+__device__ __forceinline__ void copy16_async(void *dst_smem, const void *src_gmem) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst_smem)),
+                 "l"(src_gmem)
+                 : "memory");
 }
-__device__ __forceinline__ void fence_proxy_async_smem() {
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+// The thread's copies so far, when they complete, arrive on the barrier; the
+// arrival is added to the phase's pending count here.
+__device__ __forceinline__ void mbar_arrive_on_copies(uint64_t *bar) {
+    asm volatile("cp.async.mbarrier.arrive.shared::cta.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 
 // Bounded wait on an mbarrier phase.  Gives up after `limit` polls, records
@@ -102,19 +102,19 @@ __device__ __forceinline__ double warp_sum_d(double v) {
 
 // ------------------------------------------------------------ shared layout
 // Dynamic shared memory of a tile CTA, in order:
-//   stage   `live_cap` staged records of the residual pass (the first
-//           MODEL_STAGE floats of each: all it reads); afterwards the same
-//           bytes hold the pixels of the gradient pass, PX_BYTES each
+//   stage   first the masks of the scan; then `live_cap` staged records of the
+//           residual pass (the
+//           first MODEL_STAGE floats of each: all it reads); then the pixels of the gradient pass, PX_BYTES each
 //           (px_block pixels at a time);
 //   kept    the kept list, one int per Gaussian of the exposure (local index
-//           << 2 | flags);
+//           << 1 | flags);
 //   wacc    per-warp gradient sums, `stride` floats each;
 //   part    split tiles only: the warps' partial models, one float per pixel.
 // The design passes stage whole records (they need the unit-flux amplitude
 // and the source index) and have neither gradient pixels nor partial models.
 constexpr int MODEL_STAGE = 16;  // floats of a record staged for the residual pass
 constexpr int GSTAGE = GREC;     // floats of a record staged for the design passes
-constexpr int PX_BYTES = 12;     // (u, -2 r ie^2) pairs and v of a gradient-pass pixel
+constexpr int PX_BYTES = 5;      // -2 r ie^2 of a pixel, the coordinates of its run of 8
 
 // Pixels of the tile that the gradient pass holds at a time: all of them,
 // unless `live_cap` is so small that they would need more than the 128 bytes
@@ -139,21 +139,25 @@ __host__ __device__ inline size_t design_smem_layout_bytes(int live_cap, int idx
 
 // Stage the first FLOATS floats of the records of kept entries [c0, c0 + n) of
 // an exposure (first record `gexp`) into `recs`, in list order, and wait for
-// them.  Every thread of the CTA issues the bulk copies of its records (one
-// copy each); issued by one warp, the copies of a stage queued behind each
-// other and the CTA spent about a fifth of each tile waiting for them.
-// Callers have finished reading `recs` (a barrier) before the call.
+// them: 16-byte asynchronous copies, consecutive threads on consecutive
+// sixteen bytes, whose completion arrives on the CTA's mbarrier (initialised
+// with a count of one, which thread 0 takes once every thread's copies are
+// issued).  One bulk copy per record, 64 bytes each, took longer: a stage of
+// 27 records 2,300 cycles.  Callers have finished reading `recs`, and the kept
+// list is complete, at a barrier before the call.
 template <int NT, int FLOATS>
 __device__ __forceinline__ void stage_records(float *recs, const float *gexp, const int *kept,
                                               int c0, int n, int extra_tx, uint64_t *mbar,
                                               uint32_t &phase, int *err) {
-    fence_proxy_async_smem();
-    if (threadIdx.x == 0)
-        mbar_arrive_expect_tx(mbar, (uint32_t)(n * FLOATS * 4 + extra_tx));
-    __syncthreads();  // the expected bytes are set before any copy can complete
-    for (int i = threadIdx.x; i < n; i += NT)
-        bulk_g2s(recs + (size_t)i * FLOATS, gexp + (size_t)(kept[c0 + i] >> 2) * GREC,
-                 FLOATS * 4, mbar);
+    constexpr int PER = FLOATS / 4;  // copies per record
+    for (int i = threadIdx.x; i < n * PER; i += NT) {
+        const int k = i / PER, part = i - k * PER;
+        copy16_async(recs + (size_t)i * 4,
+                     gexp + (size_t)(kept[c0 + k] >> 1) * GREC + 4 * part);
+    }
+    mbar_arrive_on_copies(mbar);
+    __syncthreads();  // every thread's arrival is pending before thread 0's
+    if (threadIdx.x == 0) mbar_arrive_expect_tx(mbar, (uint32_t)extra_tx);
     mbar_wait_bounded(mbar, phase, err);
     phase ^= 1u;
 }
@@ -201,8 +205,18 @@ __device__ __forceinline__ void ld2(const float *p, v2 &a, v2 &b) {
     b = t.y;
 }
 
+// What a thread's pixels share in the residual pass (see run_misfit): nothing,
+// y, or x.  The shared offset and its product with F are then formed once per
+// Gaussian instead of once per pixel pair -- 83 packed instructions for 8
+// pixels instead of 89, each result rounded exactly as without sharing.
+enum Share : int { SHARE_NONE = 0, SHARE_Y = 1, SHARE_X = 2 };
+template <int V>
+struct ShareTag {
+    static constexpr int value = V;
+};
+
 // Pass 1 for one Gaussian over the thread's KP pixel pairs: R -= amp G H.
-template <int KP, bool CUT>
+template <int KP>
 __device__ __forceinline__ void residual_pairs(const v2 (&X)[KP], const v2 (&Y)[KP], v2 (&R)[KP],
                                                v2 NXC, v2 NYC, v2 FXX, v2 FXY, v2 FYY, v2 HA,
                                                v2 HB, v2 KEXP2, v2 KEXPLO2) {
@@ -214,12 +228,10 @@ __device__ __forceinline__ void residual_pairs(const v2 (&X)[KP], const v2 (&Y)[
         const v2 Q = fma2(DY, VY, mul2(DX, VX));
         // the residual needs an unbiased exponential (see exp_neg_half)
         v2 Gp = exp_neg_half(Q, KEXP2, KEXPLO2);
-        if (CUT) {
-            float g0, g1, q0, q1;
-            unpk(Gp, g0, g1);
-            unpk(Q, q0, q1);
-            Gp = pk(q0 > FPHO_MAX_EXP_ARG ? 0.0f : g0, q1 > FPHO_MAX_EXP_ARG ? 0.0f : g1);
-        }
+        float g0, g1, q0, q1;
+        unpk(Gp, g0, g1);
+        unpk(Q, q0, q1);
+        Gp = pk(q0 > FPHO_MAX_EXP_ARG ? 0.0f : g0, q1 > FPHO_MAX_EXP_ARG ? 0.0f : g1);
         const v2 S = fma2(VY, VY, mul2(VX, VX));
         R[j] = fma2(fma2(S, HA, HB), Gp, R[j]);  // fma(S, -amp/24, -amp c0) = -amp H
     }
@@ -227,13 +239,8 @@ __device__ __forceinline__ void residual_pairs(const v2 (&X)[KP], const v2 (&Y)[
 
 // Pass 1 for two consecutive kept Gaussians a, b at once: their exponentials
 // are independent and interleave, and R is updated with a's term and then
-// b's, exactly as two calls of residual_pairs in order would.  The
-// exp-argument cut is applied to both; for a Gaussian without FLAG_CUT no
-// weighted pixel of the tile reaches 36 (and with a residual output every
-// pixel is in the tile box), so the cut changes nothing there.  (Skipping the
-// cut for pairs without FLAG_CUT, as a compile-time branch, measured slower:
-// it raised the split kernel's registers from 128 to 180.)
-template <int KP>
+// b's, exactly as two calls of residual_pairs in order would.
+template <int KP, int SH = SHARE_NONE>
 __device__ __forceinline__ void residual_pairs2(const v2 (&X)[KP], const v2 (&Y)[KP], v2 (&R)[KP],
                                                 const float *ra, const float *rb, v2 CM24,
                                                 v2 KEXP2, v2 KEXPLO2) {
@@ -250,8 +257,8 @@ __device__ __forceinline__ void residual_pairs2(const v2 (&X)[KP], const v2 (&Y)
     const v2 HAa = mul2(AMPa, CM24), HAb = mul2(AMPb, CM24);
 #pragma unroll
     for (int j = 0; j < KP; ++j) {
-        const v2 DXa = add2(X[j], NXa), DYa = add2(Y[j], NYa);
-        const v2 DXb = add2(X[j], NXb), DYb = add2(Y[j], NYb);
+        const v2 DXa = add2(X[SH == SHARE_X ? 0 : j], NXa), DYa = add2(Y[SH == SHARE_Y ? 0 : j], NYa);
+        const v2 DXb = add2(X[SH == SHARE_X ? 0 : j], NXb), DYb = add2(Y[SH == SHARE_Y ? 0 : j], NYb);
         const v2 VXa = fma2(FXYa, DYa, mul2(FXXa, DXa));
         const v2 VXb = fma2(FXYb, DYb, mul2(FXXb, DXb));
         const v2 VYa = fma2(FXYa, DXa, mul2(FYYa, DYa));
@@ -273,6 +280,21 @@ __device__ __forceinline__ void residual_pairs2(const v2 (&X)[KP], const v2 (&Y)
         const v2 Sb = fma2(VYb, VYb, mul2(VXb, VXb));
         R[j] = fma2(fma2(Sa, HAa, HBa), Ga, R[j]);
         R[j] = fma2(fma2(Sb, HAb, HBb), Gb, R[j]);
+    }
+}
+
+// Pass 1 for the staged records [i0, i1), two at a time; an odd last one is
+// paired with a record of zeros, whose term adds nothing.
+template <int KP, int SH>
+__device__ __forceinline__ void residual_range(const v2 (&X)[KP], const v2 (&Y)[KP], v2 (&R)[KP],
+                                               const float *recs, int i0, int i1,
+                                               const float *zero, v2 KEXP2, v2 KEXPLO2) {
+    const v2 CM24 = pk1(-1.0f / 24.0f);
+#pragma unroll 1
+    for (int i = i0; i < i1; i += 2) {
+        const float *r = recs + (size_t)i * MODEL_STAGE;
+        residual_pairs2<KP, SH>(X, Y, R, r, i + 1 < i1 ? r + MODEL_STAGE : zero, CM24, KEXP2,
+                                KEXPLO2);
     }
 }
 
@@ -319,41 +341,74 @@ __device__ __forceinline__ float lanesum(v2 v) {
 }
 
 // ------------------------------------------------------------ gradient pass
-// The pixels of the gradient pass in shared memory: x and the weight
-// r2 = -2 r ie^2 as pairs {x_2i, x_2i+1, r2_2i, r2_2i+1} (one 16-byte load is
-// two packed operands), and y.
+// The pixels of the gradient pass in shared memory: the weights r2 = -2 r ie^2
+// and, per run of eight pixels, where it starts: (u, v) = the coordinate along
+// the run at its first pixel and the shared one.  A tile whose runs share
+// nothing reads its coordinates from the patch's arrays instead.
 struct PixelStage {
-    float *xr;  // [2 pixels]
-    float *y;   // [pixels]
+    float *r2;       // [pixels]
+    float *ru, *rv;  // [pixels / 8]
 };
-// Eight consecutive pixels are a run.  In the packed order of whole
-// super-pixels every run shares one coordinate: y where x varies fastest
-// inside a super-pixel, x where y does (the order of a pixel store).  These
-// bits say which coordinate is NOT shared by the runs of a tile; pixels of
-// weight zero do not count (they add nothing to the gradient), and padding
-// pixels are such.
-constexpr int MISFIT_Y = 1, MISFIT_X = 2;
-
-// One pixel's misfit bits against the first weighted pixel of its run, and
-// that pixel's coordinates in place of its own where its weight is zero.
-// Called by whole warps whose lanes hold 32 consecutive pixels.
-__device__ __forceinline__ int run_misfit(float &x, float &y, bool weighted) {
-    const int base = threadIdx.x & 24;
-    const unsigned in_run = (__ballot_sync(0xffffffffu, weighted) >> base) & 0xffu;
-    const int first = base + (in_run ? __ffs(in_run) - 1 : 0);
-    const float x0 = __shfl_sync(0xffffffffu, x, first);
-    const float y0 = __shfl_sync(0xffffffffu, y, first);
-    const int bits = weighted ? (y != y0 ? MISFIT_Y : 0) | (x != x0 ? MISFIT_X : 0) : 0;
-    x = weighted ? x : x0;
-    y = weighted ? y : y0;
-    return bits;
+// Misfit bits of the pixels [p0, p0 + 32 N) of a tile, in every lane of the
+// calling warp: the plan's, or formed here where the caller has none.
+template <int N>
+__device__ __forceinline__ int tile_misfit(const TileArgs &A, const TileDesc &td, int tile,
+                                           int p0) {
+    if (A.tile_misfit) return A.tile_misfit[tile];
+    const int lane = threadIdx.x & 31;
+    int bits = 0, first;
+#pragma unroll 1
+    for (int i = 0; i < N; ++i) {
+        const int li = p0 + 32 * i + lane;
+        const bool ok = li < td.count;
+        const int pix = td.pix_begin + (ok ? li : 0);
+        const float x = A.pv.xpix[pix], y = A.pv.ypix[pix];
+        bits |= run_misfit(x, y, ok && A.pv.ierr[pix] != 0.0f, first);
+        bits |= run_misfit(x, y, ok, first) << MISFIT_ALL;
+    }
+    return __reduce_or_sync(0xffffffffu, bits);
 }
-__device__ __forceinline__ void put_pixel(const PixelStage &px, int p, float x, float y,
-                                          float r2) {
-    float *q = px.xr + 4 * (p >> 1) + (p & 1);
-    q[0] = x;
-    q[2] = r2;
-    px.y[p] = y;
+// What the residual pass may share, for threads that hold whole runs
+// (K = 8 consecutive pixels each), from a tile's misfit bits.
+template <int K>
+__device__ __forceinline__ int share_of(int misfit, bool all) {
+    if (K != 8) return SHARE_NONE;
+    if (all) misfit >>= MISFIT_ALL;
+    return !(misfit & MISFIT_Y) ? SHARE_Y : !(misfit & MISFIT_X) ? SHARE_X : SHARE_NONE;
+}
+// The shared coordinate of a thread's counting pixels in every pair (where
+// other pixels' values are neither weighted nor written).
+template <int KP>
+__device__ __forceinline__ void share_coordinate(v2 (&C)[KP], const bool (&counts)[2 * KP]) {
+    float c = lo(C[0]);
+#pragma unroll
+    for (int k = 2 * KP - 1; k >= 0; --k)
+        if (counts[k]) c = k & 1 ? hi(C[k / 2]) : lo(C[k / 2]);
+#pragma unroll
+    for (int j = 0; j < KP; ++j) C[j] = pk1(c);
+}
+// The runs of the pixels [b0, b0 + n) of a tile of TP (n a multiple of 32), by
+// the whole CTA: the plan's, or found here.
+template <int NT, int TP>
+__device__ __forceinline__ void stage_runs(const TileArgs &A, const TileDesc &td, int tile, int b0,
+                                           int n, bool shared_x, const PixelStage &px) {
+    if (A.runs) {
+        for (int r = threadIdx.x; r < n / 8; r += NT) {
+            const float2 uv = A.runs[(size_t)tile * (TP / 8) + b0 / 8 + r];
+            px.ru[r] = uv.x;
+            px.rv[r] = uv.y;
+        }
+        return;
+    }
+    for (int p = threadIdx.x; p < n; p += NT) {  // whole warps
+        const int li = b0 + p;
+        const bool ok = li < td.count;
+        const int pix = td.pix_begin + (ok ? li : 0);
+        const float2 uv = run_start(A.pv.xpix[pix], A.pv.ypix[pix],
+                                    ok && A.pv.ierr[pix] != 0.0f, shared_x);
+        px.ru[p >> 3] = uv.x;
+        px.rv[p >> 3] = uv.y;
+    }
 }
 
 // Moments of one Gaussian's weight W = r2 G over pixels: m[a][b] = sum W du^a
@@ -395,29 +450,27 @@ constexpr float E_CUT = FPHO_MAX_EXP_ARG * KEXP;  // exp-arguments above 36: E b
 // du whose coefficients are formed once per run, and the weight's moments in
 // du are summed before they meet dv: 11 packed instructions per pixel pair and
 // 26 scalar ones per run, against 29 packed ones per pair if every pixel
-// formed its own products.  SHARED_X: the runs share x (u = y).
-template <bool SHARED_X>
+// formed its own products.
 __device__ __forceinline__ void run_moments(const PixelStage &px, int r0, int r1,
                                             const LaneForm &f, Moments &m) {
-    const v2 NU = pk1(f.nu), E20 = pk1(f.e20);
+    const v2 E20 = pk1(f.e20);
 #pragma unroll 1
     for (int r = r0; r < r1; ++r) {
-        const float dv = (SHARED_X ? px.xr[16 * r] : px.y[8 * r]) + f.nv;
+        const float dv = px.rv[r] + f.nv;
         const float dv2 = dv * dv;
+        const v2 D = pk1(px.ru[r] + f.nu);
         const v2 E11 = pk1(f.e11 * dv), E02 = pk1(f.e02 * dv2);
-        v2 S0, S1, S2, S3, S4;
+        v2 R2[4], S0, S1, S2, S3, S4;
+        ld2(px.r2 + 8 * r, R2[0], R2[1]);
+        ld2(px.r2 + 8 * r + 4, R2[2], R2[3]);
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-            v2 U, R2;
-            ld2(px.xr + 16 * r + 4 * j, U, R2);
-            if (SHARED_X)
-                U = *reinterpret_cast<const unsigned long long *>(px.y + 8 * r + 2 * j);
-            const v2 DU = add2(U, NU);
+            const v2 DU = j ? add2(D, pk(2.0f * j, 2.0f * j + 1.0f)) : add2(D, pk(0.0f, 1.0f));
             float e0, e1;
             unpk(fma2(fma2(E20, DU, E11), DU, E02), e0, e1);
             const float g0 = e0 < E_CUT ? 0.0f : ex2f(e0);
             const float g1 = e1 < E_CUT ? 0.0f : ex2f(e1);
-            const v2 W = mul2(R2, pk(g0, g1));
+            const v2 W = mul2(R2[j], pk(g0, g1));
             const v2 T1 = mul2(W, DU), T2 = mul2(T1, DU), T3 = mul2(T2, DU);
             S0 = j ? add2(S0, W) : W;
             S1 = j ? add2(S1, T1) : T1;
@@ -428,27 +481,24 @@ __device__ __forceinline__ void run_moments(const PixelStage &px, int r0, int r1
         m.add(dv, dv2, lanesum(S0), lanesum(S1), lanesum(S2), lanesum(S3), lanesum(S4));
     }
 }
-// The same over the pixel pairs [i0, i1) of a tile whose runs share nothing.
-__device__ __forceinline__ void pixel_moments(const PixelStage &px, int i0, int i1,
+// The same over the pixels [p0, p1) of a tile whose runs share nothing;
+// `x` and `y` are the coordinates of the tile's first staged pixel.
+__device__ __forceinline__ void pixel_moments(const PixelStage &px, const float *x,
+                                              const float *y, int p0, int p1,
                                               const LaneForm &f, Moments &m) {
 #pragma unroll 1
-    for (int i = i0; i < i1; ++i) {
-        const float4 ur = *reinterpret_cast<const float4 *>(px.xr + 4 * i);
-        const float2 yy = *reinterpret_cast<const float2 *>(px.y + 2 * i);
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const float du = (h ? ur.y : ur.x) + f.nu, dv = (h ? yy.y : yy.x) + f.nv;
-            const float dv2 = dv * dv;
-            const float e = fmaf(fmaf(f.e20, du, f.e11 * dv), du, f.e02 * dv2);
-            const float w = (h ? ur.w : ur.z) * (e < E_CUT ? 0.0f : ex2f(e));
-            const float w1 = w * du, w2 = w1 * du, w3 = w2 * du;
-            m.add(dv, dv2, w, w1, w2, w3, w3 * du);
-        }
+    for (int p = p0; p < p1; ++p) {
+        const float du = x[p] + f.nu, dv = y[p] + f.nv;
+        const float dv2 = dv * dv;
+        const float e = fmaf(fmaf(f.e20, du, f.e11 * dv), du, f.e02 * dv2);
+        const float w = px.r2[p] * (e < E_CUT ? 0.0f : ex2f(e));
+        const float w1 = w * du, w2 = w1 * du, w3 = w2 * du;
+        m.add(dv, dv2, w, w1, w2, w3, w3 * du);
     }
 }
 
-// The gradient pass over `n_px` staged pixels: every kept Gaussian of the tile
-// in a lane of its own.
+// The gradient pass over `n_px` staged pixels, the first at index `pix` of the
+// patch's arrays: every kept Gaussian of the tile in a lane of its own.
 //
 // A lane forms the moments of its Gaussian's weight W = r2 G about the
 // Gaussian's centre; H = 1 + (|v|^2 - fxx - fyy)/24 is a quadratic in the
@@ -459,25 +509,25 @@ __device__ __forceinline__ void pixel_moments(const PixelStage &px, int i0, int 
 // Against pixels in the lanes and Gaussians in the loop (each thread forming
 // the sums of its own 8 pixels), the per-Gaussian work is done once for a
 // whole tile instead of once per 8 pixels, and per-row work once per row.
-// Work is dealt to the warps in units of (32 Gaussians, 64 pixels), in order
+// Work is dealt to the warps in units of (32 Gaussians, UNIT pixels), in order
 // and evenly, so that a kept list that is no multiple of 32 NW still keeps
 // every warp busy.
-template <int NW>
+template <int NW, int UNIT = 64>
 __device__ __forceinline__ void gradient_lanes(const TileArgs &A, const int *kept, int n_live,
-                                               int g0, const PixelStage &px, int n_px, int misfit,
-                                               float *wacc) {
+                                               int g0, const PixelStage &px, int pix, int n_px,
+                                               int misfit, float *wacc) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int nq = (n_px + 63) >> 6;                 // 64-pixel units
+    const int nq = (n_px + UNIT - 1) / UNIT;
     const int units = ((n_live + 31) >> 5) * nq;
     int left = units * (warp + 1) / NW - units * warp / NW;
     int g = units * warp / NW / nq, q = units * warp / NW - g * nq;
     float *row = wacc + warp * A.pgrad_stride;
-    const bool shared_x = (misfit & MISFIT_Y) && !(misfit & MISFIT_X);
+    const bool shared_x = runs_share_x(misfit);
     for (; left > 0; ++g, q = 0) {
         const int nm = min(left, nq - q);
         left -= nm;
         const bool alive = g * 32 + lane < n_live;
-        const int k = kept[min(g * 32 + lane, n_live - 1)] >> 2;
+        const int k = kept[min(g * 32 + lane, n_live - 1)] >> 1;
         const float4 *r4 = reinterpret_cast<const float4 *>(A.gtab + (size_t)(g0 + k) * GREC);
         const float4 ra = r4[0], rb = r4[1];
         const float fyy = reinterpret_cast<const float *>(r4)[R_FYY];
@@ -486,12 +536,11 @@ __device__ __forceinline__ void gradient_lanes(const TileArgs &A, const int *kep
         const LaneForm f = {shared_x ? ra.z : ra.x, shared_x ? ra.x : ra.z,
                             (shared_x ? fyy : fxx) * KEXP, 2.0f * KEXP * fxy,
                             (shared_x ? fxx : fyy) * KEXP};
-        if (shared_x)
-            run_moments<true>(px, 8 * q, 8 * (q + nm), f, m);
-        else if (!(misfit & MISFIT_Y))
-            run_moments<false>(px, 8 * q, 8 * (q + nm), f, m);
+        if (shared_x || !(misfit & MISFIT_Y))
+            run_moments(px, UNIT / 8 * q, UNIT / 8 * (q + nm), f, m);
         else
-            pixel_moments(px, 32 * q, 32 * (q + nm), f, m);
+            pixel_moments(px, A.pv.xpix + pix, A.pv.ypix + pix, UNIT * q,
+                          min(UNIT * (q + nm), n_px), f, m);
         // sums over W H and over W, in (x, y)
         const float c0 = reinterpret_cast<const float *>(r4)[R_C0];
         const float fuu = shared_x ? fyy : fxx, fvv = shared_x ? fxx : fyy;
@@ -552,70 +601,73 @@ __device__ __forceinline__ void gradient_lanes(const TileArgs &A, const int *kep
     }
 }
 
-// kept-list flag bits (the low two bits of each entry)
-constexpr int FLAG_CUT = 1;        // the exp-argument can exceed 36 inside the tile
-constexpr int FLAG_LAST_SRC = 2;   // last kept Gaussian of its source in the chunk
+// kept-list flag: the low bit of each entry
+constexpr int FLAG_LAST_SRC = 1;   // last kept Gaussian of its source
 
 // ------------------------------------------------------------ tile scan
-// One scan of the exposure's image Gaussians [g0, g1): the ordered list of
-// those that can reach the tile (box overlap, then the exact minimum of the
-// exp-argument over the tile box `bb`), each entry (local index << 2 | flags)
-// with FLAG_CUT when the exp-argument can exceed 36 inside the tile (its
-// maximum over the box is at a corner) and, with LAST_SRC, FLAG_LAST_SRC on the
-// last kept Gaussian of each source.  Returns the number kept; ends with the
-// list visible to the whole CTA.
+// The ordered list of the exposure's image Gaussians [g0, g1) that can reach
+// the tile (box overlap, then the exact minimum of the exp-argument over the
+// tile box `bb`), each entry its local index << 1 | flags; with LAST_SRC,
+// FLAG_LAST_SRC marks the last kept Gaussian of each source.  Returns the
+// number kept; the list is visible to the whole CTA after the next barrier
+// (at once with LAST_SRC).
+//
+// First every warp tests its share, 32 Gaussians at a time, and leaves one
+// mask word per 32 in shared memory (`mask`, `n_mask` words); the loads of a
+// Gaussian's box and record do not wait on each other, nor one group's on
+// another's, and no barrier stands between groups.  Then every warp ranks its
+// words against the words before them and writes its entries.  (With a
+// barrier pair and two dependent load latencies per NT Gaussians the scan was
+// 13% of a tile of the 20-source patch: 19,700 of 155,700 cycles.)
 template <int NT, bool LAST_SRC = false>
 __device__ __forceinline__ int scan_tile(const TileArgs &A, float4 bb, int g0, int g1, int npsf,
-                                         int *kept) {
+                                         int *kept, unsigned *mask, int n_mask) {
     constexpr int NW = NT / 32;
-    __shared__ int s_cnt[NW];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     int n_live = 0;
-    for (int base = g0; base < g1; base += NT) {
-        const int idx = base + tid;
-        bool live = false;
-        int flag = 0;
-        if (idx < g1) {
-            const float4 gb = A.gbox[idx];
-            live = !(gb.y < bb.x || gb.x > bb.y || gb.w < bb.z || gb.z > bb.w);
-            if (live) {
-                const float *r = A.gtab + (size_t)idx * GREC;
-                const float4 ra = *reinterpret_cast<const float4 *>(r);
-                const float4 rb = *reinterpret_cast<const float4 *>(r + 4);
-                live = keeps_tile(ra, rb, r[R_FYY], bb);
-                const float nxc = r[R_NXC], nyc = r[R_NYC];
-                const float fxx = r[R_FXX], fxy = r[R_FXY], fyy = r[R_FYY];
-                float qmax = 0.0f;
+    for (int b0 = g0; b0 < g1; b0 += 32 * n_mask) {
+        const int words = (min(g1 - b0, 32 * n_mask) + 31) >> 5;
+        if (b0 > g0) __syncthreads();  // the masks of the block before are read
+#pragma unroll 2
+        for (int w = warp; w < words; w += NW) {
+            const int idx = b0 + 32 * w + lane;
+            const int at = min(idx, g1 - 1);
+            const float4 gb = A.gbox[at];
+            const float *r = A.gtab + (size_t)at * GREC;
+            const float4 ra = *reinterpret_cast<const float4 *>(r);
+            const float4 rb = *reinterpret_cast<const float4 *>(r + 4);
+            const float fyy = r[R_FYY];
+            bool live = idx < g1 && !(gb.y < bb.x || gb.x > bb.y || gb.w < bb.z || gb.z > bb.w);
+            if (live) live = keeps_tile(ra, rb, fyy, bb);
+            const unsigned ball = __ballot_sync(0xffffffffu, live);
+            if (lane == 0) mask[w] = ball;
+        }
+        __syncthreads();
+        for (int w0 = 0; w0 < words; w0 += 32) {
+            const unsigned mine = w0 + lane < words ? mask[w0 + lane] : 0u;
+            int upto = __popc(mine);  // inclusive prefix sum over the 32 words
 #pragma unroll
-                for (int c = 0; c < 4; ++c) {
-                    const float dx = ((c & 1) ? bb.y : bb.x) + nxc;
-                    const float dy = ((c & 2) ? bb.w : bb.z) + nyc;
-                    qmax = fmaxf(qmax, dx * (fxx * dx + fxy * dy) + dy * (fyy * dy + fxy * dx));
-                }
-                flag = (qmax * (1.0f + CULL_REL) + CULL_ABS >= FPHO_MAX_EXP_ARG) ? FLAG_CUT : 0;
+            for (int o = 1; o < 32; o <<= 1) {
+                const int v = __shfl_up_sync(0xffffffffu, upto, o);
+                if (lane >= o) upto += v;
             }
+            const int n = min(32, words - w0);
+            for (int j = (warp - w0 % NW + NW) % NW; j < n; j += NW) {
+                const unsigned m = __shfl_sync(0xffffffffu, mine, j);
+                const int before = __shfl_sync(0xffffffffu, upto, j) - __popc(m);
+                if (m >> lane & 1u)
+                    kept[n_live + before + __popc(m & ((1u << lane) - 1u))] =
+                        (b0 - g0 + 32 * (w0 + j) + lane) << 1;
+            }
+            n_live += __shfl_sync(0xffffffffu, upto, 31);
         }
-        const unsigned ball = __ballot_sync(0xffffffffu, live);
-        if (lane == 0) s_cnt[warp] = __popc(ball);
-        __syncthreads();
-        int off = 0, tot = 0;
-#pragma unroll
-        for (int w = 0; w < NW; ++w) {
-            off += (w < warp) ? s_cnt[w] : 0;
-            tot += s_cnt[w];
-        }
-        if (live) {
-            const int at = n_live + off + __popc(ball & ((1u << lane) - 1u));
-            kept[at] = ((idx - g0) << 2) | flag;
-        }
-        n_live += tot;
-        __syncthreads();
     }
     if (!LAST_SRC) return n_live;
+    __syncthreads();
     // last kept Gaussian of each source (sources are contiguous in the list)
     for (int i = tid; i < n_live; i += NT) {
-        const int src = (kept[i] >> 2) / npsf;
-        const int nxt = (i + 1 < n_live) ? (kept[i + 1] >> 2) / npsf : -1;
+        const int src = (kept[i] >> 1) / npsf;
+        const int nxt = (i + 1 < n_live) ? (kept[i + 1] >> 1) / npsf : -1;
         if (nxt != src) kept[i] |= FLAG_LAST_SRC;
     }
     __syncthreads();
@@ -638,12 +690,14 @@ __device__ __forceinline__ void tile_body(const TileArgs &A, int tile, unsigned 
 
     constexpr int TP = NT * K;  // pixels per tile
     float *recs = reinterpret_cast<float *>(smem);
-    // kept list: exposure-local Gaussian index << 2 | FLAG_* bits
+    // kept list: exposure-local Gaussian index << 1 | FLAG_* bits
     int *kept = reinterpret_cast<int *>(smem + stage_bytes(TP, cap));
     float *wacc = reinterpret_cast<float *>(kept + A.idx_cap);
 
     __shared__ double s_chi2[NW];
     __shared__ int s_any_weight, s_misfit;
+    __shared__ __align__(16) float s_zero[MODEL_STAGE];
+    if (tid < MODEL_STAGE) s_zero[tid] = 0.0f;
 
     const TileDesc td = A.tiles[tile];
     const float4 bb = A.want_residual ? A.tbox_all[tile] : A.tbox_w[tile];
@@ -653,17 +707,18 @@ __device__ __forceinline__ void tile_body(const TileArgs &A, int tile, unsigned 
 
     for (int j = tid; j < NW * stride; j += NT) wacc[j] = 0.0f;
 
-    // ---- this thread's pixels: pair j holds local pixels tid + 2j*NT and tid + (2j+1)*NT
+    // ---- this thread's pixels: K consecutive ones, pair j holds pixels 2j and 2j + 1
     const float xmid = 0.5f * (bb.x + bb.y), ymid = 0.5f * (bb.z + bb.w);
     v2 X[KP], Y[KP], R[KP], R2[KP];
     float D[K], IE[K];
-    int any_w = 0, misfit = 0;
+    bool counts[K];
+    int any_w = 0;
 #pragma unroll
     for (int j = 0; j < KP; ++j) {
         float xs[2], ys[2];
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
-            const int li = tid + (2 * j + h) * NT;
+            const int li = tid * K + 2 * j + h;
             const bool ok = li < td.count;
             const int pix = td.pix_begin + (ok ? li : 0);
             xs[h] = ok ? A.pv.xpix[pix] : xmid;
@@ -671,60 +726,58 @@ __device__ __forceinline__ void tile_body(const TileArgs &A, int tile, unsigned 
             D[2 * j + h] = ok ? A.pv.data[pix] : 0.0f;
             IE[2 * j + h] = ok ? A.pv.ierr[pix] : 0.0f;
             any_w |= (IE[2 * j + h] != 0.0f);
-            if (GRAD) {
-                float x = xs[h], y = ys[h];
-                misfit |= run_misfit(x, y, IE[2 * j + h] != 0.0f);
-            }
+            counts[2 * j + h] = ok && (A.want_residual || IE[2 * j + h] != 0.0f);
         }
         X[j] = pk(xs[0], xs[1]);
         Y[j] = pk(ys[0], ys[1]);
         R[j] = pk(D[2 * j], D[2 * j + 1]);
     }
+    const int my_misfit = tile_misfit<K>(A, td, tile, warp * 32 * K);
     if (tid == 0) s_any_weight = s_misfit = 0;
 
     // ---- the ordered list of kept image Gaussians
-    const int n_live = scan_tile<NT>(A, bb, g0, g1, npsf, kept);
+    const int n_live = scan_tile<NT>(A, bb, g0, g1, npsf, kept,
+                                      reinterpret_cast<unsigned *>(recs),
+                                      (int)(stage_bytes(TP, cap) / 4));
     if (any_w) s_any_weight = 1;
-    if (misfit) atomicOr(&s_misfit, misfit);
+    if (my_misfit && lane == 0) atomicOr(&s_misfit, my_misfit);
     __syncthreads();
     const bool tile_has_weight = s_any_weight != 0;
+    const int misfit = s_misfit;
 
-    // ---- stage kept records [c0, c0 + n) into shared memory with bulk copies
+    // ---- stage kept records [c0, c0 + n) into shared memory
     auto stage = [&](int c0, int n) {
         stage_records<NT, MODEL_STAGE>(recs, A.gtab + (size_t)g0 * GREC, kept, c0, n,
                                        A.test_extra_tx, mbar, phase, A.err);
     };
 
     const v2 KEXP2 = pk1(KEXP), KEXPLO2 = pk1(KEXP_LO);
-    const v2 CM24 = pk1(-1.0f / 24.0f), C24 = pk1(1.0f / 24.0f);
     const int n_chunks = (n_live + cap - 1) / cap;
 
     // ------------------------------------------------------------ pass 1
-    for (int c = 0; c < n_chunks; ++c) {
-        const int c0 = c * cap, n = min(cap, n_live - c0);
-        if (c > 0) __syncthreads();  // previous chunk fully consumed
-        stage(c0, n);
-        if (EXACT) {
-            for (int i = 0; i < n; ++i) residual_exact<KP>(X, Y, R, recs + (size_t)i * MODEL_STAGE);
-            continue;
+    auto pass1 = [&](auto tag) {
+        constexpr int SH = decltype(tag)::value;
+        for (int c = 0; c < n_chunks; ++c) {
+            const int c0 = c * cap, n = min(cap, n_live - c0);
+            if (c > 0) __syncthreads();  // previous chunk fully consumed
+            stage(c0, n);
+            if constexpr (EXACT) {
+                for (int i = 0; i < n; ++i)
+                    residual_exact<KP>(X, Y, R, recs + (size_t)i * MODEL_STAGE);
+            } else {
+                residual_range<KP, SH>(X, Y, R, recs, 0, n, s_zero, KEXP2, KEXPLO2);
+            }
         }
-        int i = 0;
-        for (; i + 1 < n; i += 2)
-            residual_pairs2<KP>(X, Y, R, recs + (size_t)i * MODEL_STAGE, recs + (size_t)(i + 1) * MODEL_STAGE,
-                                CM24, KEXP2, KEXPLO2);
-        for (; i < n; ++i) {
-            const float *r = recs + (size_t)i * MODEL_STAGE;
-            v2 NXC, NYC, FXX, FXY, FYY, AMP, HB, C0;
-            ld2(r + R_NXC, NXC, NYC);
-            ld2(r + R_FXX, FXX, FXY);
-            ld2(r + R_FYY, FYY, AMP);
-            ld2(r + R_HB, HB, C0);
-            const v2 HA = mul2(AMP, CM24);
-            if (kept[c0 + i] & FLAG_CUT)
-                residual_pairs<KP, true>(X, Y, R, NXC, NYC, FXX, FXY, FYY, HA, HB, KEXP2, KEXPLO2);
-            else
-                residual_pairs<KP, false>(X, Y, R, NXC, NYC, FXX, FXY, FYY, HA, HB, KEXP2, KEXPLO2);
-        }
+    };
+    const int share = EXACT ? SHARE_NONE : share_of<K>(misfit, A.want_residual);
+    if (K == 8 && share == SHARE_Y) {
+        share_coordinate<KP>(Y, counts);
+        pass1(ShareTag<K == 8 ? SHARE_Y : SHARE_NONE>());
+    } else if (K == 8 && share == SHARE_X) {
+        share_coordinate<KP>(X, counts);
+        pass1(ShareTag<K == 8 ? SHARE_X : SHARE_NONE>());
+    } else {
+        pass1(ShareTag<SHARE_NONE>());
     }
 
     // ---- residual store, chi2 (double) and the per-pixel adjoint -2 r ie^2
@@ -737,7 +790,7 @@ __device__ __forceinline__ void tile_body(const TileArgs &A, int tile, unsigned 
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
             const int k = 2 * j + h;
-            const int li = tid + k * NT;
+            const int li = tid * K + k;
             if (A.want_residual && li < td.count) A.pv.residual[td.pix_begin + li] = r[h];
             const float ie = IE[k];
             const float rie = r[h] * ie;
@@ -757,21 +810,18 @@ __device__ __forceinline__ void tile_body(const TileArgs &A, int tile, unsigned 
     // at a time; every kept Gaussian in a lane
     if (GRAD && tile_has_weight && n_live > 0) {
         const int pxb = px_block(TP, cap);
-        const PixelStage px = {recs, recs + 2 * pxb};
-        const int fits = s_misfit;
+        const PixelStage px = {recs, recs + pxb, recs + pxb + pxb / 8};
         for (int b0 = 0; b0 < td.count; b0 += pxb) {
             __syncthreads();  // records (or the previous pixels) fully consumed
 #pragma unroll
             for (int k = 0; k < K; ++k) {
-                const int p = tid + k * NT - b0;  // whole warps are in or out of the block
-                float x = (k & 1) ? hi(X[k / 2]) : lo(X[k / 2]);
-                float y = (k & 1) ? hi(Y[k / 2]) : lo(Y[k / 2]);
-                if (p < 0 || p >= pxb) continue;
-                run_misfit(x, y, IE[k] != 0.0f);
-                put_pixel(px, p, x, y, (k & 1) ? hi(R2[k / 2]) : lo(R2[k / 2]));
+                const int p = tid * K + k - b0;
+                if (p >= 0 && p < pxb) px.r2[p] = k & 1 ? hi(R2[k / 2]) : lo(R2[k / 2]);
             }
+            stage_runs<NT, TP>(A, td, tile, b0, pxb, runs_share_x(misfit), px);
             __syncthreads();
-            gradient_lanes<NW>(A, kept, n_live, g0, px, min(pxb, td.count - b0), fits, wacc);
+            gradient_lanes<NW>(A, kept, n_live, g0, px, td.pix_begin + b0,
+                               min(pxb, td.count - b0), misfit, wacc);
         }
     }
     __syncthreads();
@@ -811,18 +861,26 @@ __device__ __forceinline__ void tile_body(const TileArgs &A, int tile, unsigned 
 // culling) while a launch has more tiles per resident CTA (a shorter tail).
 // Results are deterministic; the residual is summed in a different order from
 // tile_body's, so the two agree to rounding, not bit for bit.
+//
+// With PS > 1 a CTA takes one of PS parts of the tile's pixels (K / PS per
+// lane) and writes partial PS tile + part; the list of kept Gaussians and its
+// shares are the whole tile's, so every pixel's residual is the same bit for
+// bit.  For patches whose tiles do not fill the GPU's SMs evenly.
 __host__ __device__ inline size_t split_smem_layout_bytes(int nw, int k, int live_cap, int idx_cap,
                                                          int stride) {
     return tile_smem_layout_bytes(nw, 32 * k, live_cap, idx_cap, stride) + (size_t)nw * 32 * k * 4;
 }
 
-template <int NW, int K, bool GRAD = true>
-__device__ __forceinline__ void tile_body_split(const TileArgs &A, int tile, unsigned char *smem,
-                                                uint64_t *mbar, uint32_t &phase) {
-    static_assert(K % 2 == 0, "pixels per thread must be even (packed pairs)");
+template <int NW, int K, bool GRAD = true, int PS = 1>
+__device__ __forceinline__ void tile_body_split(const TileArgs &A, int tile, int part,
+                                                unsigned char *smem, uint64_t *mbar,
+                                                uint32_t &phase) {
+    static_assert(K % (2 * PS) == 0, "pixels per lane must be even (packed pairs)");
     constexpr int NT = 32 * NW;
-    constexpr int KP = K / 2;
-    constexpr int TP = 32 * K;  // pixels per tile
+    constexpr int KL = K / PS;  // pixels per lane
+    constexpr int KP = KL / 2;
+    constexpr int TP = 32 * K;   // pixels per tile
+    constexpr int PP = TP / PS;  // pixels of a part
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int cap = A.live_cap;
     const int stride = A.pgrad_stride;
@@ -830,48 +888,53 @@ __device__ __forceinline__ void tile_body_split(const TileArgs &A, int tile, uns
     float *recs = reinterpret_cast<float *>(smem);
     int *kept = reinterpret_cast<int *>(smem + stage_bytes(TP, cap));
     float *wacc = reinterpret_cast<float *>(kept + A.idx_cap);
-    float *part = wacc + (size_t)NW * stride;  // [NW][TP] partial models
+    float *pmodel = wacc + (size_t)NW * stride;  // [NW][PP] partial models
 
     __shared__ double s_chi2[NW];
+    __shared__ __align__(16) float s_zero[MODEL_STAGE];
+    if (tid < MODEL_STAGE) s_zero[tid] = 0.0f;
 
-    const TileDesc td = A.tiles[tile];
+    TileDesc td = A.tiles[tile];
     const float4 bb = A.want_residual ? A.tbox_all[tile] : A.tbox_w[tile];
     const int g0 = A.pv.gauss_start[td.exposure];
     const int g1 = A.pv.gauss_start[td.exposure + 1];
     const int npsf = A.pv.exp_npsf[td.exposure];
+    if (PS > 1) {  // this part's pixels
+        td.pix_begin += part * PP;
+        td.count = max(0, min(PP, td.count - part * PP));
+        if (td.count == 0) td.pix_begin -= part * PP;  // (an index that exists)
+    }
 
     for (int j = tid; j < NW * stride; j += NT) wacc[j] = 0.0f;
 
-    // ---- the tile's pixels, in every warp: pair j holds pixels lane + 64j, lane + 64j + 32
+    // ---- the pixels, in every warp: KL consecutive ones per lane
     const float xmid = 0.5f * (bb.x + bb.y), ymid = 0.5f * (bb.z + bb.w);
     v2 X[KP], Y[KP], R[KP];
-    int any_w = 0, misfit = 0;
+    bool counts[KL];
 #pragma unroll
     for (int j = 0; j < KP; ++j) {
         float xs[2], ys[2];
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
-            const int li = lane + (2 * j + h) * 32;
+            const int li = lane * KL + 2 * j + h;
             const bool ok = li < td.count;
             const int pix = td.pix_begin + (ok ? li : 0);
             xs[h] = ok ? A.pv.xpix[pix] : xmid;
             ys[h] = ok ? A.pv.ypix[pix] : ymid;
-            const bool weighted = ok && A.pv.ierr[pix] != 0.0f;
-            any_w |= weighted;
-            if (GRAD) {
-                float x = xs[h], y = ys[h];
-                misfit |= run_misfit(x, y, weighted);
-            }
+            counts[2 * j + h] = ok && (A.want_residual || A.pv.ierr[pix] != 0.0f);
         }
         X[j] = pk(xs[0], xs[1]);
         Y[j] = pk(ys[0], ys[1]);
         R[j] = 0ull;  // -model of this warp's Gaussians
     }
-    // every warp holds every pixel: no exchange
-    const bool tile_has_weight = __any_sync(0xffffffffu, any_w);
-    misfit = __reduce_or_sync(0xffffffffu, misfit);
+    const float4 wbox = A.tbox_w[tile];
+    const bool tile_has_weight = wbox.x <= wbox.y;  // the box of no pixels is empty
+    const int misfit = tile_misfit<KL>(A, td, tile, 0);
 
-    const int n_live = scan_tile<NT>(A, bb, g0, g1, npsf, kept);
+    const int n_live = scan_tile<NT>(A, bb, g0, g1, npsf, kept,
+                                      reinterpret_cast<unsigned *>(recs),
+                                      (int)(stage_bytes(TP, cap) / 4));
+    __syncthreads();  // the list is complete, the masks are read
 
     auto stage = [&](int c0, int n) {
         stage_records<NT, MODEL_STAGE>(recs, A.gtab + (size_t)g0 * GREC, kept, c0, n,
@@ -886,33 +949,29 @@ __device__ __forceinline__ void tile_body_split(const TileArgs &A, int tile, uns
     };
 
     const v2 KEXP2 = pk1(KEXP), KEXPLO2 = pk1(KEXP_LO);
-    const v2 CM24 = pk1(-1.0f / 24.0f), C24 = pk1(1.0f / 24.0f);
     const int n_chunks = (n_live + cap - 1) / cap;
 
     // ------------------------------------------------------------ pass 1
-    for (int c = 0; c < n_chunks; ++c) {
-        const int c0 = c * cap, n = min(cap, n_live - c0);
-        if (c > 0) __syncthreads();
-        stage(c0, n);
-        int i0, i1;
-        share(n, i0, i1);
-        int i = i0;
-        for (; i + 1 < i1; i += 2)
-            residual_pairs2<KP>(X, Y, R, recs + (size_t)i * MODEL_STAGE, recs + (size_t)(i + 1) * MODEL_STAGE,
-                                CM24, KEXP2, KEXPLO2);
-        for (; i < i1; ++i) {
-            const float *r = recs + (size_t)i * MODEL_STAGE;
-            v2 NXC, NYC, FXX, FXY, FYY, AMP, HB, C0;
-            ld2(r + R_NXC, NXC, NYC);
-            ld2(r + R_FXX, FXX, FXY);
-            ld2(r + R_FYY, FYY, AMP);
-            ld2(r + R_HB, HB, C0);
-            const v2 HA = mul2(AMP, CM24);
-            if (kept[c0 + i] & FLAG_CUT)
-                residual_pairs<KP, true>(X, Y, R, NXC, NYC, FXX, FXY, FYY, HA, HB, KEXP2, KEXPLO2);
-            else
-                residual_pairs<KP, false>(X, Y, R, NXC, NYC, FXX, FXY, FYY, HA, HB, KEXP2, KEXPLO2);
+    auto pass1 = [&](auto tag) {
+        constexpr int SH = decltype(tag)::value;
+        for (int c = 0; c < n_chunks; ++c) {
+            const int c0 = c * cap, n = min(cap, n_live - c0);
+            if (c > 0) __syncthreads();
+            stage(c0, n);
+            int i0, i1;
+            share(n, i0, i1);
+            residual_range<KP, SH>(X, Y, R, recs, i0, i1, s_zero, KEXP2, KEXPLO2);
         }
+    };
+    const int shared = share_of<K>(misfit, A.want_residual);
+    if (K == 8 && shared == SHARE_Y) {
+        share_coordinate<KP>(Y, counts);
+        pass1(ShareTag<K == 8 ? SHARE_Y : SHARE_NONE>());
+    } else if (K == 8 && shared == SHARE_X) {
+        share_coordinate<KP>(X, counts);
+        pass1(ShareTag<K == 8 ? SHARE_X : SHARE_NONE>());
+    } else {
+        pass1(ShareTag<SHARE_NONE>());
     }
 
     // ---- the residual: data plus the warps' partial (negative) models, in warp order
@@ -920,43 +979,42 @@ __device__ __forceinline__ void tile_body_split(const TileArgs &A, int tile, uns
     for (int j = 0; j < KP; ++j) {
         float m0, m1;
         unpk(R[j], m0, m1);
-        part[warp * TP + lane + 64 * j] = m0;
-        part[warp * TP + lane + 64 * j + 32] = m1;
+        pmodel[warp * PP + lane * KL + 2 * j] = m0;
+        pmodel[warp * PP + lane * KL + 2 * j + 1] = m1;
     }
     __syncthreads();
     // each thread finishes its share of the pixels: residual, chi2 (double) and
     // the gradient pass's pixels, over the staged records (no longer read)
-    const PixelStage px = {recs, recs + 2 * TP};
+    const PixelStage px = {recs, recs + PP, recs + PP + PP / 8};
     double chi2 = 0.0;
 #pragma unroll
-    for (int i = 0; i < (TP + NT - 1) / NT; ++i) {
+    for (int i = 0; i < (PP + NT - 1) / NT; ++i) {
         const int li = tid + i * NT;
-        if (li >= TP) break;  // whole warps
+        if (li >= PP) break;  // whole warps
         const bool ok = li < td.count;
         const int pix = td.pix_begin + (ok ? li : 0);
         const float d = ok ? A.pv.data[pix] : 0.0f;
         const float ie = ok ? A.pv.ierr[pix] : 0.0f;
         float r = d;
 #pragma unroll
-        for (int w = 0; w < NW; ++w) r += part[w * TP + li];
+        for (int w = 0; w < NW; ++w) r += pmodel[w * PP + li];
         if (A.want_residual && ok) A.pv.residual[pix] = r;
         const float rie = r * ie, die = d * ie;
         double c = ((double)rie - (double)die);
         c *= ((double)rie + (double)die);
         chi2 += (ie != 0.0f) ? c : 0.0;
-        if (GRAD) {
-            float x = ok ? A.pv.xpix[pix] : xmid, y = ok ? A.pv.ypix[pix] : ymid;
-            run_misfit(x, y, ie != 0.0f);
-            put_pixel(px, li, x, y, (ie != 0.0f) ? -2.0f * ((r * ie) * ie) : 0.0f);
-        }
+        if (GRAD) px.r2[li] = (ie != 0.0f) ? -2.0f * ((r * ie) * ie) : 0.0f;
     }
+    if (GRAD)
+        stage_runs<NT, PP>(A, td, tile * PS + part, 0, PP, runs_share_x(misfit), px);
     chi2 = warp_sum_d(chi2);
     if (lane == 0) s_chi2[warp] = chi2;
 
     // ------------------------------------------------------------ pass 2
     if (GRAD && tile_has_weight && n_live > 0) {
         __syncthreads();  // every pixel staged
-        gradient_lanes<NW>(A, kept, n_live, g0, px, td.count, misfit, wacc);
+        gradient_lanes<NW, 64 / PS>(A, kept, n_live, g0, px, td.pix_begin, td.count, misfit,
+                                    wacc);
     }
     __syncthreads();
 
@@ -965,13 +1023,13 @@ __device__ __forceinline__ void tile_body_split(const TileArgs &A, int tile, uns
         double c = 0.0;
 #pragma unroll
         for (int w = 0; w < NW; ++w) c += s_chi2[w];
-        A.pchi2[tile] = c;
+        A.pchi2[tile * PS + part] = c;
     }
     for (int j = tid; GRAD && j < stride; j += NT) {
         float v = 0.0f;
 #pragma unroll
         for (int w = 0; w < NW; ++w) v += wacc[w * stride + j];
-        A.pgrad[(size_t)tile * stride + j] = v;
+        A.pgrad[(size_t)(tile * PS + part) * stride + j] = v;
     }
     if (A.tile_cost && tid == 0) A.tile_cost[tile] = n_live * td.count;
     if (A.pairs && tid == 0) atomicAdd(reinterpret_cast<unsigned long long *>(A.pairs),
@@ -989,8 +1047,7 @@ constexpr int DESIGN_LIVE_CAP = 64;
 // accumulated, negated, into M, as residual_pairs does for the model.
 template <int KP>
 __device__ __forceinline__ void design_one(const v2 (&Xp)[KP], const v2 (&Yp)[KP], v2 (&M)[KP],
-                                           const float *r, int flag, v2 CM24, v2 KEXP2,
-                                           v2 KEXPLO2) {
+                                           const float *r, v2 CM24, v2 KEXP2, v2 KEXPLO2) {
     v2 NXC, NYC, FXX, FXY, FYY, AMP, HB, C0;
     ld2(r + R_NXC, NXC, NYC);
     ld2(r + R_FXX, FXX, FXY);
@@ -999,15 +1056,11 @@ __device__ __forceinline__ void design_one(const v2 (&Xp)[KP], const v2 (&Yp)[KP
     const v2 UA = pk1(r[R_JA_FLUX]);
     const v2 HA = mul2(UA, CM24);
     const v2 UB = mul2(pk1(-1.0f), mul2(UA, C0));
-    if (flag & FLAG_CUT)
-        residual_pairs<KP, true>(Xp, Yp, M, NXC, NYC, FXX, FXY, FYY, HA, UB, KEXP2, KEXPLO2);
-    else
-        residual_pairs<KP, false>(Xp, Yp, M, NXC, NYC, FXX, FXY, FYY, HA, UB, KEXP2, KEXPLO2);
+    residual_pairs<KP>(Xp, Yp, M, NXC, NYC, FXX, FXY, FYY, HA, UB, KEXP2, KEXPLO2);
 }
 
 // The same for two consecutive Gaussians a, b of one source at once (their
-// exponentials interleave), M updated with a's term and then b's, the cut
-// applied to both (see residual_pairs2).
+// exponentials interleave), M updated with a's term and then b's.
 template <int KP>
 __device__ __forceinline__ void design_pairs2(const v2 (&Xp)[KP], const v2 (&Yp)[KP],
                                               v2 (&M)[KP], const float *ra, const float *rb,
@@ -1092,7 +1145,8 @@ __device__ __forceinline__ void design_body(const TileArgs &A, int tile, unsigne
         Yp[j] = pk(ys[0], ys[1]);
         M[j] = 0ull;
     }
-    const int n_live = scan_tile<NT, true>(A, bb, g0, g1, npsf, kept);
+    const int n_live = scan_tile<NT, true>(A, bb, g0, g1, npsf, kept,
+                                            reinterpret_cast<unsigned *>(recs), cap * GSTAGE);
     const v2 KEXP2 = pk1(KEXP), KEXPLO2 = pk1(KEXP_LO), CM24 = pk1(-1.0f / 24.0f);
     for (int c0 = 0; c0 < n_live; c0 += cap) {
         const int n = min(cap, n_live - c0);
@@ -1108,7 +1162,7 @@ __device__ __forceinline__ void design_body(const TileArgs &A, int tile, unsigne
                 r += GSTAGE;
                 flag = kept[c0 + i];
             } else {
-                design_one<KP>(Xp, Yp, M, r, flag, CM24, KEXP2, KEXPLO2);
+                design_one<KP>(Xp, Yp, M, r, CM24, KEXP2, KEXPLO2);
             }
             if ((flag & FLAG_LAST_SRC) || i == n - 1) {
                 const int src = min((unsigned)__float_as_int(r[R_SRC]),
