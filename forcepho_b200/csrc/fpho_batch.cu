@@ -46,7 +46,9 @@ struct BandJob {
 };
 
 __global__ void batch_gaussians(const BatchPatch *bps, const int2 *expmap,
-                                const fpho_source *props) {
+                                const fpho_source *props, int *err) {
+    let_next_kernel_start();
+    if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) *err = 0;
     const int2 pe = expmap[blockIdx.y];
     const BatchPatch &bp = bps[pe.x];
     const int e = pe.y;
@@ -74,6 +76,8 @@ __global__ void __launch_bounds__(NT, MINB) batch_tiles(const TileArgs *args, co
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
+    let_next_kernel_start();
+    wait_for_earlier_kernel();
     uint32_t phase = 0;
     for (;;) {
         if (threadIdx.x == 0) s_item = atomicAdd(counter, 1);
@@ -94,6 +98,7 @@ __global__ void __launch_bounds__(NT, MINB) batch_tiles(const TileArgs *args, co
 // same per-component warp sums as reduce_bands, so a patch's batched result
 // equals its single-patch one bit for bit
 __global__ void batch_reduce(const BandJob *jobs, double *chi2, float *dchi2, int *counter) {
+    wait_for_earlier_kernel();
     const BandJob jb = jobs[blockIdx.x];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int j = blockIdx.y * REDUCE_WARPS + w;
@@ -458,12 +463,13 @@ extern "C" int fpho_batch_last_tile_ms(fpho_batch *b, float *ms) {
 
 static int batch_enqueue(fpho_batch *b, const fpho_source *d_props, double *d_chi2,
                          float *d_dchi2, cudaStream_t s) {
-    CUDA_TRY(cudaMemsetAsync(b->d_err, 0, sizeof(int), s));
     if (b->count_pairs) CUDA_TRY(cudaMemsetAsync(b->d_pairs, 0, sizeof(long long), s));
     if (b->n_exp_total > 0 && b->max_g > 0) {
         batch_gaussians<<<dim3((b->max_g + 127) / 128, b->n_exp_total), 128, 0, s>>>(
-            b->d_bps, b->d_expmap, d_props);
+            b->d_bps, b->d_expmap, d_props, b->d_err);
         CUDA_TRY(cudaGetLastError());
+    } else {
+        CUDA_TRY(cudaMemsetAsync(b->d_err, 0, sizeof(int), s));
     }
     if (b->ev0) CUDA_TRY(cudaEventRecord(b->ev0, s));
     if (b->n_work > 0) {
@@ -473,14 +479,15 @@ static int batch_enqueue(fpho_batch *b, const fpho_source *d_props, double *d_ch
         int n_work = b->n_work;
         int *counter = b->d_counter;
         void *kargs[] = {(void *)&args, (void *)&work, (void *)&n_work, (void *)&counter};
-        CUDA_TRY(cudaLaunchKernel(B.fn, dim3(b->grid), dim3(B.nt), kargs, b->smem, s));
+        CUDA_TRY(launch_dependent(B.fn, dim3(b->grid), dim3(B.nt), kargs, b->smem, s));
     }
     if (b->ev1) CUDA_TRY(cudaEventRecord(b->ev1, s));
     if (b->n_jobs > 0) {
-        batch_reduce<<<dim3(b->n_jobs, (b->max_stride + REDUCE_WARPS - 1) / REDUCE_WARPS),
-                       32 * REDUCE_WARPS, 0, s>>>(
-            b->d_jobs, d_chi2, d_dchi2, b->d_counter);
-        CUDA_TRY(cudaGetLastError());
+        void *rargs[] = {&b->d_jobs, &d_chi2, &d_dchi2, &b->d_counter};
+        CUDA_TRY(launch_dependent(
+            (const void *)batch_reduce,
+            dim3(b->n_jobs, (b->max_stride + REDUCE_WARPS - 1) / REDUCE_WARPS),
+            dim3(32 * REDUCE_WARPS), rargs, 0, s));
     }
     return FPHO_OK;
 }

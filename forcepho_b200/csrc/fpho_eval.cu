@@ -69,6 +69,7 @@ template <int NT, int K, bool GRAD, bool EXACT = false>
 __global__ void __launch_bounds__(NT) tile_kernel(TileArgs A) {
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ uint64_t mbar;
+    let_next_kernel_start();
     if (threadIdx.x == 0) {
         mbar_init(&mbar, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -94,6 +95,8 @@ __global__ void __launch_bounds__(NT) tile_kernel_dyn(TileArgs A, const int *ord
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
+    let_next_kernel_start();
+    wait_for_earlier_kernel();  // the order and the counter
     uint32_t phase = 0;
     for (;;) {
         if (threadIdx.x == 0) s_item = atomicAdd(counter, 1);
@@ -128,6 +131,7 @@ template <int NW, int K, bool GRAD, int MINB = 16 / NW, int PS = 1>
 __global__ void __launch_bounds__(32 * NW, MINB) split_kernel(TileArgs A) {
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ uint64_t mbar;
+    let_next_kernel_start();
     if (threadIdx.x == 0) {
         mbar_init(&mbar, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -148,6 +152,8 @@ __global__ void __launch_bounds__(32 * NW, MINB) split_kernel_dyn(TileArgs A, co
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
+    let_next_kernel_start();
+    wait_for_earlier_kernel();  // the order and the counter
     uint32_t phase = 0;
     for (;;) {
         if (threadIdx.x == 0) s_item = atomicAdd(counter, 1);
@@ -309,14 +315,14 @@ int launch_tile_kernel(int variant, const TileArgs &A, int n_tiles, cudaStream_t
         int rc = prepare_fn(pfn, dev, variant, kind, 2 + form, smem);
         if (rc) return rc;
         void *args[] = {(void *)&A};
-        CUDA_TRY(cudaLaunchKernel(pfn, dim3(n_tiles * parts), dim3(V.nt), args, smem, stream));
+        CUDA_TRY(launch_dependent(pfn, dim3(n_tiles * parts), dim3(V.nt), args, smem, stream));
         return FPHO_OK;
     }
     int rc = prepare_fn(fn, dev, variant, kind, dyn ? 1 : 0, smem);
     if (rc) return rc;
     if (!dyn) {
         void *args[] = {(void *)&A};
-        CUDA_TRY(cudaLaunchKernel(fn, dim3(n_tiles), dim3(V.nt), args, smem, stream));
+        CUDA_TRY(launch_dependent(fn, dim3(n_tiles), dim3(V.nt), args, smem, stream));
         return FPHO_OK;
     }
     int occ = 0, sms = 0;
@@ -335,7 +341,7 @@ int launch_tile_kernel(int variant, const TileArgs &A, int n_tiles, cudaStream_t
     if (occ < 1) return set_error(FPHO_ERR_LIMIT, "tile kernel cannot be resident (smem %zu)", smem);
     const int grid = std::min(n_tiles, occ * sms);
     void *args[] = {(void *)&A, (void *)&order, (void *)&n_tiles, (void *)&counter};
-    CUDA_TRY(cudaLaunchKernel(fn, dim3(grid), dim3(V.nt), args, smem, stream));
+    CUDA_TRY(launch_dependent(fn, dim3(grid), dim3(V.nt), args, smem, stream));
     return FPHO_OK;
 }
 
@@ -573,6 +579,21 @@ int refresh_struct(fpho_patch *p, cudaStream_t s) {
 }  // namespace
 
 namespace fpho {
+
+cudaError_t launch_dependent(const void *fn, dim3 grid, dim3 block, void **args, size_t smem,
+                             cudaStream_t s) {
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelExC(&cfg, fn, args);
+}
 
 cudaError_t pool_malloc(void **p, size_t bytes) {
     static std::once_flag once[64];
@@ -940,10 +961,11 @@ int enqueue_evaluate(fpho_patch *p, const fpho_source *d_prop, double *d_chi2, f
     if (rc) return rc;
     if (p->ev_tile1) CUDA_TRY(cudaEventRecord(p->ev_tile1, s));
     dim3 rg(p->n_bands, grad ? (out_stride + REDUCE_WARPS - 1) / REDUCE_WARPS : 1);
-    reduce_bands<<<rg, 32 * REDUCE_WARPS, 0, s>>>(p->d_tile_band_start, p->d_pchi2, p->d_pgrad,
-                                    7 * p->n_sources, d_chi2, grad ? d_dchi2 : nullptr,
-                                    out_stride, parts, p->d_err, d_err_out);
-    CUDA_TRY(cudaGetLastError());
+    const int stride = 7 * p->n_sources;
+    float *dchi2_out = grad ? d_dchi2 : nullptr;
+    void *args[] = {&p->d_tile_band_start, &p->d_pchi2, &p->d_pgrad, (void *)&stride, &d_chi2,
+                    &dchi2_out, &out_stride, (void *)&parts, &p->d_err, &d_err_out};
+    CUDA_TRY(launch_dependent((const void *)reduce_bands, rg, dim3(32 * REDUCE_WARPS), args, 0, s));
     return FPHO_OK;
 }
 

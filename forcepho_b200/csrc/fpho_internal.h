@@ -36,6 +36,12 @@ int launch_tile_kernel(int variant, const TileArgs &A, int n_tiles, cudaStream_t
                        bool grad, const int *order = nullptr, int *counter = nullptr,
                        bool exact = false, int parts = 1);
 
+// Launch of a kernel that may start while the kernel before it on the stream
+// runs; the kernel itself waits (wait_for_earlier_kernel) before it touches
+// what that one writes, or what any launch between the two of them read.
+cudaError_t launch_dependent(const void *fn, dim3 grid, dim3 block, void **args, size_t smem,
+                             cudaStream_t s);
+
 PatchView make_view(const fpho_patch *p);
 
 // Device memory of handles (patches, batches, store scratch) comes from the

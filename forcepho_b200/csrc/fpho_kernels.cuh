@@ -135,6 +135,7 @@ constexpr int PREP_THREADS = 1024;
 static __global__ void __launch_bounds__(PREP_THREADS) prepare_evaluation(
     PatchView pv, const fpho_source *src, float *gtab, float4 *gbox, const int *cost, int n_tiles,
     int *order, int *counter, int *err) {
+    let_next_kernel_start();
     if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) *err = 0;
     const int e = blockIdx.y;
     if (e == pv.n_exp) {
@@ -175,6 +176,7 @@ static __global__ void reduce_bands(const int *tile_band_start, const double *pc
                                     const float *pgrad, int stride, double *chi2_out,
                                     float *dchi2_out, int out_stride, int parts = 1,
                                     const int *err = nullptr, int *err_out = nullptr) {
+    wait_for_earlier_kernel();
     const int b = blockIdx.x;
     if (err_out && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) *err_out = *err;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;

@@ -810,6 +810,7 @@ __device__ __forceinline__ void tile_body(const TileArgs &A, int tile, unsigned 
     if (tid == 0) s_any_weight = s_misfit = 0;
 
     // ---- the ordered list of kept image Gaussians
+    wait_for_earlier_kernel();
     const int n_live = scan_tile<NT>(A, bb, g0, g1, npsf, kept,
                                       reinterpret_cast<unsigned *>(recs),
                                       (int)(stage_bytes(TP, cap) / 4));
@@ -1005,6 +1006,7 @@ __device__ __forceinline__ void tile_body_split(const TileArgs &A, int tile, int
     const bool tile_has_weight = wbox.x <= wbox.y;  // the box of no pixels is empty
     const int misfit = tile_misfit<KL>(A, td, tile, 0);
 
+    wait_for_earlier_kernel();
     const int n_live = scan_tile<NT>(A, bb, g0, g1, npsf, kept,
                                       reinterpret_cast<unsigned *>(recs),
                                       (int)(stage_bytes(TP, cap) / 4));
