@@ -94,23 +94,22 @@ __global__ void __launch_bounds__(NT, MINB) batch_tiles(const TileArgs *args, co
     }
 }
 
-// grid (n_jobs, ceil(max_stride / REDUCE_WARPS)), block 32 REDUCE_WARPS: the
-// same per-component warp sums as reduce_bands, so a patch's batched result
-// equals its single-patch one bit for bit
-__global__ void batch_reduce(const BandJob *jobs, double *chi2, float *dchi2, int *counter) {
+// grid (n_jobs, reduce_blocks(max_stride)): reduce_bands for every (patch, band)
+__global__ void __launch_bounds__(REDUCE_THREADS) batch_reduce(const BandJob *jobs, double *chi2,
+                                                               float *dchi2, int *counter) {
     wait_for_earlier_kernel();
     const BandJob jb = jobs[blockIdx.x];
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int j = blockIdx.y * REDUCE_WARPS + w;
-    if (j < jb.stride) {
-        const double acc = warp_column_sum(jb.pgrad + j, jb.stride, jb.t0, jb.t1, lane);
-        if (lane == 0) dchi2[jb.dchi2_off + j] = (float)acc;
+    if (blockIdx.y == 0) {
+        if (blockIdx.x == 0 && threadIdx.x == 0) *counter = 0;
+        const double c = chi2_sum(jb.pchi2, jb.t0, jb.t1);
+        if (threadIdx.x == 0) chi2[jb.chi2_index] = c;
+        return;
     }
-    if (blockIdx.y == 0 && w == 0) {
-        const double c = warp_column_sum(jb.pchi2, 1, jb.t0, jb.t1, lane);
-        if (lane == 0) chi2[jb.chi2_index] = c;
-    }
-    if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) *counter = 0;
+    const int c0 = 32 * (blockIdx.y - 1);
+    if (c0 >= jb.stride) return;
+    const double g = column_sums(jb.pgrad, jb.stride, jb.stride, c0, jb.t0, jb.t1);
+    const int j = c0 + (int)threadIdx.x;
+    if (threadIdx.x < 32 && j < jb.stride) dchi2[jb.dchi2_off + j] = (float)g;
 }
 
 // The tile shapes compiled for batches: (threads, pixels per tile, warps
@@ -486,8 +485,7 @@ static int batch_enqueue(fpho_batch *b, const fpho_source *d_props, double *d_ch
         void *rargs[] = {&b->d_jobs, &d_chi2, &d_dchi2, &b->d_counter};
         CUDA_TRY(launch_dependent(
             (const void *)batch_reduce,
-            dim3(b->n_jobs, (b->max_stride + REDUCE_WARPS - 1) / REDUCE_WARPS),
-            dim3(32 * REDUCE_WARPS), rargs, 0, s));
+            dim3(b->n_jobs, reduce_blocks(b->max_stride)), dim3(REDUCE_THREADS), rargs, 0, s));
     }
     return FPHO_OK;
 }

@@ -801,7 +801,7 @@ static void destroy_patch(fpho_patch *p) {
     free_plan(p);
     dfree(p->d_data); dfree(p->d_ierr); dfree(p->d_xpix); dfree(p->d_ypix); dfree(p->d_residual);
     dfree(p->d_exposure_start); dfree(p->d_exposure_N); dfree(p->d_band_start);
-    dfree(p->d_band_N); dfree(p->d_struct); dfree(p->d_io);
+    dfree(p->d_band_N); dfree(p->d_struct);
     if (p->h_io) cudaFreeHost(p->h_io);
     dfree(p->d_err); dfree(p->d_pairs); dfree(p->d_pnorm); dfree(p->d_atb);
     if (p->ev_tile0) cudaEventDestroy(p->ev_tile0);
@@ -906,10 +906,15 @@ extern "C" int fpho_patch_count_pairs(fpho_patch *p, int enable, long long *last
 
 namespace fpho {
 
-// Enqueue one evaluation with device-resident proposal and outputs.
-int enqueue_evaluate(fpho_patch *p, const fpho_source *d_prop, double *d_chi2, float *d_dchi2,
+// Sources whose proposal fits a kernel's arguments (32,764 bytes in all).
+constexpr int MAX_ARG_SOURCES = 64;
+
+// Enqueue one evaluation.  `prop` is device memory, or with `host_prop` host
+// memory read before this returns (MAX_ARG_SOURCES sources at most); the
+// outputs are memory that the device can write.
+int enqueue_evaluate(fpho_patch *p, const fpho_source *prop, double *d_chi2, float *d_dchi2,
                      int out_stride, bool want_residual, cudaStream_t s, bool grad,
-                     int *d_err_out = nullptr) {
+                     int *d_err_out = nullptr, bool host_prop = false) {
     if (want_residual && !p->d_residual)
         return set_error(FPHO_ERR_STATE,
                          "residual requested but the patch was created without one");
@@ -921,10 +926,23 @@ int enqueue_evaluate(fpho_patch *p, const fpho_source *d_prop, double *d_chi2, f
         // image Gaussians, the tile order and the error word in one launch
         dim3 grid(std::max((p->max_g + PREP_THREADS - 1) / PREP_THREADS, 1),
                   std::max(p->n_exp + (ordered ? 1 : 0), 1));
-        prepare_evaluation<<<grid, PREP_THREADS, 0, s>>>(pv, d_prop, p->d_gtab, p->d_gbox,
-                                                p->d_tile_cost, p->n_tiles,
-                                                ordered ? p->d_tile_order : nullptr,
-                                                p->d_tile_counter, p->d_err);
+        int *order = ordered ? p->d_tile_order : nullptr;
+        auto with_arg = [&](auto arg) {
+            std::memcpy(arg.s, prop, sizeof(fpho_source) * p->n_sources);
+            prepare_evaluation_arg<<<grid, PREP_THREADS, 0, s>>>(
+                arg, pv, p->d_gtab, p->d_gbox, p->d_tile_cost, p->n_tiles, order,
+                p->d_tile_counter, p->d_err);
+        };
+        if (!host_prop)
+            prepare_evaluation<<<grid, PREP_THREADS, 0, s>>>(pv, prop, p->d_gtab, p->d_gbox,
+                                                             p->d_tile_cost, p->n_tiles, order,
+                                                             p->d_tile_counter, p->d_err);
+        else if (p->n_sources <= 4)
+            with_arg(ProposalArg<4>());
+        else if (p->n_sources <= 15)
+            with_arg(ProposalArg<15>());
+        else
+            with_arg(ProposalArg<MAX_ARG_SOURCES>());
         CUDA_TRY(cudaGetLastError());
     }
     TileArgs A;
@@ -960,12 +978,12 @@ int enqueue_evaluate(fpho_patch *p, const fpho_source *d_prop, double *d_chi2, f
     }
     if (rc) return rc;
     if (p->ev_tile1) CUDA_TRY(cudaEventRecord(p->ev_tile1, s));
-    dim3 rg(p->n_bands, grad ? (out_stride + REDUCE_WARPS - 1) / REDUCE_WARPS : 1);
+    dim3 rg(p->n_bands, grad ? reduce_blocks(out_stride) : 1);
     const int stride = 7 * p->n_sources;
     float *dchi2_out = grad ? d_dchi2 : nullptr;
     void *args[] = {&p->d_tile_band_start, &p->d_pchi2, &p->d_pgrad, (void *)&stride, &d_chi2,
                     &dchi2_out, &out_stride, (void *)&parts, &p->d_err, &d_err_out};
-    CUDA_TRY(launch_dependent((const void *)reduce_bands, rg, dim3(32 * REDUCE_WARPS), args, 0, s));
+    CUDA_TRY(launch_dependent((const void *)reduce_bands, rg, dim3(REDUCE_THREADS), args, 0, s));
     return FPHO_OK;
 }
 
@@ -991,36 +1009,31 @@ extern "C" int fpho_evaluate_proposal(fpho_patch *p, const fpho_source *proposal
     if (!host_io)
         return enqueue_evaluate(p, proposal, chi2, dchi2, dchi2_stride, want_res, s, grad);
 
-    // [chi2 (n_bands doubles)][error word, 8 bytes][dchi2]
+    // Results go straight to pinned host memory, which the reduction kernel
+    // writes: [chi2 (n_bands doubles)][error word, 8 bytes][dchi2].  The
+    // proposal travels in the first launch's arguments, or, with more sources
+    // than they hold, in a transfer.
     const size_t gfloats = (size_t)p->n_bands * dchi2_stride;
     const size_t chi2_bytes = sizeof(double) * p->n_bands;
     const size_t head_bytes = chi2_bytes + 8;
     const size_t io_bytes = head_bytes + sizeof(float) * gfloats;
-    if (p->d_io_cap < io_bytes) {
-        dfree(p->d_io);
-        p->d_io_cap = 0;
-        int rc = dalloc(&p->d_io, io_bytes);
-        if (rc) return rc;
-        p->d_io_cap = io_bytes;
-    }
     if (p->h_io_cap < io_bytes) {
         if (p->h_io) cudaFreeHost(p->h_io);
         p->h_io = nullptr;
         p->h_io_cap = 0;
-        CUDA_TRY(cudaHostAlloc((void **)&p->h_io, io_bytes, cudaHostAllocDefault));
+        CUDA_TRY(cudaHostAlloc((void **)&p->h_io, io_bytes, cudaHostAllocMapped));
         p->h_io_cap = io_bytes;
     }
-    double *d_chi2 = reinterpret_cast<double *>(p->d_io);
-    int *d_err_out = reinterpret_cast<int *>(p->d_io + chi2_bytes);
-    float *d_dchi2 = reinterpret_cast<float *>(p->d_io + head_bytes);
-    CUDA_TRY(cudaMemcpyAsync(p->d_prop, proposal, sizeof(fpho_source) * n_sources,
-                             cudaMemcpyHostToDevice, s));
-    int rc = enqueue_evaluate(p, p->d_prop, d_chi2, d_dchi2, dchi2_stride, want_res, s, grad,
-                              d_err_out);
+    unsigned char *io = nullptr;  // the device's address of h_io
+    CUDA_TRY(cudaHostGetDevicePointer((void **)&io, p->h_io, 0));
+    const bool in_args = n_sources <= MAX_ARG_SOURCES;
+    if (!in_args)
+        CUDA_TRY(cudaMemcpyAsync(p->d_prop, proposal, sizeof(fpho_source) * n_sources,
+                                 cudaMemcpyHostToDevice, s));
+    int rc = enqueue_evaluate(p, in_args ? proposal : p->d_prop, reinterpret_cast<double *>(io),
+                              reinterpret_cast<float *>(io + head_bytes), dchi2_stride, want_res,
+                              s, grad, reinterpret_cast<int *>(io + chi2_bytes), in_args);
     if (rc) return rc;
-    // results and error word in one transfer into pinned memory
-    CUDA_TRY(cudaMemcpyAsync(p->h_io, p->d_io, grad ? io_bytes : head_bytes,
-                             cudaMemcpyDeviceToHost, s));
     CUDA_TRY(cudaStreamSynchronize(s));
     std::memcpy(chi2, p->h_io, chi2_bytes);
     if (grad) std::memcpy(dchi2, p->h_io + head_bytes, sizeof(float) * gfloats);

@@ -60,11 +60,8 @@ struct fpho_patch {
     double *d_pchi2 = nullptr;
     float *d_pgrad = nullptr;
     fpho_source *d_prop = nullptr;
-    // host-I/O evaluations: the results on the device, [chi2 (n_bands
-    // doubles)][error word, 8 bytes][dchi2], copied back in one transfer into
-    // a pinned staging buffer and from there to the caller's arrays
-    unsigned char *d_io = nullptr;
-    size_t d_io_cap = 0;
+    // host-I/O evaluations: pinned memory the reduction writes the results to,
+    // [chi2 (n_bands doubles)][error word, 8 bytes][dchi2]
     unsigned char *h_io = nullptr;
     size_t h_io_cap = 0;
     int *d_err = nullptr;

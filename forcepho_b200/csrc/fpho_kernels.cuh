@@ -132,9 +132,9 @@ __device__ __forceinline__ void order_tiles_body(const int *cost, int n_tiles, i
 // as wide as a standalone sort would be (its passes over the costs are
 // latency-bound), and one block covers an exposure's image Gaussians.
 constexpr int PREP_THREADS = 1024;
-static __global__ void __launch_bounds__(PREP_THREADS) prepare_evaluation(
-    PatchView pv, const fpho_source *src, float *gtab, float4 *gbox, const int *cost, int n_tiles,
-    int *order, int *counter, int *err) {
+__device__ __forceinline__ void prepare_body(const PatchView &pv, const fpho_source *src,
+                                             float *gtab, float4 *gbox, const int *cost,
+                                             int n_tiles, int *order, int *counter, int *err) {
     let_next_kernel_start();
     if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) *err = 0;
     const int e = blockIdx.y;
@@ -150,46 +150,91 @@ static __global__ void __launch_bounds__(PREP_THREADS) prepare_evaluation(
     const int s = i / npsf, p = i - s * npsf;
     build_one_gaussian(pv, src, e, s, p, gtab + (size_t)(g0 + i) * GREC, gbox + g0 + i);
 }
+static __global__ void __launch_bounds__(PREP_THREADS) prepare_evaluation(
+    PatchView pv, const fpho_source *src, float *gtab, float4 *gbox, const int *cost, int n_tiles,
+    int *order, int *counter, int *err) {
+    prepare_body(pv, src, gtab, gbox, cost, n_tiles, order, counter, err);
+}
+// The same with the proposal in the launch itself, for one that comes from
+// host memory: no transfer, and the caller's array is read when the call
+// returns.  N sources at most.
+template <int N>
+struct ProposalArg {
+    fpho_source s[N];
+};
+template <int N>
+static __global__ void __launch_bounds__(PREP_THREADS) prepare_evaluation_arg(
+    const __grid_constant__ ProposalArg<N> prop, PatchView pv, float *gtab, float4 *gbox,
+    const int *cost, int n_tiles, int *order, int *counter, int *err) {
+    prepare_body(pv, prop.s, gtab, gbox, cost, n_tiles, order, counter, err);
+}
 
-// Sum of a tile range [t0, t1) of one column (FP64): lane l adds tiles
-// t0 + l, t0 + l + 32, ... in order, then the lanes combine by a fixed
-// butterfly -- deterministic, and 32 loads in flight instead of one chain.
-template <typename T>
-__device__ __forceinline__ double warp_column_sum(const T *col, size_t step, int t0, int t1,
-                                                  int lane) {
+// Sums of tile partials in double, for reduce_bands and batch_reduce alike (a
+// patch's batched result equals its single one bit for bit): one block of
+// REDUCE_THREADS per 32 gradient components of a band and one for its chi2.
+// Component blocks: a warp reads a tile's 32 adjacent partials together and
+// takes every REDUCE_WARPS-th tile of [t0, t1); the warps' sums are added in
+// warp order, and the 32 results written together (to host memory when the
+// caller's arrays are there, where single words would each be a transfer of
+// their own).  Deterministic.
+constexpr int REDUCE_THREADS = 256, REDUCE_WARPS = REDUCE_THREADS / 32;
+// Blocks a band needs for `n` components and its chi2.
+__host__ __device__ inline int reduce_blocks(int n) { return (n + 31) / 32 + 1; }
+// Component block: sum of column c0 + lane (0 where it is >= n_cols), in warp 0.
+__device__ __forceinline__ double column_sums(const float *pgrad, int stride, int n_cols, int c0,
+                                              int t0, int t1) {
+    __shared__ double part[REDUCE_WARPS][32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int j = c0 + lane;
     double acc = 0.0;
-    for (int t = t0 + lane; t < t1; t += 32) acc += (double)col[(size_t)t * step];
+    if (j < n_cols) {
+        const float *col = pgrad + j;
+#pragma unroll 8
+        for (int t = t0 + w; t < t1; t += REDUCE_WARPS) acc += (double)col[(size_t)t * stride];
+    }
+    part[w][lane] = acc;
+    __syncthreads();
+    acc = 0.0;
+#pragma unroll
+    for (int v = 0; v < REDUCE_WARPS; ++v) acc += part[v][lane];
+    return acc;
+}
+// chi2 block: the sum over the tiles, in every thread.
+__device__ __forceinline__ double chi2_sum(const double *pchi2, int t0, int t1) {
+    __shared__ double part[REDUCE_WARPS];
+    double acc = 0.0;
+#pragma unroll 4
+    for (int t = t0 + (int)threadIdx.x; t < t1; t += REDUCE_THREADS) acc += pchi2[t];
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = acc;
+    __syncthreads();
+    acc = 0.0;
+#pragma unroll
+    for (int v = 0; v < REDUCE_WARPS; ++v) acc += part[v];
     return acc;
 }
 
-// Warps per block of reduce_bands and batch_reduce: one gradient component each.
-constexpr int REDUCE_WARPS = 4;
-
-// Sum tile partials per band in double.  grid (n_bands, ceil(out_stride /
-// REDUCE_WARPS)), block 32 REDUCE_WARPS: warp w of block y sums component
-// y REDUCE_WARPS + w; block y = 0, warp 0 also sums chi2.
-// A tile has `parts` partials.  With err_out, block (0, 0) also copies the evaluation's error word there
-// (beside the results, so that one transfer brings both to the host).
-static __global__ void reduce_bands(const int *tile_band_start, const double *pchi2,
-                                    const float *pgrad, int stride, double *chi2_out,
-                                    float *dchi2_out, int out_stride, int parts = 1,
-                                    const int *err = nullptr, int *err_out = nullptr) {
+// grid (n_bands, reduce_blocks(out_stride) or, without dchi2_out, 1).  A tile
+// has `parts` partials.  With err_out, block (0, 0) also copies the
+// evaluation's error word there.
+static __global__ void __launch_bounds__(REDUCE_THREADS) reduce_bands(
+    const int *tile_band_start, const double *pchi2, const float *pgrad, int stride,
+    double *chi2_out, float *dchi2_out, int out_stride, int parts = 1, const int *err = nullptr,
+    int *err_out = nullptr) {
     wait_for_earlier_kernel();
     const int b = blockIdx.x;
-    if (err_out && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) *err_out = *err;
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int t0 = parts * tile_band_start[b], t1 = parts * tile_band_start[b + 1];
-    const int j = blockIdx.y * REDUCE_WARPS + w;
-    if (dchi2_out && j < out_stride) {
-        const double acc = j < stride ? warp_column_sum(pgrad + j, stride, t0, t1, lane) : 0.0;
-        if (lane == 0) dchi2_out[(size_t)b * out_stride + j] = (float)acc;
+    if (blockIdx.y == 0) {
+        if (err_out && b == 0 && threadIdx.x == 0) *err_out = *err;
+        const double c = chi2_sum(pchi2, t0, t1);
+        if (threadIdx.x == 0) chi2_out[b] = c;
+        return;
     }
-    if (blockIdx.y == 0 && w == 0) {
-        const double c = warp_column_sum(pchi2, 1, t0, t1, lane);
-        if (lane == 0) chi2_out[b] = c;
-    }
+    const int c0 = 32 * (blockIdx.y - 1);
+    const double g = column_sums(pgrad, stride, stride, c0, t0, t1);
+    const int j = c0 + (int)threadIdx.x;
+    if (threadIdx.x < 32 && j < out_stride) dchi2_out[(size_t)b * out_stride + j] = (float)g;
 }
 
 }  // namespace fpho
