@@ -1070,13 +1070,14 @@ extern "C" int fpho_patch_design_matrix(fpho_patch *p, const void *dev_proposal,
                          p->n_sources);
     cudaStream_t s = (cudaStream_t)stream;
     CUDA_TRY(cudaMemsetAsync(dev_X, 0, sizeof(float) * (size_t)n_sources * p->npix, s));
-    CUDA_TRY(cudaMemsetAsync(p->d_err, 0, sizeof(int), s));
     const PatchView pv = make_view(p);
     if (p->max_g > 0) {
         dim3 grid((p->max_g + 127) / 128, p->n_exp);
         build_image_gaussians<<<grid, 128, 0, s>>>(
-            pv, static_cast<const fpho_source *>(dev_proposal), p->d_gtab, p->d_gbox);
+            pv, static_cast<const fpho_source *>(dev_proposal), p->d_gtab, p->d_gbox, p->d_err);
         CUDA_TRY(cudaGetLastError());
+    } else {
+        CUDA_TRY(cudaMemsetAsync(p->d_err, 0, sizeof(int), s));
     }
     TileArgs A;
     A.pv = pv;

@@ -7,8 +7,11 @@
 namespace fpho {
 
 // One thread per image Gaussian of exposure blockIdx.y: record + culling box.
+// Clears the error word.
 static __global__ void build_image_gaussians(PatchView pv, const fpho_source *src, float *gtab,
-                                             float4 *gbox) {
+                                             float4 *gbox, int *err) {
+    let_next_kernel_start();
+    if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) *err = 0;
     const int e = blockIdx.y;
     const int g0 = pv.gauss_start[e];
     const int n = pv.gauss_start[e + 1] - g0;

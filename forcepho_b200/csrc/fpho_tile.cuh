@@ -1137,7 +1137,7 @@ __device__ __forceinline__ void design_one(const v2 (&Xp)[KP], const v2 (&Yp)[KP
 
 // The same for two consecutive Gaussians a, b of one source at once (their
 // exponentials interleave), M updated with a's term and then b's.
-template <int KP>
+template <int KP, int SH = SHARE_NONE>
 __device__ __forceinline__ void design_pairs2(const v2 (&Xp)[KP], const v2 (&Yp)[KP],
                                               v2 (&M)[KP], const float *ra, const float *rb,
                                               v2 CM24, v2 KEXP2, v2 KEXPLO2) {
@@ -1156,8 +1156,8 @@ __device__ __forceinline__ void design_pairs2(const v2 (&Xp)[KP], const v2 (&Yp)
     const v2 UBa = mul2(pk1(-1.0f), mul2(UAa, C0a)), UBb = mul2(pk1(-1.0f), mul2(UAb, C0b));
 #pragma unroll
     for (int j = 0; j < KP; ++j) {
-        const v2 DXa = add2(Xp[j], NXa), DYa = add2(Yp[j], NYa);
-        const v2 DXb = add2(Xp[j], NXb), DYb = add2(Yp[j], NYb);
+        const v2 DXa = add2(Xp[SH == SHARE_X ? 0 : j], NXa), DYa = add2(Yp[SH == SHARE_Y ? 0 : j], NYa);
+        const v2 DXb = add2(Xp[SH == SHARE_X ? 0 : j], NXb), DYb = add2(Yp[SH == SHARE_Y ? 0 : j], NYb);
         const v2 VXa = fma2(FXYa, DYa, mul2(FXXa, DXa));
         const v2 VXb = fma2(FXYb, DYb, mul2(FXXb, DXb));
         const v2 VYa = fma2(FXYa, DXa, mul2(FYYa, DYa));
