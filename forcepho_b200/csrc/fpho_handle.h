@@ -25,7 +25,9 @@ struct fpho_patch {
           *d_residual = nullptr;
     int *d_exposure_start = nullptr, *d_exposure_N = nullptr;
     int16_t *d_band_start = nullptr, *d_band_N = nullptr;
-    // device metadata
+    // device metadata: one block, the pointers below into it
+    unsigned char *d_meta = nullptr;
+    size_t d_meta_cap = 0;
     float *d_rad2 = nullptr, *d_D = nullptr, *d_crpix = nullptr, *d_crval = nullptr,
           *d_CW = nullptr, *d_G = nullptr;
     int *d_npsf = nullptr, *d_psfgauss_start = nullptr;
@@ -60,6 +62,7 @@ struct fpho_patch {
     double *d_pchi2 = nullptr;
     float *d_pgrad = nullptr;
     fpho_source *d_prop = nullptr;
+    size_t gauss_cap = 0, prop_cap = 0;  // records of d_gtab / d_gbox, sources of d_prop
     // host-I/O evaluations: pinned memory the reduction writes the results to,
     // [chi2 (n_bands doubles)][error word, 8 bytes][dchi2]
     unsigned char *h_io = nullptr;

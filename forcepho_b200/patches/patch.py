@@ -174,6 +174,18 @@ class PatchBase:
         return np.split(arr, np.cumsum(self.band_N_pix[:-1]))
 
 
+def repeat_rows(mixtures, n):
+    """The PSF rows of every exposure for each of `n` sources: a list of
+    PSF_DTYPE arrays of one length to len(mixtures) * n * length rows,
+    exposure by exposure.  (Copied as whole words: numpy copies structured
+    rows field by field, ten times slower.)"""
+    words = np.concatenate([np.ascontiguousarray(m, dtype=PSF_DTYPE).view(np.uint32)
+                            for m in mixtures]).reshape(len(mixtures), 1, -1)
+    out = np.empty((len(mixtures), n, words.shape[2]), dtype=np.uint32)
+    out[:] = words
+    return out.reshape(-1).view(PSF_DTYPE)
+
+
 class Patch(PatchBase):
     """A patch whose per-scene metadata is packed from exposure WCSs, a PSF
     store and a Sersic spline table (forcepho/patches/patch.py:200-424:
@@ -317,7 +329,7 @@ class Patch(PatchBase):
         blocks, tiled, s = [], {}, 0
         for e in range(self.n_exp):      # every source of an exposure gets its band's rows
             if bands[e] not in tiled:
-                tiled[bands[e]] = np.tile(self.psfstore.lookup(bands[e]), ns)
+                tiled[bands[e]] = repeat_rows([self.psfstore.lookup(bands[e])], ns)
             self.psfgauss_start[e] = s
             blocks.append(tiled[bands[e]])
             s += len(tiled[bands[e]])

@@ -31,7 +31,7 @@ from dataclasses import dataclass, field
 
 import numpy as np
 
-from .patches.patch import PSF_DTYPE, PatchBase
+from .patches.patch import PSF_DTYPE, PatchBase, repeat_rows
 from .patches.device_patch import GPUPatchMixin
 from .sources import default_table, proposal_from_params
 
@@ -148,7 +148,7 @@ class SyntheticPatch(PatchBase, GPUPatchMixin):
         self.crpix = np.ascontiguousarray(full["crpix"][:, idx])
         self.crval = np.ascontiguousarray(full["crval"][:, idx])
         npsf = full["npsf"]
-        self.psfgauss = np.concatenate([np.tile(m, ns) for m in full["mix"]]).astype(PSF_DTYPE)
+        self.psfgauss = repeat_rows(full["mix"], ns)
         self.psfgauss_start = (np.arange(n_exp) * ns * npsf).astype(np.int32)
         self.coerce_arrays()
 
