@@ -17,6 +17,7 @@ import numpy as np
 from . import build as _build
 
 FPHO_OK = 0
+FPHO_ERR_STATE = 5
 FPHO_IO_HOST = 1
 FPHO_WANT_RESIDUAL = 2
 FPHO_CHI2_ONLY = 4
@@ -66,6 +67,11 @@ _SIGS = {
     "fpho_store_gather": (c_int, [c_void_p, c_int, c_void_p, c_void_p, c_void_p, ctypes.c_float,
                                   c_void_p, c_void_p, c_void_p, c_void_p, ctypes.c_int64,
                                   c_void_p, c_void_p, c_void_p]),
+    "fpho_store_gather_begin": (c_int, [c_void_p, c_int, c_void_p, c_void_p, c_int64_p,
+                                        ctypes.POINTER(ctypes.c_uint64), c_void_p]),
+    "fpho_store_gather_end": (c_int, [c_void_p, ctypes.c_uint64, c_int, c_void_p, ctypes.c_float,
+                                      c_void_p, c_void_p, c_void_p, c_void_p, ctypes.c_int64,
+                                      c_void_p, c_void_p, c_void_p]),
     "fpho_store_free": (c_int, [c_void_p]),
     "fpho_store_time_gather": (c_int, [c_void_p, c_int]),
     "fpho_store_last_gather_ms": (c_int, [c_void_p, ctypes.POINTER(ctypes.c_float)]),

@@ -663,6 +663,62 @@ cudaError_t pool_malloc(void **p, size_t bytes) {
     return e;
 }
 
+// Pinned blocks given back and not in use, a few at most, smallest need first.
+namespace {
+struct PinnedBlock {
+    void *p;
+    size_t bytes;
+};
+constexpr size_t PINNED_KEEP = 16, PINNED_KEEP_BYTES = 1 << 20;
+std::mutex g_pinned_mu;
+std::vector<PinnedBlock> g_pinned;
+}  // namespace
+
+cudaError_t pinned_get(void **p, size_t *bytes) {
+    *p = nullptr;
+    {
+        std::lock_guard<std::mutex> lk(g_pinned_mu);
+        size_t best = g_pinned.size();
+        for (size_t i = 0; i < g_pinned.size(); ++i)
+            if (g_pinned[i].bytes >= *bytes &&
+                (best == g_pinned.size() || g_pinned[i].bytes < g_pinned[best].bytes))
+                best = i;
+        if (best < g_pinned.size()) {
+            *p = g_pinned[best].p;
+            *bytes = g_pinned[best].bytes;
+            g_pinned.erase(g_pinned.begin() + best);
+            return cudaSuccess;
+        }
+    }
+    size_t n = 4096;
+    while (n < *bytes) n *= 2;
+    cudaError_t e = cudaHostAlloc(p, n, cudaHostAllocMapped | cudaHostAllocPortable);
+    if (e == cudaSuccess) {
+        void *dev = nullptr;
+        e = cudaHostGetDevicePointer(&dev, *p, 0);
+        // one address on host and device, as on every 64-bit platform
+        if (e == cudaSuccess && dev != *p) e = cudaErrorNotSupported;
+        if (e != cudaSuccess) {
+            cudaFreeHost(*p);
+            *p = nullptr;
+        }
+    }
+    if (e == cudaSuccess) *bytes = n;
+    return e;
+}
+
+void pinned_put(void *p, size_t bytes) {
+    if (!p) return;
+    {
+        std::lock_guard<std::mutex> lk(g_pinned_mu);
+        if (bytes <= PINNED_KEEP_BYTES && g_pinned.size() < PINNED_KEEP) {
+            g_pinned.push_back({p, bytes});
+            return;
+        }
+    }
+    cudaFreeHost(p);
+}
+
 void pool_free(void *p) {
     if (!p) return;
     cudaDeviceSynchronize();
@@ -852,7 +908,7 @@ static void destroy_patch(fpho_patch *p) {
     dfree(p->d_data); dfree(p->d_ierr); dfree(p->d_xpix); dfree(p->d_ypix); dfree(p->d_residual);
     dfree(p->d_exposure_start); dfree(p->d_exposure_N); dfree(p->d_band_start);
     dfree(p->d_band_N); dfree(p->d_struct);
-    if (p->h_io) cudaFreeHost(p->h_io);
+    pinned_put(p->h_io, p->h_io_cap);
     dfree(p->d_err); dfree(p->d_pairs); dfree(p->d_pnorm); dfree(p->d_atb);
     if (p->ev_tile0) cudaEventDestroy(p->ev_tile0);
     if (p->ev_tile1) cudaEventDestroy(p->ev_tile1);
@@ -1068,14 +1124,14 @@ extern "C" int fpho_evaluate_proposal(fpho_patch *p, const fpho_source *proposal
     const size_t head_bytes = chi2_bytes + 8;
     const size_t io_bytes = head_bytes + sizeof(float) * gfloats;
     if (p->h_io_cap < io_bytes) {
-        if (p->h_io) cudaFreeHost(p->h_io);
+        pinned_put(p->h_io, p->h_io_cap);
         p->h_io = nullptr;
         p->h_io_cap = 0;
-        CUDA_TRY(cudaHostAlloc((void **)&p->h_io, io_bytes, cudaHostAllocMapped));
-        p->h_io_cap = io_bytes;
+        size_t cap = io_bytes;
+        CUDA_TRY(pinned_get((void **)&p->h_io, &cap));
+        p->h_io_cap = cap;
     }
-    unsigned char *io = nullptr;  // the device's address of h_io
-    CUDA_TRY(cudaHostGetDevicePointer((void **)&io, p->h_io, 0));
+    unsigned char *io = p->h_io;
     const bool in_args = n_sources <= MAX_ARG_SOURCES;
     if (!in_args)
         CUDA_TRY(cudaMemcpyAsync(p->d_prop, proposal, sizeof(fpho_source) * n_sources,

@@ -8,26 +8,31 @@
 // (forcepho/patches/pixel_patch.py:124-198, 307-342; region tests
 // forcepho/region.py:91-116 and 168-192).  Here the super-pixel arrays of all
 // exposures stay in HBM (one 2048x2048 exposure is 32 MiB, so a B200 holds
-// thousands), and four kernels do the selection and the packing:
+// thousands), and up to four kernels do the selection and the packing:
 //
 //   store_count    one CTA per (chunk of 1024 super-pixels, exposure): the
 //                  region test of every super-pixel of the exposure's box
 //                  (the rows and columns a circle can reach, computed on the
-//                  host; the whole image for a rectangle), and the chunk's
-//                  count;
-//   store_scan     one CTA per exposure: exclusive prefix sum of its chunks'
-//                  counts, and the exposure's total (read back by the host,
-//                  which sizes the patch from it);
-//   store_compact  one CTA per (chunk, exposure): the same test and the rank
-//                  of each selected super-pixel, which goes to its place in a
-//                  list of the selected super-pixels in output order;
-//   store_copy     one thread per 4 output pixels of the list (float4 loads
-//                  and stores when the super-pixel side is even and the
+//                  host; the whole image for a rectangle), one bit each, and
+//                  the chunk's count;
+//   store_scan     one CTA per exposure of more than one chunk: exclusive
+//                  prefix sum of its chunks' counts, and the exposure's total
+//                  (read by the host, which sizes the patch from it);
+//   store_compact  one CTA per (chunk, exposure): the rank of each selected
+//                  super-pixel, which goes to its place in a list of the
+//                  selected super-pixels in output order;
+//   store_copy     one thread per 2 x 4 output pixels of the list (float4
+//                  loads and stores when the super-pixel side is even and the
 //                  outputs are 16-byte aligned), so every CTA moves data and
 //                  the stores are consecutive across each warp: fluxes minus
 //                  the background offset, inverse errors with the
 //                  signal-to-noise cap of forcepho/patches/pixel_patch.py:
 //                  176-205, and the pixel coordinates.
+//
+// A call's regions, exposure indices and offsets, and the totals it reads back,
+// are in pinned host memory that the kernels address directly: a few words per
+// CTA, against a transfer and its gap for each of nine small arrays (a gather
+// of one patch from 32 exposures took 120 us, 17 of them in kernels).
 //
 // Output order is the reference's: exposures in the order given, super-pixels
 // in row-major (x super-pixel, y super-pixel) order (numpy.where over the
@@ -45,6 +50,7 @@
 #include <new>
 #include <vector>
 
+#include "fpho_impl.cuh"
 #include "fpho_internal.h"
 
 using fpho::set_error;
@@ -58,24 +64,56 @@ using fpho::clear_error;
                              cudaGetErrorString(e_), __FILE__, __LINE__);               \
     } while (0)
 
+// The super-pixels a region can select in one exposure: rows x0..x0+nx-1,
+// columns y0..y0+ny-1 (a conservative box computed on the host; the whole
+// image when no box is known).  Visited in row-major order, which is the
+// order of the whole image restricted to the box.
+struct SpBox {
+    int x0, y0, nx, ny;
+};
+
+// A call's parameters in pinned host memory (addresses valid on the device).
+// What a CTA of a kernel reads of them is one aligned record: a read of host
+// memory takes a microsecond or two, and their rate bounds a call over a
+// thousand exposures (with six reads per CTA the
+// list of 32 patches' super-pixels took 16 us instead of 8).
+struct alignas(128) CountPar {
+    fpho_region region;
+    uint16_t x0, y0, nx, ny;  // box (sides are below 32768)
+};
+struct alignas(32) PackPar {
+    int exposure;  // of the store
+    int base;      // selected super-pixels before this exposure
+    float bg;      // background level
+    int reserved;
+    SpBox box;
+};
+static_assert(sizeof(CountPar) == 128 && sizeof(PackPar) == 32, "one read each");
+struct Params {
+    CountPar *count;
+    PackPar *pack;
+    int *totals;    // selected super-pixels of exposure e, written by the kernels
+};
+
 struct fpho_store {
     int nsx = 0, nsy = 0, s = 0, s2 = 0;
     int cap = 0, n = 0;
     size_t exp_floats = 0;            // nsx * nsy * 2 s^2
     float *d_pix = nullptr;           // [cap][nsx][nsy][2 s^2]
     // per-call scratch, grown on demand
-    int scratch_exp = 0;
-    int *d_chunk = nullptr;           // [scratch_exp][n_chunks]
-    int *d_total = nullptr;           // [scratch_exp]
-    int *d_exps = nullptr;            // [scratch_exp]
-    int *d_spbase = nullptr;          // [scratch_exp] selected super-pixels before exposure e
-    int *d_box = nullptr;             // [scratch_exp][4] super-pixel box of each exposure
+    int scratch_exp = 0;              // exposures h_par has room for
+    int *d_chunk = nullptr;           // [n_exp][chunks]
+    unsigned *d_flags = nullptr;      // [n_exp][chunks][32]: a bit per super-pixel
+    size_t chunk_cap = 0;             // n_exp x chunks there is room for
     int grid_chunks = 1;              // chunks per exposure of the last count pass
     int *d_list_sp = nullptr;         // [list_cap] selected super-pixels in output order
-    int *d_list_exp = nullptr;        // [list_cap] their position in the exposure list
+    int *d_list_exp = nullptr;        // [list_cap] their exposure
+    float *d_list_bg = nullptr;       // [list_cap] and its background level
     size_t list_cap = 0;
-    float *d_bg = nullptr;            // [scratch_exp]
-    fpho_region *d_regions = nullptr; // [scratch_exp]
+    unsigned char *h_par = nullptr;   // pinned: the call's parameters and totals (Params)
+    size_t h_par_bytes = 0;
+    Params par = {};                  // where they are
+    unsigned long long serial = 0;    // count passes so far
     // optional CUDA-event timing of the gather kernel
     bool time_gather = false;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
@@ -139,14 +177,6 @@ __device__ bool superpixel_selected(const fpho_region &R, int sx, int sy, int s)
     return in;
 }
 
-// The super-pixels a region can select in one exposure: rows x0..x0+nx-1,
-// columns y0..y0+ny-1 (a conservative box computed on the host; the whole
-// image when no box is known).  Visited in row-major order, which is the
-// order of the whole image restricted to the box.
-struct SpBox {
-    int x0, y0, nx, ny;
-};
-
 // Flags of this thread's 4 consecutive super-pixels of the chunk of the box
 // (bit j set if box position chunk*1024 + 4*tid + j is selected).
 __device__ unsigned thread_flags(const fpho_region &R, const SpBox &B, int chunk, int s) {
@@ -194,23 +224,35 @@ __device__ int block_exclusive_scan(int v, int *total) {
 }
 
 __global__ void __launch_bounds__(kThreads)
-store_count(const fpho_region *regions, const SpBox *boxes, int s, int n_chunks,
-            int *chunk_count) {
+store_count(Params P, int s, int n_chunks, int *chunk_count, unsigned *flags) {
+    __shared__ CountPar C;
+    fpho::let_next_kernel_start();
     const int e = blockIdx.y, chunk = blockIdx.x;
-    const SpBox B = boxes[e];
-    if (chunk >= box_chunks(B)) {
-        if (threadIdx.x == 0) chunk_count[(size_t)e * n_chunks + chunk] = 0;
-        return;
-    }
-    const unsigned f = thread_flags(regions[e], B, chunk, s);
+    if (threadIdx.x < 32)
+        reinterpret_cast<int *>(&C)[threadIdx.x] =
+            reinterpret_cast<const int *>(P.count + e)[threadIdx.x];
+    __syncthreads();
+    const fpho_region &R = C.region;
+    const SpBox B = {C.x0, C.y0, C.nx, C.ny};
+    const size_t at = (size_t)e * n_chunks + chunk;
+    const unsigned f = chunk < box_chunks(B) ? thread_flags(R, B, chunk, s) : 0u;
     const int c = __syncthreads_count(f & 1u) + __syncthreads_count(f & 2u) +
                   __syncthreads_count(f & 4u) + __syncthreads_count(f & 8u);
-    if (threadIdx.x == 0) chunk_count[(size_t)e * n_chunks + chunk] = c;
+#pragma unroll
+    for (int j = 0; j < kPerThread; ++j) {
+        const unsigned w = __ballot_sync(0xffffffffu, f >> j & 1u);
+        if ((threadIdx.x & 31) == j) flags[at * 32 + (threadIdx.x >> 5) * kPerThread + j] = w;
+    }
+    if (threadIdx.x == 0) {
+        chunk_count[at] = n_chunks == 1 ? 0 : c;  // a single chunk's offset is 0
+        if (n_chunks == 1) P.totals[e] = c;
+    }
 }
 
 // In place: counts -> exclusive offsets within the exposure; total per exposure.
 __global__ void __launch_bounds__(kThreads)
-store_scan(int n_chunks, int *chunk_count, int *total) {
+store_scan(Params P, int n_chunks, int *chunk_count) {
+    fpho::wait_for_earlier_kernel();
     int *c = chunk_count + (size_t)blockIdx.x * n_chunks;
     int carry = 0;
     for (int i0 = 0; i0 < n_chunks; i0 += kThreads) {
@@ -221,20 +263,28 @@ store_scan(int n_chunks, int *chunk_count, int *total) {
         if (i < n_chunks) c[i] = carry + ex;
         carry += t;
     }
-    if (threadIdx.x == 0) total[blockIdx.x] = carry;
+    if (threadIdx.x == 0) P.totals[blockIdx.x] = carry;
 }
 
 __global__ void __launch_bounds__(kThreads)
-store_compact(const fpho_region *regions, const SpBox *boxes, const int *chunk_off,
-              const int *spbase, int nsy, int s, int n_chunks, int *list_sp, int *list_exp) {
+store_compact(Params P, const int *chunk_off, const unsigned *flags, int nsy, int n_chunks,
+              int *list_sp, int *list_exp, float *list_bg) {
+    __shared__ PackPar C;
+    fpho::let_next_kernel_start();
     const int e = blockIdx.y, chunk = blockIdx.x;
-    const SpBox B = boxes[e];
-    if (chunk >= box_chunks(B)) return;
-    const unsigned f = thread_flags(regions[e], B, chunk, s);
+    const size_t at = (size_t)e * n_chunks + chunk;
+    if (threadIdx.x < 8)
+        reinterpret_cast<int *>(&C)[threadIdx.x] =
+            reinterpret_cast<const int *>(P.pack + e)[threadIdx.x];
+    const unsigned *fw = flags + at * 32 + (threadIdx.x >> 5) * kPerThread;
+    unsigned f = 0;
+#pragma unroll
+    for (int j = 0; j < kPerThread; ++j) f |= (fw[j] >> (threadIdx.x & 31) & 1u) << j;
     int n_sel;
-    const int r = block_exclusive_scan(__popc(f), &n_sel);
+    const int r = block_exclusive_scan(__popc(f), &n_sel);  // (a barrier: C is there)
     if (n_sel == 0) return;
-    const long long o = (long long)spbase[e] + chunk_off[(size_t)e * n_chunks + chunk] + r;
+    const SpBox B = C.box;
+    const long long o = (long long)C.base + chunk_off[at] + r;
     const int base = chunk * fpho_store::kChunk + threadIdx.x * kPerThread;
     int q = 0;
 #pragma unroll
@@ -242,7 +292,8 @@ store_compact(const fpho_region *regions, const SpBox *boxes, const int *chunk_o
         if (f & (1u << j)) {
             const int b = base + j;
             list_sp[o + q] = (B.x0 + b / B.ny) * nsy + (B.y0 + b % B.ny);
-            list_exp[o + q] = e;
+            list_exp[o + q] = C.exposure;
+            list_bg[o + q] = C.bg;
             ++q;
         }
 }
@@ -253,47 +304,67 @@ __device__ __forceinline__ void pack_pixel(float &d, float &ie, float b, bool ha
     if (max_snr > 0.f && ie > 0.f && __fmul_rn(d, ie) > max_snr) ie = __fdiv_rn(max_snr, d);
 }
 
-// VEC: 4 consecutive output pixels per thread (s^2 % 4 == 0, outputs 16-byte
-// aligned); otherwise one.  Output pixel p belongs to list entry p / s^2.
-template <bool VEC>
+// VEC: 4 consecutive output pixels per item (s^2 % 4 == 0, outputs 16-byte
+// aligned); otherwise one.  Output pixel p belongs to list entry p / s^2.  A
+// thread takes two items, a CTA's width apart, all loads first.  S: the
+// super-pixel side at compile time, or 0 (the divisions by it are then shifts).
+// Bound by memory: 15 M pixels, 362 MB, in 62 us, 0.90 of a plain copy's rate.
+template <bool VEC, int S>
 __global__ void __launch_bounds__(kThreads)
-store_copy(const float *__restrict__ pix, size_t exp_floats, const int *__restrict__ exps,
-           const int *__restrict__ list_sp, const int *__restrict__ list_exp, long long n_items,
-           const float *__restrict__ bg, float max_snr, int nsy, int s,
-           float *__restrict__ data, float *__restrict__ ierr, float *__restrict__ xpix,
-           float *__restrict__ ypix) {
-    const long long g = (long long)blockIdx.x * kThreads + threadIdx.x;
-    if (g >= n_items) return;
-    const int s2 = s * s;
-    const long long p = VEC ? g * 4 : g;
-    const long long j = p / s2;
-    const int k = (int)(p - j * s2);
-    const int e = list_exp[j], sp = list_sp[j];
-    const float *src = pix + (size_t)exps[e] * exp_floats + (size_t)sp * 2 * s2;
-    const float b = bg ? bg[e] : 0.f;
-    const int x0 = (sp / nsy) * s, y0 = (sp % nsy) * s;
-    if (VEC) {
-        float4 d = *reinterpret_cast<const float4 *>(src + k);
-        float4 ie = *reinterpret_cast<const float4 *>(src + s2 + k);
-        pack_pixel(d.x, ie.x, b, bg != nullptr, max_snr);
-        pack_pixel(d.y, ie.y, b, bg != nullptr, max_snr);
-        pack_pixel(d.z, ie.z, b, bg != nullptr, max_snr);
-        pack_pixel(d.w, ie.w, b, bg != nullptr, max_snr);
-        *reinterpret_cast<float4 *>(data + p) = d;
-        *reinterpret_cast<float4 *>(ierr + p) = ie;
-        *reinterpret_cast<float4 *>(xpix + p) =
-            make_float4((float)(x0 + k / s), (float)(x0 + (k + 1) / s), (float)(x0 + (k + 2) / s),
-                        (float)(x0 + (k + 3) / s));
-        *reinterpret_cast<float4 *>(ypix + p) =
-            make_float4((float)(y0 + k % s), (float)(y0 + (k + 1) % s), (float)(y0 + (k + 2) % s),
-                        (float)(y0 + (k + 3) % s));
-    } else {
-        float d = src[k], ie = src[s2 + k];
-        pack_pixel(d, ie, b, bg != nullptr, max_snr);
-        data[p] = d;
-        ierr[p] = ie;
-        xpix[p] = (float)(x0 + k / s);
-        ypix[p] = (float)(y0 + k % s);
+store_copy(const float *__restrict__ pix, size_t exp_floats, const int *__restrict__ list_sp,
+           const int *__restrict__ list_exp, const float *__restrict__ list_bg, unsigned n_items,
+           bool has_bg, float max_snr, unsigned nsy, unsigned side, float *__restrict__ data,
+           float *__restrict__ ierr, float *__restrict__ xpix, float *__restrict__ ypix) {
+    constexpr int N = 2;
+    const unsigned s = S ? S : side, s2 = s * s;
+    const unsigned g0 = blockIdx.x * (N * kThreads) + threadIdx.x;
+    fpho::wait_for_earlier_kernel();
+    unsigned k[N], sp[N];
+    float b[N];
+    float4 d[N], ie[N];
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+        const unsigned g = g0 + i * kThreads;
+        if (g >= n_items) continue;
+        const unsigned p = VEC ? g * 4 : g, j = p / s2;
+        k[i] = p - j * s2;
+        sp[i] = (unsigned)list_sp[j];
+        b[i] = list_bg[j];
+        const float *src =
+            pix + (size_t)list_exp[j] * exp_floats + (size_t)sp[i] * 2 * s2 + k[i];
+        if (VEC) {
+            d[i] = *reinterpret_cast<const float4 *>(src);
+            ie[i] = *reinterpret_cast<const float4 *>(src + s2);
+        } else {
+            d[i].x = src[0];
+            ie[i].x = src[s2];
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+        const unsigned g = g0 + i * kThreads;
+        if (g >= n_items) continue;
+        const unsigned p = VEC ? g * 4 : g;
+        const unsigned x0 = sp[i] / nsy * s, y0 = sp[i] % nsy * s, q = k[i];
+        pack_pixel(d[i].x, ie[i].x, b[i], has_bg, max_snr);
+        if (VEC) {
+            pack_pixel(d[i].y, ie[i].y, b[i], has_bg, max_snr);
+            pack_pixel(d[i].z, ie[i].z, b[i], has_bg, max_snr);
+            pack_pixel(d[i].w, ie[i].w, b[i], has_bg, max_snr);
+            *reinterpret_cast<float4 *>(data + p) = d[i];
+            *reinterpret_cast<float4 *>(ierr + p) = ie[i];
+            *reinterpret_cast<float4 *>(xpix + p) =
+                make_float4((float)(x0 + q / s), (float)(x0 + (q + 1) / s),
+                            (float)(x0 + (q + 2) / s), (float)(x0 + (q + 3) / s));
+            *reinterpret_cast<float4 *>(ypix + p) =
+                make_float4((float)(y0 + q % s), (float)(y0 + (q + 1) % s),
+                            (float)(y0 + (q + 2) % s), (float)(y0 + (q + 3) % s));
+        } else {
+            data[p] = d[i].x;
+            ierr[p] = ie[i].x;
+            xpix[p] = (float)(x0 + q / s);
+            ypix[p] = (float)(y0 + q % s);
+        }
     }
 }
 
@@ -316,19 +387,33 @@ void dfree(T *&p) {
     p = nullptr;
 }
 
-int ensure_scratch(fpho_store *st, int n_exp) {
+// Room for a call of n_exp exposures, `chunks` each.
+int ensure_scratch(fpho_store *st, int n_exp, int chunks) {
+    const size_t need = (size_t)n_exp * chunks;
+    if (need > st->chunk_cap) {
+        dfree(st->d_chunk);
+        dfree(st->d_flags);
+        st->chunk_cap = 0;
+        int rc;
+        if ((rc = dalloc(&st->d_chunk, need))) return rc;
+        if ((rc = dalloc(&st->d_flags, need * 32))) return rc;
+        st->chunk_cap = need;
+    }
+    return FPHO_OK;
+}
+int ensure_params(fpho_store *st, int n_exp) {
     if (n_exp <= st->scratch_exp) return FPHO_OK;
-    dfree(st->d_chunk); dfree(st->d_total); dfree(st->d_exps); dfree(st->d_spbase);
-    dfree(st->d_bg); dfree(st->d_regions); dfree(st->d_box);
+    fpho::pinned_put(st->h_par, st->h_par_bytes);
+    st->h_par = nullptr;
     st->scratch_exp = 0;
-    int rc;
-    if ((rc = dalloc(&st->d_chunk, (size_t)n_exp * st->n_chunks()))) return rc;
-    if ((rc = dalloc(&st->d_total, (size_t)n_exp))) return rc;
-    if ((rc = dalloc(&st->d_exps, (size_t)n_exp))) return rc;
-    if ((rc = dalloc(&st->d_spbase, (size_t)n_exp))) return rc;
-    if ((rc = dalloc(&st->d_box, (size_t)n_exp * 4))) return rc;
-    if ((rc = dalloc(&st->d_bg, (size_t)n_exp))) return rc;
-    if ((rc = dalloc(&st->d_regions, (size_t)n_exp))) return rc;
+    size_t bytes = (size_t)n_exp * (sizeof(CountPar) + sizeof(PackPar) + sizeof(int));
+    unsigned char *m = nullptr;
+    CUDA_TRY(fpho::pinned_get((void **)&m, &bytes));
+    st->h_par = m;
+    st->h_par_bytes = bytes;
+    st->par.count = reinterpret_cast<CountPar *>(m);
+    st->par.pack = reinterpret_cast<PackPar *>(st->par.count + n_exp);
+    st->par.totals = reinterpret_cast<int *>(st->par.pack + n_exp);
     st->scratch_exp = n_exp;
     return FPHO_OK;
 }
@@ -367,10 +452,11 @@ void region_box(const fpho_region &R, int nsx, int nsy, int s, int box[4]) {
     if (box[2] == 0 || box[3] == 0) box[2] = box[3] = 0;
 }
 
-// Validate the call's exposure list and regions, upload them, and run the
-// count and scan kernels; `totals` receives super-pixels per exposure.
+// Validate the call's exposure list and regions, put them where the kernels
+// read them, and run the count and scan kernels; the totals are in
+// st->par.totals on return.
 int count_pass(fpho_store *st, int n_exp, const int32_t *exposures, const fpho_region *regions,
-               std::vector<int> &totals, cudaStream_t s) {
+               cudaStream_t s) {
     if (!st || !exposures || !regions) return set_error(FPHO_ERR_INVALID, "NULL argument");
     if (n_exp < 1 || n_exp > 65535)
         return set_error(FPHO_ERR_INVALID, "n_exp=%d outside [1, 65535]", n_exp);
@@ -381,30 +467,91 @@ int count_pass(fpho_store *st, int n_exp, const int32_t *exposures, const fpho_r
         if (regions[e].kind != FPHO_REGION_CIRCLE && regions[e].kind != FPHO_REGION_RECT)
             return set_error(FPHO_ERR_INVALID, "region %d: unknown kind %d", e, regions[e].kind);
     }
-    int rc = ensure_scratch(st, n_exp);
+    ++st->serial;
+    int rc = ensure_params(st, n_exp);
     if (rc) return rc;
-    CUDA_TRY(cudaMemcpyAsync(st->d_exps, exposures, sizeof(int) * n_exp, cudaMemcpyHostToDevice, s));
-    CUDA_TRY(cudaMemcpyAsync(st->d_regions, regions, sizeof(fpho_region) * n_exp,
-                             cudaMemcpyHostToDevice, s));
-    std::vector<int> boxes(4 * (size_t)n_exp);
+    const Params &P = st->par;
     int nc = 1;
     for (int e = 0; e < n_exp; ++e) {
-        region_box(regions[e], st->nsx, st->nsy, st->s, &boxes[4 * (size_t)e]);
-        const long long n = (long long)boxes[4 * e + 2] * boxes[4 * e + 3];
+        int box[4];
+        region_box(regions[e], st->nsx, st->nsy, st->s, box);
+        P.count[e] = {regions[e], (uint16_t)box[0], (uint16_t)box[1], (uint16_t)box[2],
+                      (uint16_t)box[3]};
+        P.pack[e] = {exposures[e], 0, 0.0f, 0, {box[0], box[1], box[2], box[3]}};
+        const long long n = (long long)box[2] * box[3];
         nc = std::max(nc, (int)((n + fpho_store::kChunk - 1) / fpho_store::kChunk));
     }
     st->grid_chunks = nc;
-    CUDA_TRY(cudaMemcpyAsync(st->d_box, boxes.data(), sizeof(int) * boxes.size(),
-                             cudaMemcpyHostToDevice, s));
-    store_count<<<dim3(nc, n_exp), kThreads, 0, s>>>(
-        st->d_regions, reinterpret_cast<const SpBox *>(st->d_box), st->s, nc, st->d_chunk);
+    if ((rc = ensure_scratch(st, n_exp, nc))) return rc;
+    store_count<<<dim3(nc, n_exp), kThreads, 0, s>>>(P, st->s, nc, st->d_chunk, st->d_flags);
     CUDA_TRY(cudaGetLastError());
-    store_scan<<<n_exp, kThreads, 0, s>>>(nc, st->d_chunk, st->d_total);
-    CUDA_TRY(cudaGetLastError());
-    totals.assign(n_exp, 0);
-    CUDA_TRY(cudaMemcpyAsync(totals.data(), st->d_total, sizeof(int) * n_exp,
-                             cudaMemcpyDeviceToHost, s));
+    if (nc > 1) {
+        void *args[] = {(void *)&P, (void *)&nc, &st->d_chunk};
+        CUDA_TRY(fpho::launch_dependent((const void *)store_scan, dim3(n_exp), dim3(kThreads),
+                                        args, 0, s));
+    }
     CUDA_TRY(cudaStreamSynchronize(s));
+    return FPHO_OK;
+}
+
+// The list and the pixels of the count pass just made.
+int pack_pass(fpho_store *st, int n_exp, const float *background, float max_snr, float *data,
+              float *ierr, float *xpix, float *ypix, int64_t npix_capacity,
+              int32_t *exposure_start, int32_t *exposure_N, cudaStream_t s) {
+    const Params &P = st->par;
+    long long npix = 0, nsp = 0;
+    for (int e = 0; e < n_exp; ++e) {
+        const int total = P.totals[e];
+        P.pack[e].base = (int)std::min<long long>(nsp, INT32_MAX);
+        P.pack[e].bg = background ? background[e] : 0.0f;
+        exposure_start[e] = (int32_t)std::min<long long>(npix, INT32_MAX);
+        exposure_N[e] = total * st->s2;
+        npix += (long long)total * st->s2;
+        nsp += total;
+    }
+    if (npix > INT32_MAX) return set_error(FPHO_ERR_LIMIT, "the patch would have %lld pixels", npix);
+    if (npix > npix_capacity)
+        return set_error(FPHO_ERR_LIMIT, "the patch has %lld pixels; the output holds %lld", npix,
+                         (long long)npix_capacity);
+    if (npix == 0) return FPHO_OK;
+    if (!data || !ierr || !xpix || !ypix)
+        return set_error(FPHO_ERR_INVALID, "an output pixel array is NULL");
+    if ((size_t)nsp > st->list_cap) {
+        dfree(st->d_list_sp);
+        dfree(st->d_list_exp);
+        dfree(st->d_list_bg);
+        st->list_cap = 0;
+        int rc;
+        if ((rc = dalloc(&st->d_list_sp, (size_t)nsp))) return rc;
+        if ((rc = dalloc(&st->d_list_exp, (size_t)nsp))) return rc;
+        if ((rc = dalloc(&st->d_list_bg, (size_t)nsp))) return rc;
+        st->list_cap = (size_t)nsp;
+    }
+    const int nc = st->grid_chunks;
+    const bool vec = (st->s2 % 4 == 0) &&
+                     ((((uintptr_t)data) | ((uintptr_t)ierr) | ((uintptr_t)xpix) |
+                       ((uintptr_t)ypix)) % 16 == 0);
+    unsigned n_items = (unsigned)(vec ? npix / 4 : npix);
+    const unsigned blocks = (n_items + 2 * kThreads - 1) / (2 * kThreads);
+    if (st->time_gather) CUDA_TRY(cudaEventRecord(st->ev0, s));
+    store_compact<<<dim3(nc, n_exp), kThreads, 0, s>>>(P, st->d_chunk, st->d_flags, st->nsy, nc,
+                                                       st->d_list_sp, st->d_list_exp,
+                                                       st->d_list_bg);
+    CUDA_TRY(cudaGetLastError());
+    bool has_bg = background != nullptr;
+    unsigned nsy = (unsigned)st->nsy, side = (unsigned)st->s;
+    void *args[] = {&st->d_pix,     &st->exp_floats, &st->d_list_sp, &st->d_list_exp,
+                    &st->d_list_bg, &n_items,        &has_bg,        &max_snr,
+                    &nsy,           &side,           &data,          &ierr,
+                    &xpix,          &ypix};
+    const void *fn = !vec           ? (const void *)store_copy<false, 0>
+                     : st->s == 8   ? (const void *)store_copy<true, 8>
+                                    : (const void *)store_copy<true, 0>;
+    CUDA_TRY(fpho::launch_dependent(fn, dim3(blocks), dim3(kThreads), args, 0, s));
+    if (st->time_gather) CUDA_TRY(cudaEventRecord(st->ev1, s));
+    // the kernels read the parameters, which the next call overwrites
+    CUDA_TRY(cudaStreamSynchronize(s));
+    if (st->time_gather) CUDA_TRY(cudaEventElapsedTime(&st->last_gather_ms, st->ev0, st->ev1));
     return FPHO_OK;
 }
 
@@ -474,10 +621,9 @@ extern "C" int fpho_store_count(fpho_store *st, int n_exp, const int32_t *exposu
                                 const fpho_region *regions, int32_t *n_superpixels, void *stream) {
     clear_error();
     if (!n_superpixels) return set_error(FPHO_ERR_INVALID, "n_superpixels is NULL");
-    std::vector<int> totals;
-    int rc = count_pass(st, n_exp, exposures, regions, totals, (cudaStream_t)stream);
+    int rc = count_pass(st, n_exp, exposures, regions, (cudaStream_t)stream);
     if (rc) return rc;
-    std::copy(totals.begin(), totals.end(), n_superpixels);
+    std::copy(st->par.totals, st->par.totals + n_exp, n_superpixels);
     return FPHO_OK;
 }
 
@@ -489,67 +635,37 @@ extern "C" int fpho_store_gather(fpho_store *st, int n_exp, const int32_t *expos
     clear_error();
     if (!exposure_start || !exposure_N)
         return set_error(FPHO_ERR_INVALID, "exposure_start/exposure_N is NULL");
-    cudaStream_t s = (cudaStream_t)stream;
-    std::vector<int> totals;
-    int rc = count_pass(st, n_exp, exposures, regions, totals, s);
+    int rc = count_pass(st, n_exp, exposures, regions, (cudaStream_t)stream);
     if (rc) return rc;
-    std::vector<int> spbase(n_exp);
-    long long npix = 0, nsp = 0;
-    for (int e = 0; e < n_exp; ++e) {
-        spbase[e] = (int)std::min<long long>(nsp, INT32_MAX);
-        exposure_start[e] = (int32_t)std::min<long long>(npix, INT32_MAX);
-        exposure_N[e] = totals[e] * st->s2;
-        npix += (long long)totals[e] * st->s2;
-        nsp += totals[e];
-    }
-    if (npix > INT32_MAX) return set_error(FPHO_ERR_LIMIT, "the patch would have %lld pixels", npix);
-    if (npix > npix_capacity)
-        return set_error(FPHO_ERR_LIMIT, "the patch has %lld pixels; the output holds %lld", npix,
-                         (long long)npix_capacity);
-    if (npix == 0) return FPHO_OK;
-    if (!data || !ierr || !xpix || !ypix)
-        return set_error(FPHO_ERR_INVALID, "an output pixel array is NULL");
-    if ((size_t)nsp > st->list_cap) {
-        dfree(st->d_list_sp);
-        dfree(st->d_list_exp);
-        st->list_cap = 0;
-        if ((rc = dalloc(&st->d_list_sp, (size_t)nsp))) return rc;
-        if ((rc = dalloc(&st->d_list_exp, (size_t)nsp))) return rc;
-        st->list_cap = (size_t)nsp;
-    }
-    CUDA_TRY(cudaMemcpyAsync(st->d_spbase, spbase.data(), sizeof(int) * n_exp,
-                             cudaMemcpyHostToDevice, s));
-    if (background)
-        CUDA_TRY(cudaMemcpyAsync(st->d_bg, background, sizeof(float) * n_exp,
-                                 cudaMemcpyHostToDevice, s));
-    const int nc = st->grid_chunks;
-    const bool vec = (st->s2 % 4 == 0) &&
-                     ((((uintptr_t)data) | ((uintptr_t)ierr) | ((uintptr_t)xpix) |
-                       ((uintptr_t)ypix)) % 16 == 0);
-    const long long n_items = vec ? npix / 4 : npix;
-    const unsigned blocks = (unsigned)((n_items + kThreads - 1) / kThreads);
-    if (st->time_gather) CUDA_TRY(cudaEventRecord(st->ev0, s));
-    store_compact<<<dim3(nc, n_exp), kThreads, 0, s>>>(
-        st->d_regions, reinterpret_cast<const SpBox *>(st->d_box), st->d_chunk, st->d_spbase,
-        st->nsy, st->s, nc, st->d_list_sp, st->d_list_exp);
-    CUDA_TRY(cudaGetLastError());
-    const float *bgp = background ? st->d_bg : nullptr;
-    if (vec)
-        store_copy<true><<<blocks, kThreads, 0, s>>>(st->d_pix, st->exp_floats, st->d_exps,
-                                                     st->d_list_sp, st->d_list_exp, n_items, bgp,
-                                                     max_snr, st->nsy, st->s, data, ierr, xpix,
-                                                     ypix);
-    else
-        store_copy<false><<<blocks, kThreads, 0, s>>>(st->d_pix, st->exp_floats, st->d_exps,
-                                                      st->d_list_sp, st->d_list_exp, n_items, bgp,
-                                                      max_snr, st->nsy, st->s, data, ierr, xpix,
-                                                      ypix);
-    CUDA_TRY(cudaGetLastError());
-    if (st->time_gather) CUDA_TRY(cudaEventRecord(st->ev1, s));
-    // the host vectors above die on return; the stream must be done with them
-    CUDA_TRY(cudaStreamSynchronize(s));
-    if (st->time_gather) CUDA_TRY(cudaEventElapsedTime(&st->last_gather_ms, st->ev0, st->ev1));
+    return pack_pass(st, n_exp, background, max_snr, data, ierr, xpix, ypix, npix_capacity,
+                     exposure_start, exposure_N, (cudaStream_t)stream);
+}
+
+extern "C" int fpho_store_gather_begin(fpho_store *st, int n_exp, const int32_t *exposures,
+                                       const fpho_region *regions, int64_t *npix,
+                                       uint64_t *ticket, void *stream) {
+    clear_error();
+    if (!npix || !ticket) return set_error(FPHO_ERR_INVALID, "NULL argument");
+    int rc = count_pass(st, n_exp, exposures, regions, (cudaStream_t)stream);
+    if (rc) return rc;
+    *npix = 0;
+    for (int e = 0; e < n_exp; ++e) *npix += (int64_t)st->par.totals[e] * st->s2;
+    *ticket = st->serial;
     return FPHO_OK;
+}
+
+extern "C" int fpho_store_gather_end(fpho_store *st, uint64_t ticket, int n_exp,
+                                     const float *background, float max_snr, float *data,
+                                     float *ierr, float *xpix, float *ypix, int64_t npix_capacity,
+                                     int32_t *exposure_start, int32_t *exposure_N, void *stream) {
+    clear_error();
+    if (!st || !exposure_start || !exposure_N)
+        return set_error(FPHO_ERR_INVALID, "NULL argument");
+    if (ticket != st->serial || n_exp < 1 || n_exp > st->scratch_exp)
+        return set_error(FPHO_ERR_STATE, "another count or gather came between the two halves");
+    ++st->serial;  // a ticket is good once
+    return pack_pass(st, n_exp, background, max_snr, data, ierr, xpix, ypix, npix_capacity,
+                     exposure_start, exposure_N, (cudaStream_t)stream);
 }
 
 extern "C" int fpho_store_time_gather(fpho_store *st, int enable) {
@@ -577,9 +693,9 @@ extern "C" int fpho_store_free(fpho_store *st) {
     if (st->ev1) cudaEventDestroy(st->ev1);
     if (st->d_pix) cudaFree(st->d_pix);
     st->d_pix = nullptr;
-    dfree(st->d_chunk); dfree(st->d_total); dfree(st->d_exps); dfree(st->d_spbase);
-    dfree(st->d_bg); dfree(st->d_regions);
-    dfree(st->d_list_sp); dfree(st->d_list_exp); dfree(st->d_box);
+    fpho::pinned_put(st->h_par, st->h_par_bytes);
+    dfree(st->d_chunk); dfree(st->d_flags);
+    dfree(st->d_list_sp); dfree(st->d_list_exp); dfree(st->d_list_bg);
     delete st;
     return FPHO_OK;
 }

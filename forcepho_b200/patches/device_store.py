@@ -138,20 +138,32 @@ class DeviceStore:
         import torch
         idx = np.ascontiguousarray(indices, dtype=np.int32)
         reg = np.ascontiguousarray(regions, dtype=REGION_DTYPE)
-        if npix is None:
-            npix = int(self.count(idx, reg, stream).astype(np.int64).sum()) \
-                * self.super_pixel_size ** 2
-        bufs = [torch.empty(max(npix, 1), dtype=torch.float32, device="cuda") for _ in range(4)]
         bg = None if background is None else np.ascontiguousarray(background, dtype=np.float32)
         start = np.zeros(len(idx), dtype=np.int32)
         n = np.zeros(len(idx), dtype=np.int32)
         if stream is None:
             stream = torch.cuda.current_stream().cuda_stream
-        _lib.call("fpho_store_gather", self.handle, len(idx), idx.ctypes.data, reg.ctypes.data,
-                  None if bg is None else bg.ctypes.data, float(max_snr or 0.0),
-                  *[b.data_ptr() for b in bufs], int(npix), start.ctypes.data, n.ctypes.data,
-                  stream)
-        total = int(n.astype(np.int64).sum())
+        bg_ptr = None if bg is None else bg.ctypes.data
+        ticket = None
+        if npix is None:
+            need, ticket = ctypes.c_int64(), ctypes.c_uint64()
+            _lib.call("fpho_store_gather_begin", self.handle, len(idx), idx.ctypes.data,
+                      reg.ctypes.data, ctypes.byref(need), ctypes.byref(ticket), stream)
+            npix = need.value
+        bufs = [torch.empty(max(npix, 1), dtype=torch.float32, device="cuda") for _ in range(4)]
+        out = [float(max_snr or 0.0), *[b.data_ptr() for b in bufs], int(npix),
+               start.ctypes.data, n.ctypes.data, stream]
+        if ticket is not None:
+            try:
+                _lib.call("fpho_store_gather_end", self.handle, ticket, len(idx), bg_ptr, *out)
+            except _lib.FphoError as e:
+                if e.code != _lib.FPHO_ERR_STATE:
+                    raise
+                ticket = None  # another thread used the store in between
+        if ticket is None:
+            _lib.call("fpho_store_gather", self.handle, len(idx), idx.ctypes.data,
+                      reg.ctypes.data, bg_ptr, *out)
+        total = int(n.sum(dtype=np.int64))
         return [b[:total] for b in bufs], start, n
 
     def gather_many(self, groups, max_snr=None, stream=None):

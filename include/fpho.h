@@ -536,6 +536,17 @@ FPHO_API int fpho_store_gather(fpho_store *st, int n_exp, const int32_t *exposur
                                float *data, float *ierr, float *xpix, float *ypix,
                                int64_t npix_capacity, int32_t *exposure_start,
                                int32_t *exposure_N, void *stream);
+/* The same in two halves, for a caller that sizes its outputs in between:
+ * begin counts and returns the pixels the patch needs (and a ticket), end packs
+ * them.  The ticket is good for one end, and only while no other count or
+ * gather ran on the store in between (STATE otherwise).  Both synchronize. */
+FPHO_API int fpho_store_gather_begin(fpho_store *st, int n_exp, const int32_t *exposures,
+                                     const fpho_region *regions, int64_t *npix, uint64_t *ticket,
+                                     void *stream);
+FPHO_API int fpho_store_gather_end(fpho_store *st, uint64_t ticket, int n_exp,
+                                   const float *background, float max_snr, float *data,
+                                   float *ierr, float *xpix, float *ypix, int64_t npix_capacity,
+                                   int32_t *exposure_start, int32_t *exposure_N, void *stream);
 /* Enable (1) or disable (0) CUDA events around the gather kernel of every
  * following fpho_store_gather; fpho_store_last_gather_ms gives the last one's
  * milliseconds (the gather synchronizes, so it is ready on return). */
