@@ -295,6 +295,8 @@ int tile_parts(int variant, int n_tiles) {
     return best;
 }
 
+constexpr int SM_SMEM_BYTES = 228 * 1024;  // of an SM, the CTAs' 1 KB reserves included
+
 int launch_tile_kernel(int variant, const TileArgs &A, int n_tiles, cudaStream_t stream,
                        bool grad, const int *order, int *counter, bool exact, int parts) {
     if (n_tiles <= 0) return FPHO_OK;
@@ -305,7 +307,17 @@ int launch_tile_kernel(int variant, const TileArgs &A, int n_tiles, cudaStream_t
     if (!fn)
         return set_error(FPHO_ERR_STATE, "the exact-residual kernel is not compiled for the "
                          "%d-thread, %d-pixel tile", V.nt, V.tile);
-    const size_t smem = tile_smem_bytes(variant, A.live_cap, A.idx_cap, A.pgrad_stride);
+    size_t smem = tile_smem_bytes(variant, A.live_cap, A.idx_cap, A.pgrad_stride);
+    // Few tiles per SM: 16 warps of CTAs on each instead of as many as fit (the
+    // limit set by shared memory; a smaller grid would leave some SMs fuller
+    // than others).  More CTAs make every tile take longer, the last ones too:
+    // 1140 tiles 117 against 124 us, 2048 tiles 283 against 288; from some 24
+    // tiles per SM more CTAs win (4800 tiles 543 against 531, 23,040 6.09
+    // against 5.89 ms).
+    if (dyn && n_tiles < 24 * device_sms()) {
+        const size_t few = (size_t)(SM_SMEM_BYTES / (512 / V.nt + 1)) - 512;
+        smem = std::max(smem, few);
+    }
     int dev = 0;
     CUDA_TRY(cudaGetDevice(&dev));
     if (dev >= 64) return set_error(FPHO_ERR_LIMIT, "device ordinal %d >= 64", dev);

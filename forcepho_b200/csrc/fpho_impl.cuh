@@ -324,28 +324,47 @@ constexpr float KEXP_LO = -9.629815167500055e-09f;
 // Arguments above 174 give garbage that callers discard (they select 0 for
 // exp-arguments above the cutoff, and never use the value at pixels outside
 // the culling box).
-__device__ __forceinline__ v2 exp_neg_half(v2 Q, v2 KEXP2, v2 KEXPLO2) {
-    const float MAGIC = 12582912.0f;  // 1.5 * 2^23
-    const v2 t = fma2(Q, KEXP2, pk1(MAGIC));
+// N chains at once, operation by operation.
+template <int N>
+__device__ __forceinline__ void exp_neg_half(const v2 (&Q)[N], v2 (&G)[N], v2 KEXP2, v2 KEXPLO2) {
+    const v2 MAGIC = pk1(12582912.0f), MINUS1 = pk1(-1.0f);  // 1.5 * 2^23
+    v2 t[N], f[N];
+#pragma unroll
+    for (int i = 0; i < N; ++i) t[i] = fma2(Q[i], KEXP2, MAGIC);
     // MAGIC - t (one FMA, no sign-bit operation) is -n exactly
-    const v2 f = fma2(Q, KEXPLO2, fma2(Q, KEXP2, fma2(t, pk1(-1.0f), pk1(MAGIC))));
-    v2 p = pk1(1.5370704932138324e-04f);
-    p = fma2(p, f, pk1(1.3399848248809576e-03f));
-    p = fma2(p, f, pk1(9.618373587727547e-03f));
-    p = fma2(p, f, pk1(5.550329014658928e-02f));
-    p = fma2(p, f, pk1(2.4022647738456726e-01f));
-    p = fma2(p, f, pk1(6.931471824645996e-01f));
-    p = fma2(p, f, pk1(1.0f));
+#pragma unroll
+    for (int i = 0; i < N; ++i) f[i] = fma2(t[i], MINUS1, MAGIC);
+#pragma unroll
+    for (int i = 0; i < N; ++i) f[i] = fma2(Q[i], KEXP2, f[i]);
+#pragma unroll
+    for (int i = 0; i < N; ++i) f[i] = fma2(Q[i], KEXPLO2, f[i]);
+    const float c[7] = {1.5370704932138324e-04f, 1.3399848248809576e-03f, 9.618373587727547e-03f,
+                        5.550329014658928e-02f,  2.4022647738456726e-01f, 6.931471824645996e-01f,
+                        1.0f};
+#pragma unroll
+    for (int i = 0; i < N; ++i) G[i] = fma2(pk1(c[0]), f[i], pk1(c[1]));
+#pragma unroll
+    for (int k = 2; k < 7; ++k)
+#pragma unroll
+        for (int i = 0; i < N; ++i) G[i] = fma2(G[i], f[i], pk1(c[k]));
     // t's low mantissa bits hold n (two's complement); (bits(t) << 23) adds n
-    // to the exponent of p, since bits(1.5*2^23) << 23 vanishes mod 2^32.
-    uint32_t t0, t1, p0, p1;
-    asm("mov.b64 {%0, %1}, %2;" : "=r"(t0), "=r"(t1) : "l"(t));
-    asm("mov.b64 {%0, %1}, %2;" : "=r"(p0), "=r"(p1) : "l"(p));
-    p0 += t0 << 23;
-    p1 += t1 << 23;
-    v2 r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "r"(p0), "r"(p1));
-    return r;
+    // to the exponent of the polynomial, since bits(1.5*2^23) << 23 vanishes
+    // mod 2^32.
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+        uint32_t t0, t1, p0, p1;
+        asm("mov.b64 {%0, %1}, %2;" : "=r"(t0), "=r"(t1) : "l"(t[i]));
+        asm("mov.b64 {%0, %1}, %2;" : "=r"(p0), "=r"(p1) : "l"(G[i]));
+        p0 += t0 << 23;
+        p1 += t1 << 23;
+        asm("mov.b64 %0, {%1, %2};" : "=l"(G[i]) : "r"(p0), "r"(p1));
+    }
+}
+__device__ __forceinline__ v2 exp_neg_half(v2 Q, v2 KEXP2, v2 KEXPLO2) {
+    const v2 q[1] = {Q};
+    v2 g[1];
+    exp_neg_half(q, g, KEXP2, KEXPLO2);
+    return g[0];
 }
 
 }  // namespace fpho

@@ -251,49 +251,65 @@ __device__ __forceinline__ void residual_pairs(const v2 (&X)[KP], const v2 (&Y)[
 }
 
 // Pass 1 for two consecutive kept Gaussians a, b at once: their exponentials
-// are independent and interleave, and R is updated with a's term and then
-// b's, exactly as two calls of residual_pairs in order would.
+// are independent, and R is updated with a's term and then b's, exactly as two
+// calls of residual_pairs in order would.
+//
+// Written operation by operation over all 2 KP chains: a packed FMA reads three
+// register pairs and takes three cycles when all differ, two when it shares one
+// with its neighbour (measured: 3.07 and 2.25), so the chains take turns with
+// each constant.  The register file's reads are what bounds this loop.  With
+// the chains one after the other it took 8 registers more, and a fifth CTA no
+// longer fitted an SM (60-source patch 6.09 ms instead of 5.89).
 template <int KP, int SH = SHARE_NONE>
 __device__ __forceinline__ void residual_pairs2(const v2 (&X)[KP], const v2 (&Y)[KP], v2 (&R)[KP],
                                                 const float *ra, const float *rb, v2 CM24,
                                                 v2 KEXP2, v2 KEXPLO2) {
-    v2 NXa, NYa, FXXa, FXYa, FYYa, AMPa, HBa, C0a;
-    v2 NXb, NYb, FXXb, FXYb, FYYb, AMPb, HBb, C0b;
-    ld2(ra + R_NXC, NXa, NYa);
-    ld2(ra + R_FXX, FXXa, FXYa);
-    ld2(ra + R_FYY, FYYa, AMPa);
-    ld2(ra + R_HB, HBa, C0a);
-    ld2(rb + R_NXC, NXb, NYb);
-    ld2(rb + R_FXX, FXXb, FXYb);
-    ld2(rb + R_FYY, FYYb, AMPb);
-    ld2(rb + R_HB, HBb, C0b);
-    const v2 HAa = mul2(AMPa, CM24), HAb = mul2(AMPb, CM24);
+    constexpr int N = 2 * KP;  // chain i: Gaussian i / KP, pixel pair i % KP
+    v2 NX[2], NY[2], FXX[2], FXY[2], FYY[2], AMP[2], HA[2], HB[2], C0[2];
 #pragma unroll
-    for (int j = 0; j < KP; ++j) {
-        const v2 DXa = add2(X[SH == SHARE_X ? 0 : j], NXa), DYa = add2(Y[SH == SHARE_Y ? 0 : j], NYa);
-        const v2 DXb = add2(X[SH == SHARE_X ? 0 : j], NXb), DYb = add2(Y[SH == SHARE_Y ? 0 : j], NYb);
-        const v2 VXa = fma2(FXYa, DYa, mul2(FXXa, DXa));
-        const v2 VXb = fma2(FXYb, DYb, mul2(FXXb, DXb));
-        const v2 VYa = fma2(FXYa, DXa, mul2(FYYa, DYa));
-        const v2 VYb = fma2(FXYb, DXb, mul2(FYYb, DYb));
-        const v2 Qa = fma2(DYa, VYa, mul2(DXa, VXa));
-        const v2 Qb = fma2(DYb, VYb, mul2(DXb, VXb));
-        v2 Ga = exp_neg_half(Qa, KEXP2, KEXPLO2);
-        v2 Gb = exp_neg_half(Qb, KEXP2, KEXPLO2);
-        {
-            float g0, g1, q0, q1;
-            unpk(Ga, g0, g1);
-            unpk(Qa, q0, q1);
-            Ga = pk(q0 > FPHO_MAX_EXP_ARG ? 0.0f : g0, q1 > FPHO_MAX_EXP_ARG ? 0.0f : g1);
-            unpk(Gb, g0, g1);
-            unpk(Qb, q0, q1);
-            Gb = pk(q0 > FPHO_MAX_EXP_ARG ? 0.0f : g0, q1 > FPHO_MAX_EXP_ARG ? 0.0f : g1);
-        }
-        const v2 Sa = fma2(VYa, VYa, mul2(VXa, VXa));
-        const v2 Sb = fma2(VYb, VYb, mul2(VXb, VXb));
-        R[j] = fma2(fma2(Sa, HAa, HBa), Ga, R[j]);
-        R[j] = fma2(fma2(Sb, HAb, HBb), Gb, R[j]);
+    for (int g = 0; g < 2; ++g) {
+        const float *r = g ? rb : ra;
+        ld2(r + R_NXC, NX[g], NY[g]);
+        ld2(r + R_FXX, FXX[g], FXY[g]);
+        ld2(r + R_FYY, FYY[g], AMP[g]);
+        ld2(r + R_HB, HB[g], C0[g]);
+        HA[g] = mul2(AMP[g], CM24);
     }
+    v2 DX[N], DY[N], VX[N], VY[N], Q[N], S[N];
+#pragma unroll
+    for (int i = 0; i < N; ++i) DX[i] = add2(X[SH == SHARE_X ? 0 : i % KP], NX[i / KP]);
+#pragma unroll
+    for (int i = 0; i < N; ++i) DY[i] = add2(Y[SH == SHARE_Y ? 0 : i % KP], NY[i / KP]);
+#pragma unroll
+    for (int i = 0; i < N; ++i) VX[i] = mul2(FXX[i / KP], DX[i]);
+#pragma unroll
+    for (int i = 0; i < N; ++i) VX[i] = fma2(FXY[i / KP], DY[i], VX[i]);
+#pragma unroll
+    for (int i = 0; i < N; ++i) VY[i] = mul2(FYY[i / KP], DY[i]);
+#pragma unroll
+    for (int i = 0; i < N; ++i) VY[i] = fma2(FXY[i / KP], DX[i], VY[i]);
+#pragma unroll
+    for (int i = 0; i < N; ++i) Q[i] = mul2(DX[i], VX[i]);
+#pragma unroll
+    for (int i = 0; i < N; ++i) Q[i] = fma2(DY[i], VY[i], Q[i]);
+#pragma unroll
+    for (int i = 0; i < N; ++i) S[i] = mul2(VX[i], VX[i]);
+#pragma unroll
+    for (int i = 0; i < N; ++i) S[i] = fma2(VY[i], VY[i], S[i]);
+#pragma unroll
+    for (int i = 0; i < N; ++i) S[i] = fma2(S[i], HA[i / KP], HB[i / KP]);
+    // the residual needs an unbiased exponential
+    v2 G[N];
+    exp_neg_half(Q, G, KEXP2, KEXPLO2);
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+        float g0, g1, q0, q1;
+        unpk(G[i], g0, g1);
+        unpk(Q[i], q0, q1);
+        G[i] = pk(q0 > FPHO_MAX_EXP_ARG ? 0.0f : g0, q1 > FPHO_MAX_EXP_ARG ? 0.0f : g1);
+    }
+#pragma unroll
+    for (int i = 0; i < N; ++i) R[i % KP] = fma2(S[i], G[i], R[i % KP]);
 }
 
 // Pass 1 for the staged records [i0, i1), two at a time; an odd last one is
