@@ -119,6 +119,8 @@ _SIGS = {
     "fpho_bounded_lnp_grad": (c_int, [c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                                       c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p,
                                       c_int, c_void_p, c_void_p]),
+    "fpho_lnlike": (c_int, [c_void_p, c_int, c_void_p, c_void_p]),
+    "fpho_lnlike_grad": (c_int, [c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p]),
     "fpho_patch_time_tiles": (c_int, [c_void_p, c_int]),
     "fpho_patch_image_gaussians": (c_int, [c_void_p, c_int, c_void_p, c_int,
                                            ctypes.POINTER(c_int)]),

@@ -110,7 +110,9 @@ class LnLike(torch.autograd.Function):
         ev.run(theta, grad=fused)
         ctx.ev, ctx.fused, ctx.gen = ev, fused, ev.generation
         ctx.save_for_backward(theta)
-        return ev.chi2.sum() * -0.5
+        out = torch.empty((), dtype=torch.float64, device=ev.chi2.device)
+        _lib.call("fpho_lnlike", ev.chi2.data_ptr(), ev.n_bands, out.data_ptr(), _stream())
+        return out
 
     @staticmethod
     def backward(ctx, g):
@@ -118,7 +120,20 @@ class LnLike(torch.autograd.Function):
         if not ctx.fused or ev.generation != ctx.gen:
             (theta,) = ctx.saved_tensors
             ev.run(theta, grad=True)
-        return (ev.stacked() * (g * -0.5)).reshape(ctx.saved_tensors[0].shape), None
+        shape = ctx.saved_tensors[0].shape
+        g = g.contiguous()
+        try:
+            plain = g.dtype == torch.float64 and g.is_cuda and g.data_ptr() != 0
+        except RuntimeError:    # a batched gradient has no storage of its own
+            plain = False
+        if torch.is_grad_enabled() or not plain:
+            # differentiable in g (create_graph), and any other kind of g
+            return (ev.stacked() * (g * -0.5)).reshape(shape), None
+        out = torch.empty((ev.n_sources, ev.n_bands + 6), dtype=torch.float64,
+                          device=ev.dchi2.device)
+        _lib.call("fpho_lnlike_grad", ev.dchi2.data_ptr(), ev.n_bands, ev.n_sources,
+                  g.data_ptr(), out.data_ptr(), _stream())
+        return out.reshape(shape), None
 
 
 def lnlike(theta, ev):

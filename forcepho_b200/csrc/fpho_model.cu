@@ -15,6 +15,7 @@
 #include <new>
 
 #include "fpho.h"
+#include "fpho_impl.cuh"
 #include "fpho_internal.h"
 
 namespace fpho {
@@ -274,6 +275,34 @@ __global__ void __launch_bounds__(LNP_THREADS) bounded_lnp_grad_kernel(
     }
 }
 
+// lnlike = -sum chi2 / 2 over the bands, in band order.
+__global__ void lnlike_kernel(const double *chi2, int n_bands, double *out) {
+    fpho::wait_for_earlier_kernel();
+    double c = 0.0;
+    for (int b = 0; b < n_bands; ++b) c += chi2[b];
+    *out = -0.5 * c;
+}
+
+// g d lnlike / d theta: the per-band dchi2 (n_bands, n_sources, 7) stacked in
+// Scene order (n_sources, n_bands + 6) -- a flux from its band, a shape
+// parameter summed over the bands in order -- times -g / 2.
+__global__ void lnlike_grad_kernel(const float *dchi2, int n_bands, int n_sources,
+                                   const double *g, double *out) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int n = n_bands + 6;
+    fpho::wait_for_earlier_kernel();
+    if (i >= n_sources * n) return;
+    const int s = i / n, j = i - s * n;
+    double d = 0.0;
+    if (j < n_bands) {
+        d = (double)dchi2[((size_t)j * n_sources + s) * FPHO_NPARAMS];
+    } else {
+        for (int b = 0; b < n_bands; ++b)
+            d += (double)dchi2[((size_t)b * n_sources + s) * FPHO_NPARAMS + 1 + j - n_bands];
+    }
+    out[i] = d * (*g * -0.5);
+}
+
 // Spline values and derivatives at arbitrary points (for validation).
 __global__ void spline_points_kernel(SplineView S, const double *x, const double *y, int m,
                                      double *out) {
@@ -436,6 +465,32 @@ extern "C" int fpho_build_proposal_batch(const fpho_spline *s, const double *the
     proposal_kernel<false><<<(n_sources + 3) / 4, PROP_THREADS, 0, (cudaStream_t)stream>>>(
         s->view, theta, nullptr, nullptr, n_sources, 0, src_bands, src_offset, nullptr, out);
     const cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return set_error(FPHO_ERR_CUDA, "launch: %s", cudaGetErrorString(e));
+    return FPHO_OK;
+}
+
+extern "C" int fpho_lnlike(const double *chi2, int n_bands, double *out, void *stream) {
+    clear_error();
+    if (!chi2 || !out) return set_error(FPHO_ERR_INVALID, "NULL argument");
+    if (n_bands < 1) return set_error(FPHO_ERR_INVALID, "n_bands=%d < 1", n_bands);
+    void *args[] = {&chi2, &n_bands, &out};
+    const cudaError_t e = launch_dependent((const void *)lnlike_kernel, dim3(1), dim3(1), args, 0,
+                                           (cudaStream_t)stream);
+    if (e != cudaSuccess) return set_error(FPHO_ERR_CUDA, "launch: %s", cudaGetErrorString(e));
+    return FPHO_OK;
+}
+
+extern "C" int fpho_lnlike_grad(const float *dchi2, int n_bands, int n_sources, const double *g,
+                                double *out, void *stream) {
+    clear_error();
+    if (!dchi2 || !g || !out) return set_error(FPHO_ERR_INVALID, "NULL argument");
+    if (n_bands < 1 || n_sources < 1)
+        return set_error(FPHO_ERR_INVALID, "n_bands=%d or n_sources=%d < 1", n_bands, n_sources);
+    const int n = n_sources * (n_bands + 6);
+    void *args[] = {&dchi2, &n_bands, &n_sources, &g, &out};
+    const cudaError_t e =
+        launch_dependent((const void *)lnlike_grad_kernel, dim3((n + 127) / 128), dim3(128), args,
+                         0, (cudaStream_t)stream);
     if (e != cudaSuccess) return set_error(FPHO_ERR_CUDA, "launch: %s", cudaGetErrorString(e));
     return FPHO_OK;
 }

@@ -270,6 +270,15 @@ FPHO_API int fpho_bounded_lnp_grad(int n_params, const double *z, const double *
                                    double *lnp_out, double *work, int n_work,
                                    unsigned *counter, void *stream);
 
+/* The likelihood of a proposal's device results: *out = -sum chi2 / 2 over the
+ * bands (FastPosterior.evaluate, forcepho/model.py:323-387). */
+FPHO_API int fpho_lnlike(const double *chi2, int n_bands, double *out, void *stream);
+/* g d lnlike / d theta from dchi2 (n_bands, n_sources, 7), stacked in Scene
+ * order (n_sources, n_bands + 6) as FastPosterior.stack_grad
+ * (forcepho/model.py:387-405); *g is the upstream gradient.  Device pointers. */
+FPHO_API int fpho_lnlike_grad(const float *dchi2, int n_bands, int n_sources, const double *g,
+                              double *out, void *stream);
+
 /* Spline values and derivatives at m device points (x = sersic, y = rh):
  * out[m][n_radii][3] = (value, d/dsersic, d/drh). */
 FPHO_API int fpho_spline_points(const fpho_spline *s, const double *x, const double *y, int m,

@@ -71,3 +71,30 @@ def test_tile_parts(shapes):
     np.testing.assert_allclose(chi2, c, rtol=CHI2_RTOL)
     check_grad(dchi2, g, P, prop)
     assert np.max(np.abs(res - r)) <= 1e-5 * np.abs(P.data).max()
+
+
+@pytest.mark.parametrize("ns,nb", [(1, 1), (5, 3), (13, 8)])
+def test_lnlike_gradient_forms(ns, nb):
+    """The fused gradient of LnLike against the stacked torch form: plain,
+    scaled by an upstream gradient, batched and under create_graph."""
+    import torch
+    from forcepho_b200.autograd import PatchEvaluator, lnlike
+    P = patch(ns, [1] * nb, [(24, 24)] * nb, 2, seed=50 + ns)
+    P.send_to_device()
+    ev = PatchEvaluator(P)
+    theta = torch.tensor(P.params, dtype=torch.float64, device="cuda", requires_grad=True)
+    out = lnlike(theta, ev)
+    assert float(out.detach()) == pytest.approx(-0.5 * float(ev.chi2.sum()), rel=1e-14)
+    want = ev.stacked() * -0.5
+    (g,) = torch.autograd.grad(out, theta, retain_graph=True)
+    torch.testing.assert_close(g, want, rtol=1e-14, atol=0)
+    (g3,) = torch.autograd.grad(3.0 * out, theta, retain_graph=True)
+    torch.testing.assert_close(g3, 3.0 * want, rtol=1e-14, atol=0)
+    seeds = torch.tensor([1.0, -2.0], dtype=torch.float64, device="cuda")
+    (gb,) = torch.autograd.grad(out, theta, seeds, is_grads_batched=True, retain_graph=True)
+    torch.testing.assert_close(gb, seeds[:, None, None] * want, rtol=1e-14, atol=0)
+    w = torch.ones((), dtype=torch.float64, device="cuda", requires_grad=True)
+    (gc,) = torch.autograd.grad(w * out, theta, create_graph=True)
+    (dw,) = torch.autograd.grad(gc.sum(), w)
+    torch.testing.assert_close(dw, want.sum(), rtol=1e-12, atol=0)
+    P.free()
