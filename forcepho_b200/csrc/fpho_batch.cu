@@ -48,6 +48,7 @@ struct BandJob {
 __global__ void batch_gaussians(const BatchPatch *bps, const int2 *expmap,
                                 const fpho_source *props, int *err) {
     let_next_kernel_start();
+    wait_for_earlier_kernel();  // the proposals, and the last evaluation's readers
     if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) *err = 0;
     const int2 pe = expmap[blockIdx.y];
     const BatchPatch &bp = bps[pe.x];
@@ -464,9 +465,10 @@ static int batch_enqueue(fpho_batch *b, const fpho_source *d_props, double *d_ch
                          float *d_dchi2, cudaStream_t s) {
     if (b->count_pairs) CUDA_TRY(cudaMemsetAsync(b->d_pairs, 0, sizeof(long long), s));
     if (b->n_exp_total > 0 && b->max_g > 0) {
-        batch_gaussians<<<dim3((b->max_g + 127) / 128, b->n_exp_total), 128, 0, s>>>(
-            b->d_bps, b->d_expmap, d_props, b->d_err);
-        CUDA_TRY(cudaGetLastError());
+        void *gargs[] = {&b->d_bps, &b->d_expmap, &d_props, &b->d_err};
+        CUDA_TRY(launch_dependent((const void *)batch_gaussians,
+                                  dim3((b->max_g + 127) / 128, b->n_exp_total), dim3(128), gargs,
+                                  0, s));
     } else {
         CUDA_TRY(cudaMemsetAsync(b->d_err, 0, sizeof(int), s));
     }

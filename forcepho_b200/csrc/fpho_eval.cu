@@ -1045,23 +1045,29 @@ int enqueue_evaluate(fpho_patch *p, const fpho_source *prop, double *d_chi2, flo
         dim3 grid(std::max((p->max_g + PREP_THREADS - 1) / PREP_THREADS, 1),
                   std::max(p->n_exp + (ordered ? 1 : 0), 1));
         int *order = ordered ? p->d_tile_order : nullptr;
-        auto with_arg = [&](auto arg) {
+        auto launch = [&](const void *fn, void *proposal_arg, bool first) {
+            const PatchView *view = &pv;
+            void *tail[] = {&p->d_gtab, &p->d_gbox, &p->d_tile_cost, &p->n_tiles, &order,
+                            &p->d_tile_counter, &p->d_err};
+            void *args[9];
+            args[first ? 0 : 1] = proposal_arg;
+            args[first ? 1 : 0] = (void *)view;
+            std::copy(tail, tail + 7, args + 2);
+            return launch_dependent(fn, grid, dim3(PREP_THREADS), args, 0, s);
+        };
+        auto with_arg = [&](auto arg, const void *fn) {
             std::memcpy(arg.s, prop, sizeof(fpho_source) * p->n_sources);
-            prepare_evaluation_arg<<<grid, PREP_THREADS, 0, s>>>(
-                arg, pv, p->d_gtab, p->d_gbox, p->d_tile_cost, p->n_tiles, order,
-                p->d_tile_counter, p->d_err);
+            return launch(fn, &arg, true);
         };
         if (!host_prop)
-            prepare_evaluation<<<grid, PREP_THREADS, 0, s>>>(pv, prop, p->d_gtab, p->d_gbox,
-                                                             p->d_tile_cost, p->n_tiles, order,
-                                                             p->d_tile_counter, p->d_err);
+            CUDA_TRY(launch((const void *)prepare_evaluation, (void *)&prop, false));
         else if (p->n_sources <= 4)
-            with_arg(ProposalArg<4>());
+            CUDA_TRY(with_arg(ProposalArg<4>(), (const void *)prepare_evaluation_arg<4>));
         else if (p->n_sources <= 15)
-            with_arg(ProposalArg<15>());
+            CUDA_TRY(with_arg(ProposalArg<15>(), (const void *)prepare_evaluation_arg<15>));
         else
-            with_arg(ProposalArg<MAX_ARG_SOURCES>());
-        CUDA_TRY(cudaGetLastError());
+            CUDA_TRY(with_arg(ProposalArg<MAX_ARG_SOURCES>(),
+                              (const void *)prepare_evaluation_arg<MAX_ARG_SOURCES>));
     }
     TileArgs A;
     A.pv = pv;

@@ -139,6 +139,7 @@ __device__ __forceinline__ void prepare_body(const PatchView &pv, const fpho_sou
                                              float *gtab, float4 *gbox, const int *cost,
                                              int n_tiles, int *order, int *counter, int *err) {
     let_next_kernel_start();
+    wait_for_earlier_kernel();  // the proposal, and the last evaluation's readers
     if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) *err = 0;
     const int e = blockIdx.y;
     if (e == pv.n_exp) {

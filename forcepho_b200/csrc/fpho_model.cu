@@ -165,6 +165,7 @@ __global__ void __launch_bounds__(PROP_THREADS) proposal_kernel(
     int n_bands, const int *src_bands, const long long *src_off, double *q_out,
     fpho_source *out) {
     __shared__ double s_tx[SPL_MAX_KNOTS], s_ty[SPL_MAX_KNOTS];
+    let_next_kernel_start();
     const SplineView L = knots_to_shared(S, s_tx, s_ty);
     const int lane = threadIdx.x & 31;
     const int s = blockIdx.x * (PROP_THREADS / 32) + (threadIdx.x >> 5);
