@@ -681,7 +681,7 @@ struct PinnedBlock {
     void *p;
     size_t bytes;
 };
-constexpr size_t PINNED_KEEP = 16, PINNED_KEEP_BYTES = 1 << 20;
+constexpr size_t PINNED_KEEP = 16;
 std::mutex g_pinned_mu;
 std::vector<PinnedBlock> g_pinned;
 }  // namespace
@@ -893,9 +893,18 @@ extern "C" int fpho_patch_retrieve(fpho_patch *p, int which, float *host_out, vo
     }
     if (!src) return set_error(FPHO_ERR_STATE, "array %d is not allocated", which);
     cudaStream_t s = (cudaStream_t)stream;
-    CUDA_TRY(cudaMemcpyAsync(host_out, src, (size_t)p->npix * sizeof(float),
-                             cudaMemcpyDeviceToHost, s));
-    CUDA_TRY(cudaStreamSynchronize(s));
+    const size_t bytes = (size_t)p->npix * sizeof(float);
+    // an array that fits a kept pinned block goes through one: a transfer to
+    // pageable memory costs more than this one and the copy after it
+    void *pin = nullptr;
+    size_t cap = bytes;
+    if (bytes <= PINNED_KEEP_BYTES) CUDA_TRY(pinned_get(&pin, &cap));
+    cudaError_t ce = cudaMemcpyAsync(pin ? pin : host_out, src, bytes, cudaMemcpyDeviceToHost, s);
+    if (ce == cudaSuccess) ce = cudaStreamSynchronize(s);
+    if (ce == cudaSuccess && pin) std::memcpy(host_out, pin, bytes);
+    if (pin) pinned_put(pin, cap);
+    if (ce != cudaSuccess)
+        return set_error(FPHO_ERR_CUDA, "copy of a pixel array: %s", cudaGetErrorString(ce));
     return FPHO_OK;
 }
 

@@ -58,6 +58,7 @@ PatchView make_view(const fpho_patch *p);
 // freed): allocating and freeing one took from 0.1 to 13 ms beside other
 // allocations.  `bytes`: in, the least needed; out, the block's size, which
 // pinned_put is told.
+constexpr size_t PINNED_KEEP_BYTES = 1 << 20;
 cudaError_t pinned_get(void **p, size_t *bytes);
 void pinned_put(void *p, size_t bytes);
 cudaError_t pool_malloc(void **p, size_t bytes);
