@@ -16,7 +16,7 @@ Printed JSON (rank 0):
              timed per step with an L2 flush between steps (max over ranks);
   e2e        the same through GPUProposer.evaluate_proposal with the proposal
              in pinned host memory and results copied back every step;
-  roofline   the pixel-tile kernel: algorithmic FP32 flops (105 per evaluated
+  roofline   the pixel-tile kernel: FP32 flops of its two passes (53 per evaluated
              pixel-Gaussian pair) / its CUDA-event time, against the FP32 FMA
              throughput measured live by a probe kernel on the same GPU;
   cpu_baseline  the reference's own CPU kernel (built from its sources into
@@ -44,7 +44,9 @@ ROOT = os.path.dirname(os.path.abspath(__file__))
 sys.path.insert(0, ROOT)
 
 METRIC = "chi2+grad evals/s & pix·gauss/s: batched vs plain, 1 B200, rel err ≤1e-6"
-FLOPS_PER_PAIR = 105          # 18 (model) + 87 (gradient) FP32 flops, FMA = 2
+# FP32 flops per evaluated pair, FMA = 2: 36 of the residual pass (18 of them the
+# exponential) and 17 of the gradient pass (its sums shared along pixel runs)
+FLOPS_PER_PAIR = 53
 WORKLOAD = "field20: 20 src, 8 bands x 4 exp x 128x128 px, 5-gauss PSF, 9 radii"
 # DRAM bytes (read + write) of one tile-kernel launch on this workload, from an
 # ncu capture of one launch of the split tile kernel: the 16 B per pixel of the
@@ -148,6 +150,17 @@ class ClockSampler:
 
 
 # ------------------------------------------------------------------ CPU reference
+NO_REFERENCE = "the reference CPU kernel (oracle/_ref) is not built: its sources are absent"
+
+
+def have_reference(n_sources):
+    """Whether the reference CPU kernel is built, or can be built here."""
+    from oracle import oracle as O
+    if not O.ref_available(n_sources):
+        O.build()
+    return O.ref_available(n_sources)
+
+
 def cpu_reference_time(P, prop, reps, cores):
     """Seconds per full evaluation (all bands) of the reference CPU kernel,
     bands spread over `cores` spawn worker processes."""
@@ -214,6 +227,9 @@ def run_reference(args):
     if rank != 0:
         return 0
     P = make_workload(args.seed, device_render=False)
+    if not have_reference(P.n_sources):
+        print(json.dumps({"impl": "reference", "unavailable": NO_REFERENCE}), flush=True)
+        return 0
     prop = P.proposal()
     cores = len(os.sched_getaffinity(0))
     times = cpu_reference_time(P, prop, args.warmup + args.steps, min(cores, P.n_bands))
@@ -933,7 +949,9 @@ def run_ours(args):
         packing = packing_leg(args, torch, args.packing_patches)
 
     cpu = None
-    if rank == 0 and world == 1 and not args.no_cpu_baseline:
+    if rank == 0 and world == 1 and not args.no_cpu_baseline and not have_reference(P.n_sources):
+        cpu = {"value": None, "kind": "reference", "unavailable": NO_REFERENCE}
+    elif rank == 0 and world == 1 and not args.no_cpu_baseline:
         cores = len(os.sched_getaffinity(0))
         use = min(cores, nb)
         times = cpu_reference_time(P, prop, 5, use)
