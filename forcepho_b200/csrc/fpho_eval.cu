@@ -1,11 +1,15 @@
 // fpho_eval.cu -- patch handles and single-patch evaluation behind the C ABI
 // of include/fpho.h.
 //
-// Per evaluation, three kernels run on the caller's stream:
-//   build_image_gaussians  one thread per image Gaussian (exposure, source, PSF
+// Per evaluation, three kernels run on the caller's stream, each started while
+// the one before it ends (launch_dependent):
+//   prepare_evaluation     one thread per image Gaussian (exposure, source, PSF
 //                          component): record + culling box into the workspace;
-//   tile_kernel<NT,K>      one CTA per pixel tile (fpho_tile.cuh);
-//   reduce_bands           FP64 sum of the tile partials of each band.
+//                          small proposals arrive in the launch's arguments;
+//   split_kernel*, tile_kernel*   one CTA per pixel tile or part of one, or
+//                          persistent CTAs over them (fpho_tile.cuh);
+//   reduce_bands           FP64 sum of the partials of each band, written to the
+//                          caller's device buffers or to pinned host memory.
 #include <cuda_runtime.h>
 
 #include <algorithm>
