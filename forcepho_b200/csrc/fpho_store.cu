@@ -114,6 +114,7 @@ struct fpho_store {
     size_t h_par_bytes = 0;
     Params par = {};                  // where they are
     unsigned long long serial = 0;    // count passes so far
+    int counted = 0;                  // exposures of the last one
     // optional CUDA-event timing of the gather kernel
     bool time_gather = false;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
@@ -468,6 +469,7 @@ int count_pass(fpho_store *st, int n_exp, const int32_t *exposures, const fpho_r
             return set_error(FPHO_ERR_INVALID, "region %d: unknown kind %d", e, regions[e].kind);
     }
     ++st->serial;
+    st->counted = n_exp;
     int rc = ensure_params(st, n_exp);
     if (rc) return rc;
     const Params &P = st->par;
@@ -661,8 +663,11 @@ extern "C" int fpho_store_gather_end(fpho_store *st, uint64_t ticket, int n_exp,
     clear_error();
     if (!st || !exposure_start || !exposure_N)
         return set_error(FPHO_ERR_INVALID, "NULL argument");
-    if (ticket != st->serial || n_exp < 1 || n_exp > st->scratch_exp)
+    if (ticket != st->serial)
         return set_error(FPHO_ERR_STATE, "another count or gather came between the two halves");
+    if (n_exp != st->counted)
+        return set_error(FPHO_ERR_INVALID, "n_exp=%d but %d exposures were counted", n_exp,
+                         st->counted);
     ++st->serial;  // a ticket is good once
     return pack_pass(st, n_exp, background, max_snr, data, ierr, xpix, ypix, npix_capacity,
                      exposure_start, exposure_N, (cudaStream_t)stream);

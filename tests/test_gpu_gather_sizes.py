@@ -110,3 +110,23 @@ def test_gather_halves():
             end()
         assert exc.value.code == _lib.FPHO_ERR_STATE
     st.free()
+
+
+@pytest.mark.parametrize("n_exp", [0, 1, 3])
+def test_gather_halves_of_different_lengths_are_refused(n_exp):
+    import torch
+    from forcepho_b200 import _lib
+    st, _, rng = store(8, 256, 4)
+    idx = np.arange(4, dtype=np.int32)
+    st.count(idx, circles(idx, 256, [30.0], rng))      # four exposures' totals are about
+    npix, ticket = ctypes.c_int64(), ctypes.c_uint64()
+    recs = circles(idx[:2], 256, [30.0], rng)
+    _lib.call("fpho_store_gather_begin", st.handle, 2, idx.ctypes.data, recs.ctypes.data,
+              ctypes.byref(npix), ctypes.byref(ticket), None)
+    bufs = [torch.zeros(npix.value, device="cuda") for _ in range(4)]
+    start, n = np.zeros(4, np.int32), np.zeros(4, np.int32)
+    with pytest.raises(_lib.FphoError, match="exposures were counted"):
+        _lib.call("fpho_store_gather_end", st.handle, ticket, n_exp, None, 0.0,
+                  *[b.data_ptr() for b in bufs], npix.value, start.ctypes.data, n.ctypes.data,
+                  None)
+    st.free()
