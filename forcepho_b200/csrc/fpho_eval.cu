@@ -898,11 +898,14 @@ extern "C" int fpho_patch_retrieve(fpho_patch *p, int which, float *host_out, vo
     if (!src) return set_error(FPHO_ERR_STATE, "array %d is not allocated", which);
     cudaStream_t s = (cudaStream_t)stream;
     const size_t bytes = (size_t)p->npix * sizeof(float);
-    // an array that fits a kept pinned block goes through one: a transfer to
-    // pageable memory costs more than this one and the copy after it
+    // pageable memory that fits a kept pinned block is filled through one: a
+    // transfer to it costs more than one to the block and the copy after it
     void *pin = nullptr;
     size_t cap = bytes;
-    if (bytes <= PINNED_KEEP_BYTES) CUDA_TRY(pinned_get(&pin, &cap));
+    cudaPointerAttributes at;
+    CUDA_TRY(cudaPointerGetAttributes(&at, host_out));
+    if (bytes <= PINNED_KEEP_BYTES && at.type == cudaMemoryTypeUnregistered)
+        CUDA_TRY(pinned_get(&pin, &cap));
     cudaError_t ce = cudaMemcpyAsync(pin ? pin : host_out, src, bytes, cudaMemcpyDeviceToHost, s);
     if (ce == cudaSuccess) ce = cudaStreamSynchronize(s);
     if (ce == cudaSuccess && pin) std::memcpy(host_out, pin, bytes);
@@ -1163,7 +1166,25 @@ extern "C" int fpho_evaluate_proposal(fpho_patch *p, const fpho_source *proposal
         p->h_io_cap = cap;
     }
     unsigned char *io = p->h_io;
-    const bool in_args = n_sources <= MAX_ARG_SOURCES;
+    bool in_args = n_sources <= MAX_ARG_SOURCES;
+    if (in_args) {
+        // Memory that the device can write (pinned, managed) may still get its
+        // proposal from work in `s`: the transfer waits for that.  Pageable
+        // memory is read now, as a transfer would; device memory, which is not
+        // what the flag says, is left to the transfer.
+        cudaPointerAttributes at;
+        CUDA_TRY(cudaPointerGetAttributes(&at, proposal));
+        if (at.type == cudaMemoryTypeDevice) {
+            in_args = false;
+        } else if (at.type != cudaMemoryTypeUnregistered) {
+            const cudaError_t busy = cudaStreamQuery(s);
+            if (busy == cudaErrorNotReady)
+                cudaGetLastError();  // not an error, but kept as the last one
+            else
+                CUDA_TRY(busy);
+            in_args = busy == cudaSuccess;
+        }
+    }
     if (!in_args)
         CUDA_TRY(cudaMemcpyAsync(p->d_prop, proposal, sizeof(fpho_source) * n_sources,
                                  cudaMemcpyHostToDevice, s));
