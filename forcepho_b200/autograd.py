@@ -123,7 +123,8 @@ class LnLike(torch.autograd.Function):
         shape = ctx.saved_tensors[0].shape
         g = g.contiguous()
         try:
-            plain = g.dtype == torch.float64 and g.is_cuda and g.data_ptr() != 0
+            plain = (g.dtype == torch.float64 and g.is_cuda and not g.is_neg()
+                     and g.data_ptr() != 0)
         except RuntimeError:    # a batched gradient has no storage of its own
             plain = False
         if torch.is_grad_enabled() or not plain:

@@ -98,3 +98,18 @@ def test_lnlike_gradient_forms(ns, nb):
     (dw,) = torch.autograd.grad(gc.sum(), w)
     torch.testing.assert_close(dw, want.sum(), rtol=1e-12, atol=0)
     P.free()
+
+
+def test_lnlike_gradient_of_a_lazy_negative():
+    """An upstream gradient whose sign is a flag on the tensor, not in memory."""
+    import torch
+    from forcepho_b200.autograd import PatchEvaluator, lnlike
+    P = patch(2, [1], [(24, 24)], 2, seed=61)
+    P.send_to_device()
+    ev = PatchEvaluator(P)
+    theta = torch.tensor(P.params, dtype=torch.float64, device="cuda", requires_grad=True)
+    up = torch.tensor(1.0 + 2.0j, dtype=torch.complex128, device="cuda").conj().imag
+    assert up.is_neg() and float(up) == -2.0
+    (g,) = torch.autograd.grad(lnlike(theta, ev), theta, up)
+    torch.testing.assert_close(g, ev.stacked(), rtol=1e-14, atol=0)
+    P.free()
