@@ -1055,7 +1055,20 @@ int enqueue_evaluate(fpho_patch *p, const fpho_source *prop, double *d_chi2, flo
     if (p->count_pairs) CUDA_TRY(cudaMemsetAsync(p->d_pairs, 0, sizeof(long long), s));
     const PatchView pv = make_view(p);
     // the order only matters when the tiles outnumber what runs at once
-    const bool ordered = p->schedule == 1 && p->n_tiles > 4 * device_sms();
+    const int sms = device_sms();
+    const bool ordered = p->schedule == 1 && p->n_tiles > 4 * sms;
+    // one CTA per tile otherwise, or per part of one (the exact mode has no parts)
+    const int parts =
+        p->exact_residual ? 1 : std::min(tile_parts(p->variant, p->n_tiles), p->max_parts);
+    // The tile kernel's CTAs may start beside the first kernel's, which saves
+    // 2 us, but then go where those leave room, unevenly.  CTAs that fill the SMs
+    // to the same number each cannot spare that and start after it: 144 tiles of
+    // 30 sources 108 against 135 us, 432 tiles of 20 sources 115 against 124
+    // (chi2 only 63.5 against 69.6; none to 12 SMs short of even).  With more
+    // room early is better: 224 tiles 37.9 against 39.6, 264 quarters 29.7
+    // against 30.2, 448 tiles 98 against 100 (32 SMs short and more).
+    const int ctas = p->n_tiles * parts;
+    bool early = ordered || (sms - ctas % sms) % sms >= sms / 8;
     {
         // image Gaussians, the tile order and the error word in one launch
         dim3 grid(std::max((p->max_g + PREP_THREADS - 1) / PREP_THREADS, 1),
@@ -1064,11 +1077,11 @@ int enqueue_evaluate(fpho_patch *p, const fpho_source *prop, double *d_chi2, flo
         auto launch = [&](const void *fn, void *proposal_arg, bool first) {
             const PatchView *view = &pv;
             void *tail[] = {&p->d_gtab, &p->d_gbox, &p->d_tile_cost, &p->n_tiles, &order,
-                            &p->d_tile_counter, &p->d_err};
-            void *args[9];
+                            &p->d_tile_counter, &p->d_err, &early};
+            void *args[10];
             args[first ? 0 : 1] = proposal_arg;
             args[first ? 1 : 0] = (void *)view;
-            std::copy(tail, tail + 7, args + 2);
+            std::copy(tail, tail + 8, args + 2);
             return launch_dependent(fn, grid, dim3(PREP_THREADS), args, 0, s);
         };
         auto with_arg = [&](auto arg, const void *fn) {
@@ -1103,9 +1116,6 @@ int enqueue_evaluate(fpho_patch *p, const fpho_source *prop, double *d_chi2, flo
     A.tile_misfit = p->d_tile_misfit;
     A.runs = p->d_runs;
     A.test_extra_tx = p->test_extra_tx;
-    // one CTA per tile otherwise, or per part of one (the exact mode has no parts)
-    const int parts =
-        p->exact_residual ? 1 : std::min(tile_parts(p->variant, p->n_tiles), p->max_parts);
     if (p->ev_tile0) CUDA_TRY(cudaEventRecord(p->ev_tile0, s));
     int rc;
     if (ordered) {

@@ -137,8 +137,9 @@ __device__ __forceinline__ void order_tiles_body(const int *cost, int n_tiles, i
 constexpr int PREP_THREADS = 1024;
 __device__ __forceinline__ void prepare_body(const PatchView &pv, const fpho_source *src,
                                              float *gtab, float4 *gbox, const int *cost,
-                                             int n_tiles, int *order, int *counter, int *err) {
-    let_next_kernel_start();
+                                             int n_tiles, int *order, int *counter, int *err,
+                                             bool early) {
+    if (early) let_next_kernel_start();
     wait_for_earlier_kernel();  // the proposal, and the last evaluation's readers
     if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) *err = 0;
     const int e = blockIdx.y;
@@ -156,8 +157,8 @@ __device__ __forceinline__ void prepare_body(const PatchView &pv, const fpho_sou
 }
 static __global__ void __launch_bounds__(PREP_THREADS) prepare_evaluation(
     PatchView pv, const fpho_source *src, float *gtab, float4 *gbox, const int *cost, int n_tiles,
-    int *order, int *counter, int *err) {
-    prepare_body(pv, src, gtab, gbox, cost, n_tiles, order, counter, err);
+    int *order, int *counter, int *err, bool early) {
+    prepare_body(pv, src, gtab, gbox, cost, n_tiles, order, counter, err, early);
 }
 // The same with the proposal in the launch itself, for one that comes from
 // host memory: no transfer, and the caller's array is read when the call
@@ -169,8 +170,8 @@ struct ProposalArg {
 template <int N>
 static __global__ void __launch_bounds__(PREP_THREADS) prepare_evaluation_arg(
     const __grid_constant__ ProposalArg<N> prop, PatchView pv, float *gtab, float4 *gbox,
-    const int *cost, int n_tiles, int *order, int *counter, int *err) {
-    prepare_body(pv, prop.s, gtab, gbox, cost, n_tiles, order, counter, err);
+    const int *cost, int n_tiles, int *order, int *counter, int *err, bool early) {
+    prepare_body(pv, prop.s, gtab, gbox, cost, n_tiles, order, counter, err, early);
 }
 
 // Sums of tile partials in double, for reduce_bands and batch_reduce alike (a
