@@ -750,9 +750,11 @@ __device__ __forceinline__ int scan_tile(const TileArgs &A, float4 bb, int g0, i
                                *reinterpret_cast<const float4 *>(r + 4), r[R_FYY], bb))
                     atomicOr(&mask[(at - b0) >> 5], 1u << ((at - b0) & 31));
             }
-            const int next = lane + 32 < queued ? queue[lane + 32] : 0;
-            __syncwarp();
-            queue[lane] = next;
+            const bool more = lane + 32 < queued;
+            const int next = more ? queue[lane + 32] : 0;
+            __syncwarp();  // every slot is read before it is filled again,
+            if (more) queue[lane] = next;
+            __syncwarp();  // and this is in place before another lane queues
             queued = max(queued - 32, 0);
         };
 #pragma unroll 2
