@@ -12,10 +12,10 @@
 //      reference's Gaussian order (ComputeResidualImage, common_kernel.cc:57-83);
 //   4. chi2 per pixel in double, exactly as compute_gaussians_kernel.cc:286-293;
 //   5. gradient pass, one kept Gaussian per lane (gradient_lanes): each lane
-//      walks the tile's pixels, broadcast from shared memory, and sums the
-//      moments of its Gaussian's weight; the derivatives of the model w.r.t.
-//      the Gaussian's image-space parameters (A, x, y, fxx, fyy, fxy) and the
-//      Gaussian's Jacobian are formed from them once
+//      walks the tile's pixels, broadcast from shared memory, and forms the
+//      twelve sums of its Gaussian's weight from which the derivatives of the
+//      model w.r.t. the Gaussian's image-space parameters (A, x, y, fxx, fyy,
+//      fxy) and, through its Jacobian, w.r.t. the source's follow
 //      (ComputeGaussianDerivative, common_kernel.cc:95-143, with the per-pixel
 //      Jacobian product moved out of the pixel loop);
 //   6. per-source sums are reduced across the warp and the CTA in a fixed
@@ -440,170 +440,222 @@ __device__ __forceinline__ void stage_runs(const TileArgs &A, const TileDesc &td
     }
 }
 
-// Moments of one Gaussian's weight W = r2 G over pixels: m[a][b] = sum W du^a
-// dv^b, a + b <= 4, (u, v) the coordinate along the runs and the shared one.
-struct Moments {
-    float m00 = 0.f, m10 = 0.f, m20 = 0.f, m30 = 0.f, m40 = 0.f, m01 = 0.f, m11 = 0.f, m21 = 0.f,
-          m31 = 0.f, m02 = 0.f, m12 = 0.f, m22 = 0.f, m03 = 0.f, m13 = 0.f, m04 = 0.f;
-    // adds one run's moments along u (s_a = sum W du^a) at its dv
-    __device__ __forceinline__ void add(float dv, float dv2, float s0, float s1, float s2,
-                                        float s3, float s4) {
-        const float dv3 = dv2 * dv, dv4 = dv2 * dv2;
-        m00 += s0;
-        m10 += s1;
-        m20 += s2;
-        m30 += s3;
-        m40 += s4;
-        m01 = fmaf(dv, s0, m01);
-        m11 = fmaf(dv, s1, m11);
-        m21 = fmaf(dv, s2, m21);
-        m31 = fmaf(dv, s3, m31);
-        m02 = fmaf(dv2, s0, m02);
-        m12 = fmaf(dv2, s1, m12);
-        m22 = fmaf(dv2, s2, m22);
-        m03 = fmaf(dv3, s0, m03);
-        m13 = fmaf(dv3, s1, m13);
-        m04 = fmaf(dv4, s0, m04);
-    }
-    // adds moments `c` taken about a point d further along u
-    __device__ __forceinline__ void add_shifted(const Moments &c, float d) {
-        const float d2 = d * d, d3 = d2 * d, d4 = d2 * d2;
-        m00 += c.m00;
-        m10 += fmaf(d, c.m00, c.m10);
-        m20 += fmaf(d2, c.m00, fmaf(2.0f * d, c.m10, c.m20));
-        m30 += fmaf(d3, c.m00, fmaf(3.0f * d2, c.m10, fmaf(3.0f * d, c.m20, c.m30)));
-        m40 += fmaf(d4, c.m00, fmaf(4.0f * d3, c.m10, fmaf(6.0f * d2, c.m20,
-                                                         fmaf(4.0f * d, c.m30, c.m40))));
-        m01 += c.m01;
-        m11 += fmaf(d, c.m01, c.m11);
-        m21 += fmaf(d2, c.m01, fmaf(2.0f * d, c.m11, c.m21));
-        m31 += fmaf(d3, c.m01, fmaf(3.0f * d2, c.m11, fmaf(3.0f * d, c.m21, c.m31)));
-        m02 += c.m02;
-        m12 += fmaf(d, c.m02, c.m12);
-        m22 += fmaf(d2, c.m02, fmaf(2.0f * d, c.m12, c.m22));
-        m03 += c.m03;
-        m13 += fmaf(d, c.m03, c.m13);
-        m04 += c.m04;
+// The sums over pixels that the derivatives of one Gaussian need, with the
+// weight W = r2 G, the offset (du, dv) from its centre, v = F (du, dv) and the
+// pixel correction H: of W H (1, vu, vv, du^2, du dv, dv^2), and of W the same.
+template <typename T>
+struct GradSums {
+    T h0 = 0, hu = 0, hv = 0, huu = 0, huv = 0, hvv = 0;
+    T w0 = 0, wu = 0, wv = 0, wuu = 0, wuv = 0, wvv = 0;
+    __device__ __forceinline__ void add(const GradSums<float> &o) {
+        h0 += o.h0; hu += o.hu; hv += o.hv; huu += o.huu; huv += o.huv; hvv += o.hvv;
+        w0 += o.w0; wu += o.wu; wv += o.wv; wuu += o.wuu; wuv += o.wuv; wvv += o.wvv;
     }
 };
 
-// One Gaussian in a lane: the exponent's quadratic form in (du, dv), scaled so
-// that G = 2^E.
+// One Gaussian in a lane.  Along a run (u) at offset dv the exp-argument is
+//   fuu t^2 + 2 fx t dv + k dv^2,  t = du + rq dv,
+// rq being fuv / fuu to the nearest half: fx = fuv - rq fuu is small, so that
+// nothing cancels for a long thin Gaussian, and t has no more bits than the
+// offsets, so that it is exact where they are.  (In du and dv the three terms
+// cancel, and each coefficient's rounding is the same at every pixel: that
+// error does not average out.)  vu = fuu t + fx dv and vv = fuv t + kv dv.
 struct LaneForm {
-    float nu, nv;      // -centre
-    float e20, e11, e02;
+    float nu, nv;            // -centre
+    float fuu, rq, fx, k;
+    float hA, h11, h02, c0;  // H = hA t^2 + h11 t dv + h02 dv^2 + c0
+    __device__ __forceinline__ LaneForm(float nu_, float nv_, float fuu_, float fuv, float fvv,
+                                        float c0_)
+        : nu(nu_), nv(nv_), fuu(fuu_), c0(c0_) {
+        rq = fuu > 0.0f ? 0.5f * rintf(2.0f * fuv / fuu) : 0.0f;
+        const double x = (double)fuv - (double)rq * fuu, y = (double)fvv - (double)rq * fuv;
+        const float kv = (float)y;
+        fx = (float)x;
+        k = (float)(y - rq * x);
+        hA = (fuu * fuu + fuv * fuv) * (1.0f / 24.0f);
+        h11 = (fuu * fx + fuv * kv) * (1.0f / 12.0f);
+        h02 = (fx * fx + kv * kv) * (1.0f / 24.0f);
+    }
+    // the sums with vu and vv, from those with t and dv in their place
+    __device__ __forceinline__ void finish(GradSums<double> &m, float fuv, float fvv) const {
+        const double kv = (double)fvv - (double)rq * fuv;
+        const double ht = m.hu, wt = m.wu;
+        m.hu = fuu * ht + fx * m.hv;
+        m.hv = fuv * ht + kv * m.hv;
+        m.wu = fuu * wt + fx * m.wv;
+        m.wv = fuv * wt + kv * m.wv;
+    }
 };
-constexpr float E_CUT = FPHO_MAX_EXP_ARG * KEXP;  // exp-arguments above 36: E below this
-// F along the run above which moments are not taken about the run's middle (a
-// Gaussian narrower than a pixel: with the middle used for all, the error of
-// the q gradient against 64 bits tripled on one patch of eleven, 4.8e-6 to
-// 1.4e-5; up to F = 2 no gradient column's error changed).
-constexpr float NARROW = 1.0f;
+// F along the run above which the sums along a run are not taken about its
+// middle (a Gaussian not much wider than a pixel).  The error of the sums of one
+// Gaussian against double, in those of a kernel that forms every derivative at
+// every pixel, over PSF components of 1 to 2 pixels: 0.9 with 1/4, 1.2 with 1/2,
+// 1.3 with 1; the 20-source patch takes 333, 331 and 329 us.
+constexpr float NARROW = 0.25f;
 
 // A slot of the staged weights: the second half of a run is staged in reverse
 // (pixels 0 1 2 3 7 6 5 4), so that the packed pairs 0 and 2, 1 and 3 of a run
 // hold mirror pixels.
 __device__ __forceinline__ int run_slot(int p) { return (p & 4) ? (p ^ 3) : p; }
 
-// Moments over the runs [r0, r1).  Along a run the exponent is a quadratic in
-// du whose coefficients are formed once per run, and the weight's moments in
-// du are summed before they meet dv.
+// Sums over the runs [r0, r1).  The sums s_a = sum W t^a (a <= 4) of a run give
+// all twelve of its sums, since H is a quadratic in t there.  They are added up
+// eight runs at a time in float, then in double: a lane walks up to 256 pixels,
+// and a float sum of that length loses what a sum over 32 lanes does not.
 //
-// CENTRED: the moments along a run are taken about the run's middle, where the
-// offsets are the constants -7/2 ... 7/2 and mirror pixels share their even and
-// negate their odd powers, and are shifted to the Gaussian's centre once for
-// all runs that start at the same u: 12 packed and 35 scalar instructions per
-// run against 44 packed and 5 scalar ones (20-source patch 334 -> 309 us,
-// 60-source patch 6.57 -> 6.19 ms).  Rounding is then relative to W (7/2)^a, not to
-// W du^a, so this form is for Gaussians wide enough along the run that the two
-// compare (NARROW below).
+// CENTRED: s_a is taken about the run's middle, where the offsets are the
+// constants -7/2 ... 7/2 and mirror pixels share their even and negate their odd
+// powers, and then moved by the middle's offset.  Rounding is then relative to
+// W (7/2)^a, not to W t^a, so this form is for Gaussians wide enough along the
+// run that the two compare (NARROW above).
+//
+// Moments about the centre up to the fourth order, in du and dv and all in float,
+// took 30 us less of the 20-source patch's 333 and 600 less of the 60-source
+// patch's 6500, but their error against double was up to three times that of
+// derivatives formed at every pixel for PSF components, ten for q = 0.2 (here:
+// 0.4 to 1.1 times).
 template <bool CENTRED>
-__device__ __forceinline__ void run_moments(const PixelStage &px, int r0, int r1,
-                                            const LaneForm &f, Moments &m) {
-    const v2 E20 = pk1(f.e20);
-    Moments c;           // about the runs' middle
-    float u0 = px.ru[r0];
+__device__ __forceinline__ void run_sums(const PixelStage &px, int r0, int r1, const LaneForm &f,
+                                         GradSums<double> &m) {
+    const v2 FUU = pk1(f.fuu), KEXP2 = pk1(KEXP);
 #pragma unroll 1
-    for (int r = r0; r < r1; ++r) {
-        const float u = px.ru[r];
-        if (CENTRED && u != u0) {  // (the same in every lane)
-            m.add_shifted(c, (u0 + f.nu) + 3.5f);
-            c = Moments();
-            u0 = u;
-        }
-        const float dv = px.rv[r] + f.nv;
-        const float dv2 = dv * dv;
-        const float d = u + f.nu;
-        const v2 E11 = pk1(f.e11 * dv), E02 = pk1(f.e02 * dv2);
-        v2 W[4];
-        ld2(px.r2 + 8 * r, W[0], W[1]);
-        ld2(px.r2 + 8 * r + 4, W[2], W[3]);
-        v2 DU[4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const float k0 = j < 2 ? 2.0f * j : 11.0f - 2.0f * j;
-            DU[j] = pk(d + k0, d + (j < 2 ? k0 + 1.0f : k0 - 1.0f));
-            float e0, e1;
-            unpk(fma2(fma2(E20, DU[j], E11), DU[j], E02), e0, e1);
-            const float g0 = e0 < E_CUT ? 0.0f : ex2f(e0);
-            const float g1 = e1 < E_CUT ? 0.0f : ex2f(e1);
-            W[j] = mul2(W[j], pk(g0, g1));
-        }
-        if (CENTRED) {
-            // sums and differences of mirror pixels, 7/2 5/2 and 3/2 1/2 off the
-            // middle; scalars, whose constants are immediates (as packed
-            // operands they would take sixteen registers)
-            const v2 NEG = pk1(-1.0f);
-            float a, b, g, h, p, q, s, t;
-            unpk(add2(W[2], W[0]), a, b);
-            unpk(add2(W[3], W[1]), g, h);
-            unpk(fma2(W[0], NEG, W[2]), p, q);
-            unpk(fma2(W[1], NEG, W[3]), s, t);
-            c.add(dv, dv2, (a + b) + (g + h),
-                  fmaf(3.5f, p, fmaf(2.5f, q, fmaf(1.5f, s, 0.5f * t))),
-                  fmaf(12.25f, a, fmaf(6.25f, b, fmaf(2.25f, g, 0.25f * h))),
-                  fmaf(42.875f, p, fmaf(15.625f, q, fmaf(3.375f, s, 0.125f * t))),
-                  fmaf(150.0625f, a, fmaf(39.0625f, b, fmaf(5.0625f, g, 0.0625f * h))));
-        } else {
-            v2 S0, S1, S2, S3, S4;
+    for (int r = r0; r < r1;) {
+        const int end = min(r1, (r | 7) + 1);
+        GradSums<float> c;  // hu, hv, wu, wv: sums with t and dv in the place of vu and vv
+#pragma unroll 1
+        for (; r < end; ++r) {
+            const float dv = px.rv[r] + f.nv, dv2 = dv * dv;
+            const float d = (px.ru[r] + f.nu) + 3.5f;  // the run's middle: du, t
+            const float t = fmaf(f.rq, dv, d);
+            const v2 Q1 = pk1(2.0f * f.fx * dv), Q0 = pk1(f.k * dv2);
+            v2 W[4], T[4];
+            ld2(px.r2 + 8 * r, W[0], W[1]);
+            ld2(px.r2 + 8 * r + 4, W[2], W[3]);
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
-                const v2 T1 = mul2(W[j], DU[j]), T2 = mul2(T1, DU[j]), T3 = mul2(T2, DU[j]);
-                S0 = j ? add2(S0, W[j]) : W[j];
-                S1 = j ? add2(S1, T1) : T1;
-                S2 = j ? add2(S2, T2) : T2;
-                S3 = j ? add2(S3, T3) : T3;
-                S4 = j ? fma2(T3, DU[j], S4) : mul2(T3, DU[j]);
+                const float z = j < 2 ? 2.0f * j - 3.5f : 7.5f - 2.0f * j;
+                T[j] = pk(t + z, t + (j < 2 ? z + 1.0f : z - 1.0f));
+                const v2 Q = fma2(fma2(FUU, T[j], Q1), T[j], Q0);
+                float q0, q1, e0, e1;
+                unpk(Q, q0, q1);
+                unpk(mul2(Q, KEXP2), e0, e1);
+                W[j] = mul2(W[j], pk(q0 > FPHO_MAX_EXP_ARG ? 0.0f : ex2f(e0),
+                                     q1 > FPHO_MAX_EXP_ARG ? 0.0f : ex2f(e1)));
             }
-            m.add(dv, dv2, lanesum(S0), lanesum(S1), lanesum(S2), lanesum(S3), lanesum(S4));
+            const float hB = f.h11 * dv, hC = fmaf(f.h02, dv2, f.c0);
+            float s0, st, suu, su, p0, pt, puu, pu;
+            if (CENTRED) {
+                // sums and differences of mirror pixels, 7/2 5/2 and 3/2 1/2 off
+                // the middle; scalars, whose constants are immediates (as packed
+                // operands they would take sixteen registers)
+                const v2 NEG = pk1(-1.0f);
+                float a0, a1, a2, a3, b0, b1, b2, b3;
+                unpk(add2(W[2], W[0]), a0, a1);
+                unpk(add2(W[3], W[1]), a2, a3);
+                unpk(fma2(W[0], NEG, W[2]), b0, b1);
+                unpk(fma2(W[1], NEG, W[3]), b2, b3);
+                const float z0 = (a0 + a1) + (a2 + a3);
+                const float z1 = fmaf(3.5f, b0, fmaf(2.5f, b1, fmaf(1.5f, b2, 0.5f * b3)));
+                const float z2 = fmaf(12.25f, a0, fmaf(6.25f, a1, fmaf(2.25f, a2, 0.25f * a3)));
+                const float z3 =
+                    fmaf(42.875f, b0, fmaf(15.625f, b1, fmaf(3.375f, b2, 0.125f * b3)));
+                const float z4 =
+                    fmaf(150.0625f, a0, fmaf(39.0625f, a1, fmaf(5.0625f, a2, 0.0625f * a3)));
+                // H about the middle: hA z^2 + h1 z + h0
+                const float hm = fmaf(f.hA, t, hB);
+                const float h1 = fmaf(f.hA, t, hm), h0 = fmaf(hm, t, hC);
+                const float q0 = fmaf(f.hA, z2, fmaf(h1, z1, h0 * z0));
+                const float q1 = fmaf(f.hA, z3, fmaf(h1, z2, h0 * z1));
+                const float q2 = fmaf(f.hA, z4, fmaf(h1, z3, h0 * z2));
+                s0 = z0;
+                st = fmaf(t, z0, z1);
+                su = fmaf(d, z0, z1);
+                suu = fmaf(d, z1 + su, z2);
+                p0 = q0;
+                pt = fmaf(t, q0, q1);
+                pu = fmaf(d, q0, q1);
+                puu = fmaf(d, q1 + pu, q2);
+            } else {
+                v2 S0, S1, S2, S3, S4;
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const v2 T1 = mul2(W[j], T[j]), T2 = mul2(T1, T[j]), T3 = mul2(T2, T[j]);
+                    S0 = j ? add2(S0, W[j]) : W[j];
+                    S1 = j ? add2(S1, T1) : T1;
+                    S2 = j ? add2(S2, T2) : T2;
+                    S3 = j ? add2(S3, T3) : T3;
+                    S4 = j ? fma2(T3, T[j], S4) : mul2(T3, T[j]);
+                }
+                s0 = lanesum(S0);
+                st = lanesum(S1);
+                const float s2 = lanesum(S2), s3 = lanesum(S3), s4 = lanesum(S4);
+                p0 = fmaf(f.hA, s2, fmaf(hB, st, hC * s0));
+                pt = fmaf(f.hA, s3, fmaf(hB, s2, hC * st));
+                const float p2 = fmaf(f.hA, s4, fmaf(hB, s3, hC * s2));
+                const float x = d - t;  // du = t + x
+                su = fmaf(x, s0, st);
+                suu = fmaf(x, st + su, s2);
+                pu = fmaf(x, p0, pt);
+                puu = fmaf(x, pt + pu, p2);
+            }
+            c.h0 += p0;
+            c.hu += pt;
+            c.hv = fmaf(dv, p0, c.hv);
+            c.huu += puu;
+            c.huv = fmaf(dv, pu, c.huv);
+            c.hvv = fmaf(dv2, p0, c.hvv);
+            c.w0 += s0;
+            c.wu += st;
+            c.wv = fmaf(dv, s0, c.wv);
+            c.wuu += suu;
+            c.wuv = fmaf(dv, su, c.wuv);
+            c.wvv = fmaf(dv2, s0, c.wvv);
         }
+        m.add(c);
     }
-    if (CENTRED) m.add_shifted(c, (u0 + f.nu) + 3.5f);
 }
-// The same over the pixels [p0, p1) of a tile whose runs share nothing;
+// The same over the pixels [p0, p1) of a tile whose runs share nothing (u is x);
 // `x` and `y` are the coordinates of the tile's first staged pixel.
-__device__ __forceinline__ void pixel_moments(const PixelStage &px, const float *x,
-                                              const float *y, int p0, int p1,
-                                              const LaneForm &f, Moments &m) {
+__device__ __forceinline__ void pixel_sums(const PixelStage &px, const float *x, const float *y,
+                                           int p0, int p1, const LaneForm &f, float fuv,
+                                           float fvv, GradSums<double> &m) {
 #pragma unroll 1
-    for (int p = p0; p < p1; ++p) {
-        const float du = x[p] + f.nu, dv = y[p] + f.nv;
-        const float dv2 = dv * dv;
-        const float e = fmaf(fmaf(f.e20, du, f.e11 * dv), du, f.e02 * dv2);
-        const float w = px.r2[run_slot(p)] * (e < E_CUT ? 0.0f : ex2f(e));
-        const float w1 = w * du, w2 = w1 * du, w3 = w2 * du;
-        m.add(dv, dv2, w, w1, w2, w3, w3 * du);
+    for (int p = p0; p < p1;) {
+        const int end = min(p1, (p | 15) + 1);
+        GradSums<float> c;
+#pragma unroll 1
+        for (; p < end; ++p) {
+            const float r2 = px.r2[run_slot(p)];
+            if (r2 == 0.0f) continue;  // (the same in every lane)
+            const float du = x[p] + f.nu, dv = y[p] + f.nv;
+            const float vu = fmaf(fuv, dv, f.fuu * du), vv = fmaf(fuv, du, fvv * dv);
+            const float q = fmaf(dv, vv, du * vu);
+            const float w = r2 * (q > FPHO_MAX_EXP_ARG ? 0.0f : ex2f(q * KEXP));
+            const float h = w * fmaf(fmaf(vv, vv, vu * vu), 1.0f / 24.0f, f.c0);
+            const float duu = du * du, duv = du * dv, dvv = dv * dv;
+            c.h0 += h;
+            c.hu = fmaf(h, vu, c.hu);
+            c.hv = fmaf(h, vv, c.hv);
+            c.huu = fmaf(h, duu, c.huu);
+            c.huv = fmaf(h, duv, c.huv);
+            c.hvv = fmaf(h, dvv, c.hvv);
+            c.w0 += w;
+            c.wu = fmaf(w, vu, c.wu);
+            c.wv = fmaf(w, vv, c.wv);
+            c.wuu = fmaf(w, duu, c.wuu);
+            c.wuv = fmaf(w, duv, c.wuv);
+            c.wvv = fmaf(w, dvv, c.wvv);
+        }
+        m.add(c);
     }
 }
 
 // The gradient pass over `n_px` staged pixels, the first at index `pix` of the
 // patch's arrays: every kept Gaussian of the tile in a lane of its own.
 //
-// A lane forms the moments of its Gaussian's weight W = r2 G about the
-// Gaussian's centre; H = 1 + (|v|^2 - fxx - fyy)/24 is a quadratic in the
-// offsets, so every sum the derivatives need (sum W H, sum W H d, sum W H d
-// d^T, sum W, sum W d, sum W d d^T) is a combination of them, taken once per
-// Gaussian; then its Jacobian, and a sum over the lanes of each source.
+// A lane forms the twelve sums of GradSums; every derivative is a combination of
+// them, taken once per Gaussian; then its Jacobian, and a sum over the lanes of
+// each source.
 //
 // Against pixels in the lanes and Gaussians in the loop (each thread forming
 // the sums of its own 8 pixels), the per-Gaussian work is done once for a
@@ -628,59 +680,46 @@ __device__ __forceinline__ void gradient_lanes(const TileArgs &A, const int *kep
         const bool alive = g * 32 + lane < n_live;
         const int k = kept[min(g * 32 + lane, n_live - 1)] >> 1;
         const float4 *r4 = reinterpret_cast<const float4 *>(A.gtab + (size_t)(g0 + k) * GREC);
-        const float4 ra = r4[0], rb = r4[1];
-        const float fyy = reinterpret_cast<const float *>(r4)[R_FYY];
-        const float fxx = rb.x, fxy = rb.z;
-        Moments m;
-        const LaneForm f = {shared_x ? ra.z : ra.x, shared_x ? ra.x : ra.z,
-                            (shared_x ? fyy : fxx) * KEXP, 2.0f * KEXP * fxy,
-                            (shared_x ? fxx : fyy) * KEXP};
-        if (shared_x || !(misfit & MISFIT_Y)) {
-            if (__any_sync(0xffffffffu, !((shared_x ? fyy : fxx) <= NARROW)))
-                run_moments<false>(px, UNIT / 8 * q, UNIT / 8 * (q + nm), f, m);
-            else
-                run_moments<true>(px, UNIT / 8 * q, UNIT / 8 * (q + nm), f, m);
-        } else {
-            pixel_moments(px, A.pv.xpix + pix, A.pv.ypix + pix, UNIT * q,
-                          min(UNIT * (q + nm), n_px), f, m);
-        }
-        // sums over W H and over W, in (x, y)
-        const float c0 = reinterpret_cast<const float *>(r4)[R_C0];
-        const float fuu = shared_x ? fyy : fxx, fvv = shared_x ? fxx : fyy;
-        const float h20 = (fuu * fuu + fxy * fxy) * (1.0f / 24.0f);
-        const float h11 = 2.0f * fxy * (fuu + fvv) * (1.0f / 24.0f);
-        const float h02 = (fvv * fvv + fxy * fxy) * (1.0f / 24.0f);
-        const float gA = c0 * m.m00 + h20 * m.m20 + h11 * m.m11 + h02 * m.m02;
-        const float hu = c0 * m.m10 + h20 * m.m30 + h11 * m.m21 + h02 * m.m12;
-        const float hv = c0 * m.m01 + h20 * m.m21 + h11 * m.m12 + h02 * m.m03;
-        const float huu = c0 * m.m20 + h20 * m.m40 + h11 * m.m31 + h02 * m.m22;
-        const float hxy = c0 * m.m11 + h20 * m.m31 + h11 * m.m22 + h02 * m.m13;
-        const float hvv = c0 * m.m02 + h20 * m.m22 + h11 * m.m13 + h02 * m.m04;
-        const float hx = shared_x ? hv : hu, hy = shared_x ? hu : hv;
-        const float hxx = shared_x ? hvv : huu, hyy = shared_x ? huu : hvv;
-        const float wx = shared_x ? m.m01 : m.m10, wy = shared_x ? m.m10 : m.m01;
-        const float wxx = shared_x ? m.m02 : m.m20, wyy = shared_x ? m.m20 : m.m02;
-        const float wxy = m.m11, w0 = m.m00;
-        // derivatives w.r.t. (A, x, y, fxx, fyy, fxy): v = F d
-        const float sVx = fxx * wx + fxy * wy, sVy = fxy * wx + fyy * wy;
-        const float gx = fxx * hx + fxy * hy - (fxx * sVx + fxy * sVy) * (1.0f / 12.0f);
-        const float gy = fxy * hx + fyy * hy - (fxy * sVx + fyy * sVy) * (1.0f / 12.0f);
-        const float t1 = fxx * wxx + fxy * wxy;   // sum W dx vx
-        const float t2 = fyy * wyy + fxy * wxy;   // sum W dy vy
-        const float t3 = fxy * (wxx + wyy) + (fxx + fyy) * wxy;
-        const float gfxx = t1 * (1.0f / 12.0f) - 0.5f * hxx - w0 * (1.0f / 24.0f);
-        const float gfyy = t2 * (1.0f / 12.0f) - 0.5f * hyy - w0 * (1.0f / 24.0f);
-        const float gfxy = t3 * (1.0f / 12.0f) - hxy;
-        // the Jacobian (amp factors are folded into its rows)
+        const bool in_runs = shared_x || !(misfit & MISFIT_Y);
+        GradSums<double> m;
+        const float4 ra = r4[0];
+        float fxx = r4[1].x, fxy = r4[1].z, fyy = r4[2].x;
+        const LaneForm f(shared_x ? ra.z : ra.x, shared_x ? ra.x : ra.z, shared_x ? fyy : fxx, fxy,
+                         shared_x ? fxx : fyy, r4[3].z);
+        if (!in_runs)
+            pixel_sums(px, A.pv.xpix + pix, A.pv.ypix + pix, UNIT * q, min(UNIT * (q + nm), n_px),
+                       f, fxy, fyy, m);
+        else if (__any_sync(0xffffffffu, !(f.fuu <= NARROW)))
+            run_sums<false>(px, UNIT / 8 * q, UNIT / 8 * (q + nm), f, m);
+        else
+            run_sums<true>(px, UNIT / 8 * q, UNIT / 8 * (q + nm), f, m);
+        // the record is read again here: kept through the loops, it would take
+        // the registers of the fifth CTA on an SM
+        asm volatile("" : "+l"(r4));
+        fxx = r4[1].x, fxy = r4[1].z, fyy = r4[2].x;
+        if (in_runs) f.finish(m, fxy, shared_x ? fxx : fyy);
+        // derivatives w.r.t. (A, x, y, fxx, fyy, fxy) and, through the Jacobian
+        // (amp factors are folded into its rows), the parameters; in double
+        // until they are summed over a Gaussian's derivatives, which cancel
+        const double hx = shared_x ? m.hv : m.hu, hy = shared_x ? m.hu : m.hv;
+        const double wx = shared_x ? m.wv : m.wu, wy = shared_x ? m.wu : m.wv;
+        const double hxx = shared_x ? m.hvv : m.huu, hyy = shared_x ? m.huu : m.hvv;
+        const double wxx = shared_x ? m.wvv : m.wuu, wyy = shared_x ? m.wuu : m.wvv;
+        const double fx = fxx, fz = fxy, fy = fyy, gA = m.h0;
+        const double gx = hx - (fx * wx + fz * wy) * (1.0 / 12.0);
+        const double gy = hy - (fz * wx + fy * wy) * (1.0 / 12.0);
+        const double gfxx = (fx * wxx + fz * m.wuv) * (1.0 / 12.0) - 0.5 * hxx - m.w0 * (1.0 / 24.0);
+        const double gfyy = (fy * wyy + fz * m.wuv) * (1.0 / 12.0) - 0.5 * hyy - m.w0 * (1.0 / 24.0);
+        const double gfxy = (fz * (wxx + wyy) + (fx + fy) * m.wuv) * (1.0 / 12.0) - m.huv;
         const float4 j0 = r4[4], j1 = r4[5], j2 = r4[6], j3 = r4[7];
         float P[7];
-        P[0] = j0.x * gA;
-        P[1] = fmaf(j1.z, gy, j1.y * gx);
-        P[2] = fmaf(j2.x, gy, j1.w * gx);
-        P[3] = fmaf(j2.w, gfyy, fmaf(j2.z, gfxy, fmaf(j2.y, gfxx, j0.y * gA)));
-        P[4] = fmaf(j3.z, gfyy, fmaf(j3.y, gfxy, fmaf(j3.x, gfxx, j0.z * gA)));
-        P[5] = j0.w * gA;
-        P[6] = j1.x * gA;
+        P[0] = (float)(j0.x * gA);
+        P[1] = (float)(j1.y * gx + j1.z * gy);
+        P[2] = (float)(j1.w * gx + j2.x * gy);
+        P[3] = (float)(j0.y * gA + j2.y * gfxx + j2.z * gfxy + j2.w * gfyy);
+        P[4] = (float)(j0.z * gA + j3.x * gfxx + j3.y * gfxy + j3.z * gfyy);
+        P[5] = (float)(j0.w * gA);
+        P[6] = (float)(j1.x * gA);
         // per-source sums: sources are contiguous in the kept list, so each
         // source's first lane collects the lanes after it
         const int src = alive ? (int)min((unsigned)__float_as_int(j3.w),
