@@ -554,7 +554,10 @@ int upload_meta(fpho_patch *p, const fpho_patch_struct *h, cudaStream_t s,
     // rows first, straight from the caller's array, then everything else in
     // one transfer.  (A block of its own for each of 15 arrays, freed, allocated
     // and copied one by one, with a device synchronisation each, took 0.45 ms
-    // of a flux solve.)
+    // of a flux solve.)  The caller's arrays may be read now, pinned ones that
+    // earlier work in `s` fills too: when a patch is created, the transfers of its
+    // index arrays, which are pageable, have waited for that work, and when
+    // metadata are replaced, the synchronisation above has.
     const size_t es = (size_t)ne * nsrc;
     std::vector<unsigned char> rest;
     const size_t psf_bytes = ((size_t)nrows * sizeof(fpho_psfgauss) + 255) / 256 * 256;

@@ -182,6 +182,9 @@ FPHO_API int fpho_patch_free(fpho_patch *p);
  *             dchi2_stride >= 7*n_sources (210 gives the reference's
  *             fpho_response layout; entries past 7*n_sources are zeroed).
  *   flags     FPHO_IO_HOST, FPHO_WANT_RESIDUAL
+ * With FPHO_IO_HOST a proposal in pinned or managed memory may still be filled
+ * by earlier work in `stream`; what work in another stream fills must be
+ * complete (the legacy default stream's implicit order does not cover it).
  * n_sources must equal the patch's n_sources. */
 FPHO_API int fpho_evaluate_proposal(fpho_patch *p, const fpho_source *proposal, int n_sources,
                            double *chi2, float *dchi2, int dchi2_stride,

@@ -49,6 +49,42 @@ def test_proposal_memory(ns):
     P.free()
 
 
+@pytest.mark.parametrize("name", ["rad2", "D", "crpix", "crval", "CW", "G"])
+def test_pinned_metadata_in_stream_order(name):
+    """Metadata in pinned memory that earlier work in the (non-blocking) stream
+    still has to fill, when a patch is created and when its metadata are replaced."""
+    import torch
+    from forcepho_b200 import _lib
+    from forcepho_b200.patches.device_patch import DevicePatch
+    P, prop = case(3)
+    raw = np.frombuffer(prop.tobytes(), dtype=np.uint8).copy()
+    want = evaluate(P, raw.ctypes.data, _lib.FPHO_IO_HOST)
+    good = getattr(P, name)
+    dev = torch.from_numpy(good.copy()).cuda()
+    pinned = torch.from_numpy(good * 1.5).pin_memory()
+    setattr(P, name, pinned.numpy())
+    s = torch.cuda.Stream()
+    a = torch.rand(4096, 4096, device="cuda")
+    torch.cuda.synchronize()
+    for replace in (False, True):
+        pinned.mul_(1.5)
+        with torch.cuda.stream(s):
+            for _ in range(8):              # some milliseconds ahead of the copy
+                a = a @ a * 1e-4
+            pinned.copy_(dev, non_blocking=True)
+            if replace:
+                st = P.host_struct()
+                _lib.call("fpho_patch_replace_meta", P.device_patch.handle, st.ctypes.data,
+                          s.cuda_stream)
+            else:
+                P.device_patch.free()
+                P.device_patch = DevicePatch(P, True, stream=s.cuda_stream)
+            got = evaluate(P, raw.ctypes.data, _lib.FPHO_IO_HOST)
+        for g, w in zip(got, want):
+            np.testing.assert_array_equal(g, w)
+    P.free()
+
+
 def test_retrieve_memory():
     import torch
     from forcepho_b200 import _lib
