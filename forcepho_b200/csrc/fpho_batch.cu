@@ -88,9 +88,9 @@ __global__ void __launch_bounds__(NT, MINB) batch_tiles(const TileArgs *args, co
         if (it >= n_work) break;
         const int2 w = work[it];
         if constexpr (SPLIT > 0)
-            tile_body_split<SPLIT, K>(args[w.x], w.y, 0, smem, &mbar, phase);
+            tile_body_split<SPLIT, K, true, 1, false>(args[w.x], w.y, 0, smem, &mbar, phase);
         else
-            tile_body<NT, K>(args[w.x], w.y, smem, &mbar, phase);
+            tile_body<NT, K, true, false, false>(args[w.x], w.y, smem, &mbar, phase);
         __syncthreads();  // shared memory of this tile fully consumed
     }
 }

@@ -107,7 +107,7 @@ __global__ void __launch_bounds__(NT) tile_kernel_dyn(TileArgs A, const int *ord
         __syncthreads();
         const int item = s_item;
         if (item >= n_tiles) break;
-        tile_body<NT, K, GRAD, EXACT>(A, order[item], smem, &mbar, phase);
+        tile_body<NT, K, GRAD, EXACT, false>(A, order[item], smem, &mbar, phase);
         __syncthreads();
     }
 }
@@ -164,7 +164,7 @@ __global__ void __launch_bounds__(32 * NW, MINB) split_kernel_dyn(TileArgs A, co
         __syncthreads();
         const int item = s_item;
         if (item >= n_tiles) break;
-        tile_body_split<NW, K, GRAD>(A, order[item], 0, smem, &mbar, phase);
+        tile_body_split<NW, K, GRAD, 1, false>(A, order[item], 0, smem, &mbar, phase);
         __syncthreads();
     }
 }

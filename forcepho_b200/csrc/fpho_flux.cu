@@ -111,6 +111,7 @@ __global__ void __launch_bounds__(NT) normal_tiles(TileArgs A, double *pnorm, in
     const int g1 = A.pv.gauss_start[td.exposure + 1];
     const int npsf = A.pv.exp_npsf[td.exposure];
     for (int j = tid; j < ns * (TP + 1); j += NT) rows[j] = 0.0f;
+    wait_for_earlier_kernel();  // before the pixel arrays, which a kernel may have filled
     for (int li = tid; li < TP; li += NT) {
         const bool ok = li < td.count;
         ws[li] = ok ? A.pv.ierr[td.pix_begin + li] : 0.0f;
@@ -135,7 +136,6 @@ __global__ void __launch_bounds__(NT) normal_tiles(TileArgs A, double *pnorm, in
         Yp[j] = pk(yv[0], yv[1]);
         M[j] = 0ull;
     }
-    wait_for_earlier_kernel();
     const int n_live = scan_tile<NT, true>(A, bb, g0, g1, npsf, kept,
                                             reinterpret_cast<unsigned *>(recs), cap * GSTAGE);
     const v2 KEXP2 = pk1(KEXP), KEXPLO2 = pk1(KEXP_LO), CM24 = pk1(-1.0f / 24.0f);
@@ -238,6 +238,7 @@ __global__ void __launch_bounds__(32 * MMA_WARPS) normal_tiles_mma(TileArgs A, d
     const int g1 = A.pv.gauss_start[td.exposure + 1];
     const int npsf = A.pv.exp_npsf[td.exposure];
     for (int j = tid; j < nr * MMA_ROW; j += NT) rows[j] = 0.0f;
+    wait_for_earlier_kernel();  // before the pixel arrays, which a kernel may have filled
     const float xmid = 0.5f * (bb.x + bb.y), ymid = 0.5f * (bb.z + bb.w);
     constexpr int KP = MMA_K / 2;
     float w[MMA_K], y[MMA_K];
@@ -262,7 +263,6 @@ __global__ void __launch_bounds__(32 * MMA_WARPS) normal_tiles_mma(TileArgs A, d
         M[j] = X[j] = 0ull;
     }
     const int share = share_of<8>(A.tile_misfit[tile], false);
-    wait_for_earlier_kernel();
     const int n_live = scan_tile<NT, true>(A, bb, g0, g1, npsf, kept,
                                            reinterpret_cast<unsigned *>(recs),
                                            MMA_STAGE * GSTAGE);

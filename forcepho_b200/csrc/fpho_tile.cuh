@@ -852,7 +852,8 @@ __device__ __forceinline__ int scan_tile(const TileArgs &A, float4 bb, int g0, i
 // GRAD = false runs the residual pass and chi2 only (no gradient pass, no
 // gradient partials written).  EXACT = true runs the residual pass in the
 // reference's float arithmetic (residual_exact) instead of the packed pass.
-template <int NT, int K, bool GRAD = true, bool EXACT = false>
+// WAIT = false: the caller has waited for the kernels before.
+template <int NT, int K, bool GRAD = true, bool EXACT = false, bool WAIT = true>
 __device__ __forceinline__ void tile_body(const TileArgs &A, int tile, unsigned char *smem,
                                           uint64_t *mbar, uint32_t &phase) {
     static_assert(K % 2 == 0, "pixels per thread must be even (packed pairs)");
@@ -882,6 +883,9 @@ __device__ __forceinline__ void tile_body(const TileArgs &A, int tile, unsigned 
     for (int j = tid; j < NW * stride; j += NT) wacc[j] = 0.0f;
 
     // ---- this thread's pixels: K consecutive ones, pair j holds pixels 2j and 2j + 1
+    // (the caller may reach the pixel arrays through the device struct, and fill
+    // them in a kernel before this one)
+    if (WAIT) wait_for_earlier_kernel();
     const float xmid = 0.5f * (bb.x + bb.y), ymid = 0.5f * (bb.z + bb.w);
     v2 X[KP], Y[KP], R[KP], R2[KP];
     float D[K], IE[K];
@@ -910,7 +914,6 @@ __device__ __forceinline__ void tile_body(const TileArgs &A, int tile, unsigned 
     if (tid == 0) s_any_weight = s_misfit = 0;
 
     // ---- the ordered list of kept image Gaussians
-    wait_for_earlier_kernel();
     const int n_live = scan_tile<NT>(A, bb, g0, g1, npsf, kept,
                                       reinterpret_cast<unsigned *>(recs),
                                       (int)(stage_bytes(TP, cap) / 4));
@@ -1046,7 +1049,7 @@ __host__ __device__ inline size_t split_smem_layout_bytes(int nw, int k, int liv
     return tile_smem_layout_bytes(nw, 32 * k, live_cap, idx_cap, stride) + (size_t)nw * 32 * k * 4;
 }
 
-template <int NW, int K, bool GRAD = true, int PS = 1>
+template <int NW, int K, bool GRAD = true, int PS = 1, bool WAIT = true>
 __device__ __forceinline__ void tile_body_split(const TileArgs &A, int tile, int part,
                                                 unsigned char *smem, uint64_t *mbar,
                                                 uint32_t &phase) {
@@ -1082,7 +1085,9 @@ __device__ __forceinline__ void tile_body_split(const TileArgs &A, int tile, int
 
     for (int j = tid; j < NW * stride; j += NT) wacc[j] = 0.0f;
 
-    // ---- the pixels, in every warp: KL consecutive ones per lane
+    // ---- the pixels, in every warp: KL consecutive ones per lane (after the
+    // wait, as in tile_body)
+    if (WAIT) wait_for_earlier_kernel();
     const float xmid = 0.5f * (bb.x + bb.y), ymid = 0.5f * (bb.z + bb.w);
     v2 X[KP], Y[KP], R[KP];
     bool counts[KL];
@@ -1106,7 +1111,6 @@ __device__ __forceinline__ void tile_body_split(const TileArgs &A, int tile, int
     const bool tile_has_weight = wbox.x <= wbox.y;  // the box of no pixels is empty
     const int misfit = tile_misfit<KL>(A, td, tile, 0);
 
-    wait_for_earlier_kernel();
     const int n_live = scan_tile<NT>(A, bb, g0, g1, npsf, kept,
                                       reinterpret_cast<unsigned *>(recs),
                                       (int)(stage_bytes(TP, cap) / 4));
