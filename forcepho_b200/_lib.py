@@ -51,6 +51,7 @@ _SIGS = {
     "fpho_abi_version": (c_int, []),
     "fpho_sizeof": (c_int, [c_int]),
     "fpho_patch_create": (c_int, [c_void_p, c_int, c_int, c_void_p, ctypes.POINTER(c_void_p)]),
+    "fpho_test_fail_alloc": (c_int, [c_int]),
     "fpho_patch_replace_meta": (c_int, [c_void_p, c_void_p, c_void_p]),
     "fpho_patch_swap_data_residual": (c_int, [c_void_p, c_void_p]),
     "fpho_patch_retrieve": (c_int, [c_void_p, c_int, c_void_p, c_void_p]),

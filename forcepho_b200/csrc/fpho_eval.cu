@@ -440,6 +440,7 @@ void free_plan(fpho_patch *p) {
     dfree(p->d_tiles); dfree(p->d_tbox_all); dfree(p->d_tbox_w); dfree(p->d_tile_band_start);
     dfree(p->d_tile_misfit); dfree(p->d_runs);
     dfree(p->d_pchi2); dfree(p->d_pgrad);
+    p->pgrad_cap = 0;
     dfree(p->d_tile_cost); dfree(p->d_tile_order); dfree(p->d_tile_counter);
 }
 
@@ -485,7 +486,14 @@ int read_pixel_index(fpho_patch *p, const fpho_patch_struct *h, int n_bands) {
     return FPHO_OK;
 }
 
+// Floats of the gradient partials of `tiles` tiles.
+size_t pgrad_floats(const fpho_patch *p, size_t tiles, int n_sources) {
+    return tiles * p->max_parts * 7 * n_sources;
+}
+
 // Validate and upload the per-scene metadata; derive the image-Gaussian index.
+// A failure before the first transfer leaves the patch as it was: its sizes and
+// pointers change once every block that the new scene needs is there.
 int upload_meta(fpho_patch *p, const fpho_patch_struct *h, cudaStream_t s,
                 bool validate_only = false) {
     if (!h->rad2 || !h->D || !h->crpix || !h->crval || !h->CW || !h->G || !h->n_psf_per_source ||
@@ -540,16 +548,6 @@ int upload_meta(fpho_patch *p, const fpho_patch_struct *h, cudaStream_t s,
     // kernels on any stream may still read the metadata and the workspace that
     // are replaced here
     if (p->d_meta) CUDA_TRY(cudaDeviceSynchronize());
-    p->n_sources = nsrc;
-    p->n_radii = nrad;
-    p->n_psf_per_source = npsf;
-    p->psfgauss_start = pstart;
-    p->exp_npsf = exp_npsf;
-    p->gauss_start = gstart;
-    p->n_gauss = (int)ng;
-    p->max_g = 0;
-    for (int e = 0; e < ne; ++e) p->max_g = std::max(p->max_g, gstart[e + 1] - gstart[e]);
-    p->n_psfrows = nrows;
     // One device block for all metadata, kept while it is large enough: the PSF
     // rows first, straight from the caller's array, then everything else in
     // one transfer.  (A block of its own for each of 15 arrays, freed, allocated
@@ -567,7 +565,11 @@ int upload_meta(fpho_patch *p, const fpho_patch_struct *h, cudaStream_t s,
         if (bytes) std::memcpy(rest.data() + at, src, bytes);
         return psf_bytes + at;
     };
-    rest.reserve(es * 48 + 64 * (size_t)ne + 8192);
+    try {
+        rest.reserve(es * 48 + 64 * (size_t)ne + 8192);  // all that is put
+    } catch (const std::bad_alloc &) {
+        return set_error(FPHO_ERR_NOMEM, "host allocation failed");
+    }
     const size_t o_rad2 = put(h->rad2, sizeof(float) * nrad);
     const size_t o_D = put(h->D, sizeof(float) * es * 4);
     const size_t o_CW = put(h->CW, sizeof(float) * es * 4);
@@ -580,27 +582,43 @@ int upload_meta(fpho_patch *p, const fpho_patch_struct *h, cudaStream_t s,
     const size_t o_enpsf = put(exp_npsf.data(), sizeof(int) * ne);
     const size_t o_gstart = put(gstart.data(), sizeof(int) * (ne + 1));
     const size_t bytes = psf_bytes + rest.size();
-    int rc;
-    if (p->d_meta_cap < bytes) {
-        dfree(p->d_meta);
-        p->d_meta_cap = 0;
-        if ((rc = dalloc(&p->d_meta, bytes))) return rc;
-        p->d_meta_cap = bytes;
+    const size_t pgrad = pgrad_floats(p, (size_t)p->n_tiles, nsrc);
+    unsigned char *new_meta = nullptr;
+    float *new_gtab = nullptr, *new_pgrad = nullptr;
+    float4 *new_gbox = nullptr;
+    fpho_source *new_prop = nullptr;
+    int rc = FPHO_OK;
+    if (p->d_meta_cap < bytes) rc = dalloc(&new_meta, bytes);
+    const bool grow = (size_t)ng > p->gauss_cap || !p->d_gtab;
+    if (!rc && grow) rc = dalloc(&new_gtab, (size_t)ng * GREC);
+    if (!rc && grow) rc = dalloc(&new_gbox, (size_t)ng);
+    if (!rc && (size_t)nsrc > p->prop_cap) rc = dalloc(&new_prop, (size_t)nsrc);
+    if (!rc && pgrad > p->pgrad_cap) rc = dalloc(&new_pgrad, pgrad);
+    if (rc) {
+        dfree(new_meta); dfree(new_gtab); dfree(new_gbox); dfree(new_prop); dfree(new_pgrad);
+        return rc;
     }
-    if ((size_t)ng > p->gauss_cap || !p->d_gtab) {
-        dfree(p->d_gtab);
-        dfree(p->d_gbox);
-        p->gauss_cap = 0;
-        if ((rc = dalloc(&p->d_gtab, (size_t)ng * GREC))) return rc;
-        if ((rc = dalloc(&p->d_gbox, (size_t)ng))) return rc;
-        p->gauss_cap = (size_t)ng;
-    }
-    if ((size_t)nsrc > p->prop_cap) {
-        dfree(p->d_prop);
-        p->prop_cap = 0;
-        if ((rc = dalloc(&p->d_prop, (size_t)nsrc))) return rc;
-        p->prop_cap = (size_t)nsrc;
-    }
+    auto install = [](auto *&old, auto *fresh, size_t &cap, size_t n) {
+        if (!fresh) return;
+        dfree(old);
+        old = fresh;
+        cap = n;
+    };
+    install(p->d_meta, new_meta, p->d_meta_cap, bytes);
+    install(p->d_gtab, new_gtab, p->gauss_cap, (size_t)ng);
+    install(p->d_gbox, new_gbox, p->gauss_cap, (size_t)ng);
+    install(p->d_prop, new_prop, p->prop_cap, (size_t)nsrc);
+    install(p->d_pgrad, new_pgrad, p->pgrad_cap, pgrad);
+    p->n_sources = nsrc;
+    p->n_radii = nrad;
+    p->n_psf_per_source = npsf;
+    p->psfgauss_start = pstart;
+    p->exp_npsf = exp_npsf;
+    p->gauss_start = gstart;
+    p->n_gauss = (int)ng;
+    p->max_g = 0;
+    for (int e = 0; e < ne; ++e) p->max_g = std::max(p->max_g, gstart[e + 1] - gstart[e]);
+    p->n_psfrows = nrows;
     unsigned char *m = p->d_meta;
     p->d_psfgauss = reinterpret_cast<fpho_psfgauss *>(m);
     p->d_rad2 = reinterpret_cast<float *>(m + o_rad2);
@@ -664,7 +682,13 @@ cudaError_t launch_dependent(const void *fn, dim3 grid, dim3 block, void **args,
     return cudaLaunchKernelExC(&cfg, fn, args);
 }
 
+static thread_local int t_fail_alloc = 0;  // see fpho_test_fail_alloc
+
 cudaError_t pool_malloc(void **p, size_t bytes) {
+    if (t_fail_alloc > 0 && --t_fail_alloc == 0) {
+        *p = nullptr;
+        return cudaErrorMemoryAllocation;
+    }
     static std::once_flag once[64];
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
@@ -789,7 +813,9 @@ int build_plan(fpho_patch *p, cudaStream_t s) {
     p->max_parts = p->n_tiles > 4 * device_sms() ? 1 : MAX_TILE_PARTS;
     const size_t partials = tiles.size() * p->max_parts;
     if ((rc = dalloc(&p->d_pchi2, partials))) return rc;
-    if ((rc = dalloc(&p->d_pgrad, partials * 7 * p->n_sources))) return rc;
+    const size_t pgrad = pgrad_floats(p, tiles.size(), p->n_sources);
+    if ((rc = dalloc(&p->d_pgrad, pgrad))) return rc;
+    p->pgrad_cap = pgrad;
     if ((rc = dalloc(&p->d_tile_cost, tiles.size()))) return rc;
     if ((rc = dalloc(&p->d_tile_order, tiles.size()))) return rc;
     if ((rc = dalloc(&p->d_tile_counter, 1))) return rc;
@@ -866,15 +892,8 @@ extern "C" int fpho_patch_replace_meta(fpho_patch *p, const fpho_patch_struct *h
     clear_error();
     if (!p || !host) return set_error(FPHO_ERR_INVALID, "NULL argument");
     cudaStream_t s = (cudaStream_t)stream;
-    const int old_nsrc = p->n_sources;
     int rc = upload_meta(p, host, s);
-    if (rc) return rc;
-    if (p->n_sources != old_nsrc) {
-        dfree(p->d_pgrad);
-        if ((rc = dalloc(&p->d_pgrad, (size_t)p->n_tiles * p->max_parts * 7 * p->n_sources)))
-            return rc;
-    }
-    return refresh_struct(p, s);
+    return rc ? rc : refresh_struct(p, s);
 }
 
 extern "C" int fpho_patch_swap_data_residual(fpho_patch *p, void *stream) {
@@ -987,6 +1006,13 @@ extern "C" int fpho_patch_set_test_stall(fpho_patch *p, int on) {
     if (on && p->schedule == 1 && p->n_tiles > 4 * device_sms())
         return set_error(FPHO_ERR_STATE, "the test stall needs one CTA per tile (schedule 0)");
     p->test_extra_tx = on ? 16 : 0;
+    return FPHO_OK;
+}
+
+extern "C" int fpho_test_fail_alloc(int n) {
+    clear_error();
+    if (n < 0) return set_error(FPHO_ERR_INVALID, "n=%d < 0", n);
+    fpho::t_fail_alloc = n;
     return FPHO_OK;
 }
 

@@ -62,7 +62,8 @@ struct fpho_patch {
     double *d_pchi2 = nullptr;
     float *d_pgrad = nullptr;
     fpho_source *d_prop = nullptr;
-    size_t gauss_cap = 0, prop_cap = 0;  // records of d_gtab / d_gbox, sources of d_prop
+    // records of d_gtab / d_gbox, sources of d_prop, floats of d_pgrad
+    size_t gauss_cap = 0, prop_cap = 0, pgrad_cap = 0;
     // host-I/O evaluations: pinned memory the reduction writes the results to,
     // [chi2 (n_bands doubles)][error word, 8 bytes][dchi2]
     unsigned char *h_io = nullptr;
