@@ -561,10 +561,12 @@ static int enqueue_normal(fpho_patch *p, const fpho_source *d_prop, double *d_at
     const NormalShape &S = kNormalShapes[shape];
     const int idx_cap = std::max(p->max_g, 1);
     const int live_cap = std::min(p->live_cap, DESIGN_LIVE_CAP);
-    // on the tensor cores where the rows fit in shared memory as doubles
+    // on the tensor cores where the rows fit in shared memory (with what that
+    // kernel has there statically)
+    constexpr size_t MMA_STATIC = 256;
     const size_t mma_smem = mma_smem_bytes(idx_cap, ns);
     const bool mma = tile == MMA_TILE && live_cap == DESIGN_LIVE_CAP &&
-                     ns <= NORMAL_MMA_SOURCES && mma_smem <= 227 * 1024;
+                     ns <= NORMAL_MMA_SOURCES && mma_smem + MMA_STATIC <= 227 * 1024;
     const void *fn = mma ? (const void *)normal_tiles_mma : S.fn;
     const size_t smem = mma ? mma_smem : normal_smem_bytes(tile, live_cap, idx_cap, ns);
     if (smem > 227 * 1024)

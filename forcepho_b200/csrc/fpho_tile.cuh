@@ -102,9 +102,9 @@ __device__ __forceinline__ double warp_sum_d(double v) {
 
 // ------------------------------------------------------------ shared layout
 // Dynamic shared memory of a tile CTA, in order:
-//   stage   first the masks of the scan; then `live_cap` staged records of the
-//           residual pass (the
-//           first MODEL_STAGE floats of each: all it reads); then the pixels of the gradient pass, PX_BYTES each
+//   stage   first the masks and queues of the scan; then `live_cap` staged records
+//           of the residual pass (the first MODEL_STAGE floats of each: all it
+//           reads); then the pixels of the gradient pass, PX_BYTES each
 //           (px_block pixels at a time);
 //   kept    the kept list, one int per Gaussian of the exposure (local index
 //           << 1 | flags);
@@ -124,10 +124,16 @@ __host__ __device__ inline int px_block(int tile_pixels, int live_cap) {
     while (n * PX_BYTES > live_cap * 128) n >>= 1;
     return n;
 }
+// The scan's queues (scan_tile), and the least it has with its masks.  128 bytes
+// per record, less the 128 of static shared memory that a tile kernel has had
+// since, is what a patch's limits are counted with; no stage takes more.
+constexpr int QUEUE = 64;  // Gaussians a warp queues
+constexpr size_t MIN_STAGE = 32 * 128 - 128;
 __host__ __device__ inline size_t stage_bytes(int tile_pixels, int live_cap) {
     const size_t rec = (size_t)live_cap * MODEL_STAGE * 4;
     const size_t px = ((size_t)px_block(tile_pixels, live_cap) * PX_BYTES + 127) / 128 * 128;
-    return rec > px ? rec : px;
+    const size_t n = rec > px ? rec : px;
+    return n > MIN_STAGE ? n : MIN_STAGE;
 }
 __host__ __device__ inline size_t tile_smem_layout_bytes(int nw, int tile_pixels, int live_cap,
                                                          int idx_cap, int stride) {
@@ -755,7 +761,8 @@ constexpr int FLAG_LAST_SRC = 1;   // last kept Gaussian of its source
 // (at once with LAST_SRC).
 //
 // First every warp tests its share, 32 Gaussians at a time, and leaves one
-// mask word per 32 in shared memory (`mask`, `n_mask` words); the loads of a
+// mask word per 32 in shared memory (`work`, `n_work` words, the last QUEUE of
+// every warp its queue); the loads of a
 // Gaussian's box and record do not wait on each other, nor one group's on
 // another's, and no barrier stands between groups.  A Gaussian whose
 // exp-argument at the tile point nearest its centre is clearly below 36 is
@@ -768,12 +775,13 @@ constexpr int FLAG_LAST_SRC = 1;   // last kept Gaussian of its source
 // in every group 16,300 of 142,100.)
 template <int NT, bool LAST_SRC = false>
 __device__ __forceinline__ int scan_tile(const TileArgs &A, float4 bb, int g0, int g1, int npsf,
-                                         int *kept, unsigned *mask, int n_mask) {
+                                         int *kept, unsigned *work, int n_work) {
     constexpr int NW = NT / 32;
-    __shared__ int s_queue[NW][64];
+    const int n_mask = n_work - NW * QUEUE;
+    unsigned *mask = work;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const unsigned below = (1u << lane) - 1u;
-    int *queue = s_queue[warp];
+    int *queue = reinterpret_cast<int *>(work + n_mask + warp * QUEUE);
     int n_live = 0;
     for (int b0 = g0; b0 < g1; b0 += 32 * n_mask) {
         const int words = (min(g1 - b0, 32 * n_mask) + 31) >> 5;
