@@ -685,10 +685,8 @@ cudaError_t launch_dependent(const void *fn, dim3 grid, dim3 block, void **args,
 static thread_local int t_fail_alloc = 0;  // see fpho_test_fail_alloc
 
 cudaError_t pool_malloc(void **p, size_t bytes) {
-    if (t_fail_alloc > 0 && --t_fail_alloc == 0) {
-        *p = nullptr;
-        return cudaErrorMemoryAllocation;
-    }
+    *p = nullptr;
+    if (t_fail_alloc > 0 && --t_fail_alloc == 0) return cudaErrorMemoryAllocation;
     static std::once_flag once[64];
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
@@ -714,22 +712,24 @@ struct PinnedBlock {
 };
 constexpr size_t PINNED_KEEP = 16;
 std::mutex g_pinned_mu;
-std::vector<PinnedBlock> g_pinned;
+PinnedBlock g_pinned[PINNED_KEEP];
+size_t g_pinned_n = 0;
 }  // namespace
 
 cudaError_t pinned_get(void **p, size_t *bytes) {
     *p = nullptr;
+    if (t_fail_alloc > 0 && --t_fail_alloc == 0) return cudaErrorMemoryAllocation;
     {
         std::lock_guard<std::mutex> lk(g_pinned_mu);
-        size_t best = g_pinned.size();
-        for (size_t i = 0; i < g_pinned.size(); ++i)
+        size_t best = g_pinned_n;
+        for (size_t i = 0; i < g_pinned_n; ++i)
             if (g_pinned[i].bytes >= *bytes &&
-                (best == g_pinned.size() || g_pinned[i].bytes < g_pinned[best].bytes))
+                (best == g_pinned_n || g_pinned[i].bytes < g_pinned[best].bytes))
                 best = i;
-        if (best < g_pinned.size()) {
+        if (best < g_pinned_n) {
             *p = g_pinned[best].p;
             *bytes = g_pinned[best].bytes;
-            g_pinned.erase(g_pinned.begin() + best);
+            g_pinned[best] = g_pinned[--g_pinned_n];
             return cudaSuccess;
         }
     }
@@ -754,8 +754,8 @@ void pinned_put(void *p, size_t bytes) {
     if (!p) return;
     {
         std::lock_guard<std::mutex> lk(g_pinned_mu);
-        if (bytes <= PINNED_KEEP_BYTES && g_pinned.size() < PINNED_KEEP) {
-            g_pinned.push_back({p, bytes});
+        if (bytes <= PINNED_KEEP_BYTES && g_pinned_n < PINNED_KEEP) {
+            g_pinned[g_pinned_n++] = {p, bytes};
             return;
         }
     }
@@ -920,14 +920,15 @@ extern "C" int fpho_patch_retrieve(fpho_patch *p, int which, float *host_out, vo
     if (!src) return set_error(FPHO_ERR_STATE, "array %d is not allocated", which);
     cudaStream_t s = (cudaStream_t)stream;
     const size_t bytes = (size_t)p->npix * sizeof(float);
-    // pageable memory that fits a kept pinned block is filled through one: a
-    // transfer to it costs more than one to the block and the copy after it
+    // pageable memory that fits a kept pinned block is filled through one, if there
+    // is one: a transfer to it costs more than one to the block and the copy after it
     void *pin = nullptr;
     size_t cap = bytes;
     cudaPointerAttributes at;
     CUDA_TRY(cudaPointerGetAttributes(&at, host_out));
-    if (bytes <= PINNED_KEEP_BYTES && at.type == cudaMemoryTypeUnregistered)
-        CUDA_TRY(pinned_get(&pin, &cap));
+    if (bytes <= PINNED_KEEP_BYTES && at.type == cudaMemoryTypeUnregistered &&
+        pinned_get(&pin, &cap) != cudaSuccess)
+        cudaGetLastError();  // without a block, directly
     cudaError_t ce = cudaMemcpyAsync(pin ? pin : host_out, src, bytes, cudaMemcpyDeviceToHost, s);
     if (ce == cudaSuccess) ce = cudaStreamSynchronize(s);
     if (ce == cudaSuccess && pin) std::memcpy(host_out, pin, bytes);

@@ -442,8 +442,8 @@ FPHO_API int fpho_patch_set_exact_residual(fpho_patch *p, int on);
  * persistent schedule over many tiles. */
 FPHO_API int fpho_patch_set_test_stall(fpho_patch *p, int on);
 /* For tests of the error path only (no reference counterpart): the n-th of the
- * calling thread's device allocations for handles from now on fails with
- * FPHO_ERR_NOMEM; 0 for none. */
+ * calling thread's allocations for handles, device or pinned, from now on
+ * fails; 0 for none. */
 FPHO_API int fpho_test_fail_alloc(int n);
 
 /* Enable counting of evaluated (pixel, image Gaussian) pairs, i.e. pairs that

@@ -100,3 +100,16 @@ def test_retrieve_memory():
     np.testing.assert_array_equal(out, P.data)
     np.testing.assert_array_equal(pinned.numpy(), P.data)
     P.free()
+
+
+def test_retrieve_without_a_pinned_block():
+    from forcepho_b200 import _lib
+    P, _ = case(1)
+    out = np.zeros(len(P.data), np.float32)
+    _lib.call("fpho_test_fail_alloc", 1)
+    try:
+        _lib.call("fpho_patch_retrieve", P.device_patch.handle, 0, out.ctypes.data, None)
+    finally:
+        _lib.call("fpho_test_fail_alloc", 0)
+    np.testing.assert_array_equal(out, P.data)
+    P.free()
