@@ -87,6 +87,7 @@ _SIGS = {
                                            c_void_p, c_void_p]),
     "fpho_variant_info": (c_int, [c_int, ctypes.POINTER(c_int)]),
     "fpho_variant_shape": (c_int, [c_int, ctypes.POINTER(c_int)]),
+    "fpho_patch_tile_form": (c_int, [c_void_p, ctypes.POINTER(c_int)]),
     "fpho_patch_count_pairs": (c_int, [c_void_p, c_int, ctypes.POINTER(ctypes.c_longlong)]),
     "fpho_patch_error_word": (c_int, [c_void_p, ctypes.POINTER(c_int)]),
     "fpho_evaluate_proposal": (c_int, [c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_int,

@@ -1056,6 +1056,29 @@ extern "C" int fpho_variant_shape(int variant, int out[3]) {
     return variant_count();
 }
 
+namespace fpho {
+
+// Whether an evaluation takes its tiles in order of cost, by persistent CTAs:
+// the order only matters when the tiles outnumber what runs at once.
+static bool in_order(const fpho_patch *p) {
+    return p->schedule == 1 && p->n_tiles > 4 * device_sms();
+}
+// CTAs per tile otherwise (the exact mode has no parts).
+static int parts_of(const fpho_patch *p) {
+    if (in_order(p) || p->exact_residual) return 1;
+    return std::min(tile_parts(p->variant, p->n_tiles), p->max_parts);
+}
+
+}  // namespace fpho
+
+extern "C" int fpho_patch_tile_form(const fpho_patch *p, int out[2]) {
+    clear_error();
+    if (!p || !out) return set_error(FPHO_ERR_INVALID, "NULL argument");
+    out[0] = fpho::in_order(p) ? 1 : 0;
+    out[1] = fpho::parts_of(p);
+    return FPHO_OK;
+}
+
 extern "C" int fpho_patch_count_pairs(fpho_patch *p, int enable, long long *last_count) {
     clear_error();
     if (!p) return set_error(FPHO_ERR_INVALID, "NULL patch");
@@ -1084,12 +1107,9 @@ int enqueue_evaluate(fpho_patch *p, const fpho_source *prop, double *d_chi2, flo
                          "residual requested but the patch was created without one");
     if (p->count_pairs) CUDA_TRY(cudaMemsetAsync(p->d_pairs, 0, sizeof(long long), s));
     const PatchView pv = make_view(p);
-    // the order only matters when the tiles outnumber what runs at once
     const int sms = device_sms();
-    const bool ordered = p->schedule == 1 && p->n_tiles > 4 * sms;
-    // one CTA per tile otherwise, or per part of one (the exact mode has no parts)
-    const int parts =
-        p->exact_residual ? 1 : std::min(tile_parts(p->variant, p->n_tiles), p->max_parts);
+    const bool ordered = in_order(p);
+    const int parts = parts_of(p);
     // The tile kernel's CTAs may start beside the first kernel's, which saves
     // 2 us, but then go where those leave room, unevenly.  CTAs that fill the SMs
     // to the same number each cannot spare that and start after it: 144 tiles of

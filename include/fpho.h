@@ -446,6 +446,10 @@ FPHO_API int fpho_patch_set_test_stall(fpho_patch *p, int on);
  * fails; 0 for none. */
 FPHO_API int fpho_test_fail_alloc(int n);
 
+/* How the next evaluation runs its tiles: out[0] 1 for persistent CTAs over
+ * them, out[1] the CTAs per tile otherwise (1, 2 or 4). */
+FPHO_API int fpho_patch_tile_form(const fpho_patch *p, int out[2]);
+
 /* Enable counting of evaluated (pixel, image Gaussian) pairs, i.e. pairs that
  * survive the per-tile culling; *last_count receives the count of the last
  * evaluation (synchronizes).  last_count may be NULL. */
