@@ -16,7 +16,7 @@ Printed JSON (rank 0):
              timed per step with an L2 flush between steps (max over ranks);
   e2e        the same through GPUProposer.evaluate_proposal with the proposal
              in pinned host memory and results copied back every step;
-  roofline   the pixel-tile kernel: FP32 flops of its two passes (53 per evaluated
+  roofline   the pixel-tile kernel: FP32 flops of its two passes (56 per evaluated
              pixel-Gaussian pair) / its CUDA-event time, against the FP32 FMA
              throughput measured live by a probe kernel on the same GPU;
   cpu_baseline  the reference's own CPU kernel (built from its sources into
@@ -45,8 +45,9 @@ sys.path.insert(0, ROOT)
 
 METRIC = "chi2+grad evals/s & pix·gauss/s: batched vs plain, 1 B200, rel err ≤1e-6"
 # FP32 flops per evaluated pair, FMA = 2: 36 of the residual pass (18 of them the
-# exponential) and 17 of the gradient pass (its sums shared along pixel runs)
-FLOPS_PER_PAIR = 53
+# exponential) and 20 of the gradient pass (its sums shared along pixel runs; 23
+# for Gaussians not much wider than a pixel)
+FLOPS_PER_PAIR = 56
 WORKLOAD = "field20: 20 src, 8 bands x 4 exp x 128x128 px, 5-gauss PSF, 9 radii"
 # DRAM bytes (read + write) of one tile-kernel launch on this workload, from an
 # ncu capture of one launch of the split tile kernel: the 16 B per pixel of the

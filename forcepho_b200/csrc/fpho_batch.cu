@@ -126,7 +126,7 @@ const BatchShape kBatchShapes[] = {
     {64, 256, 0, (const void *)batch_tiles<64, 4, 0, 8>},
     {128, 512, 0, (const void *)batch_tiles<128, 4, 0, 4>},
     // split tiles with the registers capped at 128 (left free, the compiler
-    // takes 156 and fewer CTAs fit), and at 96 for 5 CTAs per SM
+    // takes up to 143 and fewer CTAs fit), and at 96 for 5 CTAs per SM
     {128, 256, 4, (const void *)batch_tiles<128, 8, 4, 4>},  // 4 warps share 256-pixel tiles
     {64, 256, 2, (const void *)batch_tiles<64, 8, 2, 8>},    // 2 warps share 256-pixel tiles
     {128, 256, 4, (const void *)batch_tiles<128, 8, 4, 5>},  // 4 warps, 5 CTAs per SM
@@ -469,10 +469,10 @@ static int batch_enqueue(fpho_batch *b, const fpho_source *d_props, double *d_ch
     if (b->n_exp_total > 0 && b->max_g > 0) {
         // Tile CTAs that start beside this kernel's go where those leave room,
         // some SMs getting several and others none.  Where they do not fill the
-        // SMs, that decides when the last is done, and they start after it (371
-        // tiles 296 against 496 us, 840 tiles 56.4 against 67.6); where they do,
-        // starting early is better (1681 tiles 342 against 366, 2532 tiles 370
-        // against 383).
+        // SMs, that decides when the last is done, and they start after it (626
+        // tiles 295 against 385 us, 840 tiles 61.5 against 74.0); where they do,
+        // starting early is better (1681 tiles 366 against 400, 2532 tiles 406
+        // against 421).
         void *gargs[] = {&b->d_bps, &b->d_expmap, &d_props, &b->d_err, &b->full};
         CUDA_TRY(launch_dependent((const void *)batch_gaussians,
                                   dim3((b->max_g + 127) / 128, b->n_exp_total), dim3(128), gargs,

@@ -130,7 +130,7 @@ __global__ void __launch_bounds__(NT) design_kernel(TileArgs A, float *X, long l
 // pixels per thread, 32 K pixels per tile.  MINB asks the compiler for at
 // least MINB resident CTAs per SM, a register cap of 64K / (32 NW MINB); the
 // default, 16 / NW, caps at 128 registers a thread (left free, the compiler
-// takes up to 180 and halves the resident warps).
+// takes up to 141 and fewer warps are resident).
 template <int NW, int K, bool GRAD, int MINB = 16 / NW, int PS = 1>
 __global__ void __launch_bounds__(32 * NW, MINB) split_kernel(TileArgs A) {
     extern __shared__ __align__(128) unsigned char smem[];
@@ -237,7 +237,7 @@ static const Variant kVariants[] = {
     FPHO_VARIANT(256, 4), FPHO_VARIANT(128, 8), FPHO_VARIANT(64, 8), FPHO_VARIANT(32, 8),
     FPHO_SPLIT_PARTED(4, 8, 4, 64, 4), FPHO_SPLIT(2, 8, 64, 4), FPHO_SPLIT(8, 8, 64, 4),
     FPHO_SPLIT(4, 4, 32, 4), FPHO_SPLIT_MINB(4, 8, 5, 64, 4),
-    FPHO_SPLIT_MINB(4, 6, 5, 32, 6),  // 192-pixel tiles, 95 registers: 5 CTAs per SM
+    FPHO_SPLIT_MINB(4, 6, 5, 32, 6),  // 192-pixel tiles, up to 96 registers: 5 CTAs per SM
 };
 #undef FPHO_VARIANT
 #undef FPHO_VARIANT_EXACT
@@ -315,9 +315,9 @@ int launch_tile_kernel(int variant, const TileArgs &A, int n_tiles, cudaStream_t
     // Few tiles per SM: 16 warps of CTAs on each instead of as many as fit (the
     // limit set by shared memory; a smaller grid would leave some SMs fuller
     // than others).  More CTAs make every tile take longer, the last ones too:
-    // 1140 tiles 117 against 124 us, 2048 tiles 283 against 288; from some 24
-    // tiles per SM more CTAs win (4800 tiles 543 against 531, 23,040 6.09
-    // against 5.89 ms).
+    // 1170 tiles 400 against 426 us, 2048 tiles 346 against 350, 3072 tiles 464
+    // against 466; from some 24 tiles per SM more CTAs win (4800 tiles 744 against
+    // 721, 23,040 6.70 against 6.52 ms).
     if (dyn && n_tiles < 24 * device_sms()) {
         const size_t few = (size_t)(SM_SMEM_BYTES / (512 / V.nt + 1)) - 512;
         smem = std::max(smem, few);
@@ -1113,10 +1113,10 @@ int enqueue_evaluate(fpho_patch *p, const fpho_source *prop, double *d_chi2, flo
     // The tile kernel's CTAs may start beside the first kernel's, which saves
     // 2 us, but then go where those leave room, unevenly.  CTAs that fill the SMs
     // to the same number each cannot spare that and start after it: 144 tiles of
-    // 30 sources 108 against 135 us, 432 tiles of 20 sources 115 against 124
-    // (chi2 only 63.5 against 69.6; none to 12 SMs short of even).  With more
-    // room early is better: 224 tiles 37.9 against 39.6, 264 quarters 29.7
-    // against 30.2, 448 tiles 98 against 100 (32 SMs short and more).
+    // 30 sources 115 against 151 us, 432 tiles of 20 sources 125 against 140
+    // (chi2 only 63.5 against 73.7; none to 12 SMs short of even).  With more
+    // room early is better, if by little: 256 tiles 85.1 against 86.1, 795
+    // persistent ones 75 against 77.
     const int ctas = p->n_tiles * parts;
     bool early = ordered || (sms - ctas % sms) % sms >= sms / 8;
     {

@@ -52,6 +52,9 @@ PatchView make_view(const fpho_patch *p);
 // usable from any stream; pool_free first waits for the device, as cudaFree
 // does, so memory still read by a kernel is never reused.  The pool keeps
 // the high-water mark of handle memory until the process exits.
+cudaError_t pool_malloc(void **p, size_t bytes);
+void pool_free(void *p);
+
 // Pinned host memory that kernels address directly (at the same address).  A
 // block given back, which no kernel may still use, is kept for the next
 // pinned_get of the process (16 blocks of up to 1 MiB at most; others are
@@ -61,7 +64,5 @@ PatchView make_view(const fpho_patch *p);
 constexpr size_t PINNED_KEEP_BYTES = 1 << 20;
 cudaError_t pinned_get(void **p, size_t *bytes);
 void pinned_put(void *p, size_t bytes);
-cudaError_t pool_malloc(void **p, size_t bytes);
-void pool_free(void *p);
 
 }  // namespace fpho

@@ -175,7 +175,9 @@ static __global__ void __launch_bounds__(PREP_THREADS) prepare_evaluation_arg(
 }
 
 // Sums of tile partials in double, for reduce_bands and batch_reduce alike (a
-// patch's batched result equals its single one bit for bit): one block of
+// patch's batched result equals its single one with the same tile shape bit for
+// bit, unless that one deals its tiles to several CTAs, which adds their
+// partials in another order): one block of
 // REDUCE_THREADS per 32 gradient components of a band and one for its chi2.
 // Component blocks: a warp reads a tile's 32 adjacent partials together and
 // takes every REDUCE_WARPS-th tile of [t0, t1); the warps' sums are added in

@@ -265,7 +265,7 @@ __device__ __forceinline__ void residual_pairs(const v2 (&X)[KP], const v2 (&Y)[
 // with its neighbour (measured: 3.07 and 2.25), so the chains take turns with
 // each constant.  The register file's reads are what bounds this loop.  With
 // the chains one after the other it took 8 registers more, and a fifth CTA no
-// longer fitted an SM (60-source patch 6.09 ms instead of 5.89).
+// longer fitted an SM (60-source patch 3% slower).
 template <int KP, int SH = SHARE_NONE>
 __device__ __forceinline__ void residual_pairs2(const v2 (&X)[KP], const v2 (&Y)[KP], v2 (&R)[KP],
                                                 const float *ra, const float *rb, v2 CM24,
